@@ -68,6 +68,7 @@ struct atsat_dyn {
     double* rm_tab = nullptr;            // 1 / rm(i)
     double* cor_j = nullptr;
     ColGeo* geo = nullptr;
+    StageGeo* sgeo = nullptr;            // FP64 path: the stage kernel's column table
     double** six = nullptr;              // device array: aux_u, aux_v, aux_w, rhs_u, rhs_v, rhs_w
     unsigned long long* counter = nullptr;
     std::vector<ColGeo> geo_h;
@@ -286,6 +287,7 @@ void build_constants(atsat_dyn* h) {
     K.inv_dphi2 = 1.0 / (g.dphi * g.dphi);
     K.coeff_energy_p = p.u_0 * p.u_0 / (p.cp_mix * p.t_ref);
     K.to_nd = 1.0 / (p.r_mix * p.u_0 * p.u_0 * 1.0e-5);
+    K.dps_scale = K.inv_2dr * K.to_nd;
     K.r_mix = p.r_mix;
     K.rR = p.r_mix * p.R_mix;
     K.buoy_c = p.g / (K.rR * p.t_ref);
@@ -302,6 +304,7 @@ void build_constants(atsat_dyn* h) {
     K.inv_sc_re_h2s = 1.0 / (p.sc_h2s * p.re);
     K.inv_sc_re_nh3 = 1.0 / (p.sc_nh3 * p.re);
     K.inv_sc_re_nh4sh = 1.0 / (p.sc_nh4sh * p.re);
+    K.nh3_as_h2o = K.inv_sc_re_nh3 == K.inv_sc_re_h2o;
     K.inv_sig_k = 1.0 / 0.85;
     K.inv_sig_w = 1.0 / 0.5;
     K.turb_coupling = p.turb_coupling;
@@ -317,6 +320,7 @@ void build_constants(atsat_dyn* h) {
     K.precip_coupling = p.precip_coupling;
     K.precip_num = L_m;
     K.precip_den = 1.0 / (p.r_mix * p.cp_mix * p.u_0 * p.t_ref);
+    K.precip_factor = K.precip_coupling * K.precip_num * K.precip_den;
     K.tmf_chem = p.thermal_massflux * p.chemical_reaction;
     K.species_divu = p.species_divu;
     K.tke_max = 1000.0 / (p.u_0 * p.u_0);
@@ -391,18 +395,6 @@ void build_geometry(atsat_dyn* h, const double* vbar0, const double* ubar0) {
             c.src_the = c.p_inv_rm / (2.0 * g.dthe);
             c.src_phi = c.p_inv_rmsinthe / (2.0 * g.dphi);
             c.p_inv_den = 1.0 / c.p_den;
-            {
-                const double i2dr = 1.0 / (2.0 * g.dr), i2dthe = 1.0 / (2.0 * g.dthe), i2dphi = 1.0 / (2.0 * g.dphi);
-                c.t_the = i2dthe * c.inv_rm;
-                c.t_phi = i2dphi * c.inv_rmsinthe;
-                c.d_r1 = c.two_inv_rm * i2dr;
-                c.d_t2 = c.inv_rm2 * inv_dthe2;
-                c.d_t1 = c.costhe_inv_rm2sinthe * i2dthe;
-                c.d_p2 = c.inv_rm2sinthe2 * inv_dphi2;
-                c.x_v1 = 2.0 * c.inv_rm2 * i2dthe;
-                c.x_v2 = 2.0 * c.costhe * c.inv_rm2sinthe2 * i2dphi;
-                c.x_w1 = 2.0 * c.inv_rm2sinthe * i2dphi;
-            }
         }
     }
 }
@@ -425,7 +417,7 @@ void build_mixed_constants(atsat_dyn* h) {
     F.inv_sig_k = (float)K.inv_sig_k; F.inv_sig_w = (float)K.inv_sig_w;
     F.turb_coupling = (float)K.turb_coupling; F.inv_pr_t = (float)K.inv_pr_t;
     F.chem = (float)K.chem; F.precip_coupling = (float)K.precip_coupling;
-    F.precip_factor = (float)(K.precip_coupling * K.precip_num * K.precip_den);
+    F.precip_factor = (float)K.precip_factor;
     F.rad_factor = (float)(K.rad_coupling * K.rad_num / K.rad_den_c);
     F.r_mix = (float)K.r_mix;
     F.tke_max = (float)K.tke_max; F.dis_min = (float)K.dis_min;
@@ -434,6 +426,45 @@ void build_mixed_constants(atsat_dyn* h) {
     F.kb = p.buoy_legacy ? 1.0f : (float)K.kbuoy;
     F.bref_scale = p.buoy_legacy ? 0.0f : 1.0f;
     F.tke_max_d = K.tke_max; F.dis_min_d = K.dis_min;
+}
+
+// the FP64 stage kernel's column table, from the geometry
+cudaError_t upload_stage_geo(atsat_dyn* h) {
+    const KConst& K = h->kc;
+    std::vector<StageGeo> sg(h->geo_h.size());
+    for (size_t n = 0; n < sg.size(); n++) {
+        const ColGeo& c = h->geo_h[n];
+        StageGeo& s = sg[n];
+        const double dr1 = c.two_inv_rm * K.inv_2dr;
+        const double dt2 = c.inv_rm2 * K.inv_dthe2, dt1 = c.costhe_inv_rm2sinthe * K.inv_2dthe;
+        s.s_the = K.inv_2dthe * c.inv_rm;
+        s.s_phi = K.inv_2dphi * c.inv_rmsinthe;
+        s.l_rp = K.inv_dr2 + dr1;
+        s.l_rm = K.inv_dr2 - dr1;
+        s.lu_rp = K.inv_dr2 + 2.0 * dr1;
+        s.lu_rm = K.inv_dr2 - 2.0 * dr1;
+        s.l_tp = dt2 + dt1;
+        s.l_tm = dt2 - dt1;
+        s.l_p = c.inv_rm2sinthe2 * K.inv_dphi2;
+        s.l_0 = -2.0 * (K.inv_dr2 + dt2 + s.l_p);
+        s.inv_rm = c.inv_rm;
+        s.cot = c.cotanthe;
+        s.v_metric = c.v_metric;
+        s.u_metric = 2.0 * c.inv_rm2;
+        s.x_v1 = 2.0 * c.inv_rm2 * K.inv_2dthe;
+        s.x_v2 = 2.0 * c.costhe * c.inv_rm2sinthe2 * K.inv_2dphi;
+        s.x_w1 = 2.0 * c.inv_rm2sinthe * K.inv_2dphi;
+        s.c_rad = K.cor_rad_on * K.Coriolis * c.cor_rad;
+        s.c_the = K.Coriolis * c.cor_the;
+        s.c_v = K.Coriolis * c.cor_phi * c.costhe;
+        s.c_u = K.Coriolis * c.cor_phi * c.sinthe_true;
+        s.c_0 = s.c_v * c.vbar0 + s.c_u * c.ubar0;
+        s.cent_rad = K.centrifugal * c.cent_rad;
+        s.cent_the = K.centrifugal * c.cent_the;
+    }
+    const cudaError_t e = cudaMemcpyAsync(h->sgeo, sg.data(), sizeof(StageGeo) * sg.size(), cudaMemcpyHostToDevice,
+                                          h->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(h->stream);
 }
 
 cudaError_t upload_geof(atsat_dyn* h) {
@@ -825,7 +856,7 @@ StageIO<double> make_io(atsat_dyn* h, double* const* in, double* const* out) {
     io.aux[1] = h->f[ATSAT_F_AUX_V];
     io.aux[2] = h->f[ATSAT_F_AUX_W];
     io.buoy = h->buoy;
-    io.geo = h->geo;
+    io.geo = h->sgeo;
     return io;
 }
 
@@ -1874,7 +1905,7 @@ int atsat_dyn_create(const atsat_dyn_grid* g, const atsat_dyn_params* p, atsat_d
     const bool fp64_stage = p->precision != ATSAT_DYN_MIXED;
     const int64_t nbig = ATSAT_NFIELDS + (fp64_stage ? 2 * NPROG : 0) + 2;
     const int64_t nsmall = 2LL * K.im * 16 + K.im + K.jm + K.im + K.jm + 64;
-    const size_t bytes = (size_t)(nbig * K.fsz + nsmall) * 8 + sizeof(ColGeo) * (size_t)K.im * K.jm + 4096;
+    const size_t bytes = (size_t)(nbig * K.fsz + nsmall) * 8 + (sizeof(ColGeo) + (fp64_stage ? sizeof(StageGeo) : 0)) * (size_t)K.im * K.jm + 4096;
     if ((e = cudaMalloc(&h->slab, bytes)) != cudaSuccess) return cuda_fail(e, "cudaMalloc");
     if ((e = cudaMemsetAsync(h->slab, 0, bytes, h->stream)) != cudaSuccess) return cuda_fail(e, "cudaMemset");
     double* q = h->slab;
@@ -1896,6 +1927,10 @@ int atsat_dyn_create(const atsat_dyn_grid* g, const atsat_dyn_params* p, atsat_d
     h->six = reinterpret_cast<double**>(q); q += 8;
     q = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(q) + 255) & ~uintptr_t(255));
     h->geo = reinterpret_cast<ColGeo*>(q);
+    if (fp64_stage) {
+        h->sgeo = reinterpret_cast<StageGeo*>(h->geo + (size_t)K.im * K.jm);
+        if ((e = upload_stage_geo(h)) != cudaSuccess) return cuda_fail(e, "stage geometry upload");
+    }
     if (p->precision == ATSAT_DYN_MIXED) {
         // 118 arrays of fsz floats (the tensor maps' fourth dimension), then the two column tables
         h->n32 = 2 * NPROG + 2 + 3 * NPROG + 2 + NFZ + NCONV;
@@ -2101,6 +2136,7 @@ int atsat_dyn_set_tables(atsat_dyn_t h, const double* cell_vbar0, const double* 
     CK(h, cudaMemcpyAsync(h->geo, h->geo_h.data(), sizeof(ColGeo) * h->geo_h.size(), cudaMemcpyHostToDevice,
                           h->stream));
     if (h->geof) CK(h, upload_geof(h));
+    if (h->sgeo) CK(h, upload_stage_geo(h));
     h->has_pbaro = (p_baro != nullptr);
     if (p_baro) {
         const KConst& K = h->kc;

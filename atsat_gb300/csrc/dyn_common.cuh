@@ -97,12 +97,23 @@ struct alignas(16) ColGeo {
     // the source factors times the centred-difference scales (exp_rm / (2 dr), 1 / (2 dthe rm),
     // 1 / (2 dphi rm sin)) and 1 / p_den: one product per term instead of two, no FP64 division
     double src_r, src_the, src_phi, p_inv_den;
-    // the FP64 stage's stencil scales folded into one coefficient per term (raw differences a0 = f(i+1) -
-    // f(i-1), b0, c0 along theta and phi, second differences a1, b1, c1): transport v b0 t_the + w c0 t_phi,
-    // diffusion a0 d_r1 + b1 d_t2 + b0 d_t1 + c1 d_p2, and the cross terms of the u, v, w diffusion
-    double t_the, t_phi, d_r1, d_t2, d_t1, d_p2, x_v1, x_v2, x_w1, pad_c;
 };
-static_assert(sizeof(ColGeo) == 46 * 8, "ColGeo layout");
+static_assert(sizeof(ColGeo) == 36 * 8, "ColGeo layout");
+
+// The FP64 stage kernel's column table: every factor a cell of column (i, j) multiplies with, formed once on the
+// host. Diffusion as one weight per stencil value (l_rp for f(i+1), l_rm for f(i-1), l_tp / l_tm along theta,
+// l_p for both phi neighbours, l_0 for the centre; lu_rp / lu_rm for u, whose radial term is 4/rm du/dr), the
+// gradients' scales (s_the = 1 / (2 dtheta rm), s_phi = 1 / (2 dphi rm sin)), the cross terms of the u, v, w
+// diffusion (x_*) and the body forces (c_v v + c_u u - c_0 is the phi Coriolis term with the held means).
+struct alignas(16) StageGeo {
+    double s_the, s_phi, l_rp, l_rm;
+    double lu_rp, lu_rm, l_tp, l_tm;
+    double l_p, l_0, inv_rm, cot;
+    double v_metric, u_metric, x_v1, x_v2;
+    double x_w1, c_rad, c_the, c_v;
+    double c_u, c_0, cent_rad, cent_the;
+};
+static_assert(sizeof(StageGeo) == 24 * 8, "StageGeo layout");
 
 // Grid-wide constants, every one formed on the host in the reference's own expression order.
 struct KConst {
@@ -113,11 +124,13 @@ struct KConst {
     int adiabatic, adiabatic_rho, buoy_legacy, hydro_buoy;
     int t_limiter, cell_hold, rad_on, precip_on;
     int tmf_on, divu_on, press_incr, press_src;
-    int rigid_lid, press_wall, pad_i0, pad_i1;
+    int rigid_lid, press_wall;
+    int nh3_as_h2o, pad_i1;        // the ammonia group has the water group's Schmidt number
     double dr;
     double inv_2dr, inv_2dthe, inv_2dphi, inv_dr2, inv_dthe2, inv_dphi2;
     double coeff_energy_p;         // u_0 u_0 / (cp_mix t_ref)
     double to_nd;                  // 1 / (r_mix u_0 u_0 1e-5)
+    double dps_scale;              // inv_2dr to_nd
     double r_mix;
     double rR, t_ref, g;           // r_mix R_mix, for the buoyancy b = g p / (rR t t_ref)
     double buoy_c;                 // g / (rR t_ref)
@@ -131,6 +144,7 @@ struct KConst {
     double metric_on, cor_rad_on;
     double rad_coupling, rad_num, rad_den_c;   // L_rad; cp_mix u_0 t_ref
     double precip_coupling, precip_num, precip_den;
+    double precip_factor;          // precip_coupling precip_num precip_den
     double tmf_chem;               // thermal_massflux * chemical_reaction
     double species_divu;
     double tke_max, dis_min;
@@ -164,7 +178,7 @@ struct StageIO {
     double* rhs[NPROG];            // rhs_* (written where the mode asks for it)
     double* aux[3];                // aux_u/v/w
     const double* buoy;            // buoy_ref_level[im]
-    const ColGeo* geo;             // [im * jm]
+    const StageGeo* geo;           // [im * jm]
 };
 
 // ---- mixed precision (rk_mixed.cu) ----

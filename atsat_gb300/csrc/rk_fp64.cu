@@ -23,6 +23,27 @@ __device__ __forceinline__ double ldg(const double* p) { return __ldg(p); }
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
 
+// Comparisons on the integer pipe: GB300's FP64 pipe issues two operations per SM per cycle and a DSETP takes a
+// slot like an addition. Each test settles the common case on the double's high word and leaves the rest to the
+// comparison itself.
+__device__ __forceinline__ uint32_t hi_word(double x) {
+    uint32_t lo, hi;
+    split_f64(x, lo, hi);
+    return hi;
+}
+__device__ __forceinline__ bool finite(double x) { return (hi_word(x) & 0x7FF00000u) != 0x7FF00000u; }
+// true: lim < x < inf for sure (lim > 0); false: unknown
+__device__ __forceinline__ bool surely_above(double x, double lim) { return hi_word(x) - hi_word(lim) - 1u < 0x7FEFFFFFu - hi_word(lim); }
+// max(0, x) of a finite x, +0 for x = -0
+__device__ __forceinline__ double positive(double x) { return (hi_word(x) >> 31) ? 0.0 : x; }
+// x clipped to [-0.5, 0.5], 0 where x is not finite
+__device__ __forceinline__ double clip_half(double x) {
+    const uint32_t a = hi_word(x) & 0x7FFFFFFFu;
+    if (a < 0x3FE00000u) return x;
+    if (a >= 0x7FF00000u) return 0.0;
+    return (hi_word(x) >> 31) ? -0.5 : 0.5;
+}
+
 template <int MODE>
 __device__ __forceinline__ void emit(const StageIO<double>& io, const StageParams& sp, const KConst& K, int q,
                                      int64_t c, double r) {
@@ -32,7 +53,7 @@ __device__ __forceinline__ void emit(const StageIO<double>& io, const StageParam
     }
     double y;
     if (MODE == MODE_STAGE) {
-        const double a = (sp.stage == 0) ? sp.wgt * r : io.acc[q][c] + sp.wgt * r;
+        const double a = fma(sp.wgt, r, (sp.stage == 0) ? 0.0 : io.acc[q][c]);
         io.acc[q][c] = a;
         y = ldg(io.yn[q] + c) + sp.c_in * r;
     } else {
@@ -40,49 +61,78 @@ __device__ __forceinline__ void emit(const StageIO<double>& io, const StageParam
         y = ldg(io.yn[q] + c) + sp.sixth_dt * a;
         if (sp.write_all_rhs || q < 3) io.rhs[q][c] = r;
     }
-    if (q == ATSAT_F_TKE) y = smin(smax(y, 0.0), K.tke_max);
-    else if (q == ATSAT_F_DIS) y = smax(y, K.dis_min);
+    if (q == ATSAT_F_TKE) {
+        if (hi_word(y) >= hi_word(K.tke_max)) y = smin(smax(y, 0.0), K.tke_max);
+    } else if (q == ATSAT_F_DIS) {
+        if (!surely_above(y, K.dis_min)) y = smax(y, K.dis_min);
+    }
     io.out[q][c] = y;
 }
 
-// The stencil of one field as raw differences: a0 = f(i+1) - f(i-1), a1 = f(i+1) - 2 f + f(i-1), and b0, b1
-// along theta, c0, c1 along phi. fma(-2, x, p) equals p - 2x bit for bit (the product is exact).
-struct R6 { double a0, a1, b0, b1, c0, c1; };
+// The stencil of one field: the centre and its six neighbours.
+struct S7 { double c, rp, rm, tp, tm, pe, pw; };
 
-__device__ __forceinline__ void raw6(const double* __restrict__ f, int64_t c, int64_t plane, int kp, int dkw,
-                                     int dke, R6& r) {
-    const double x = ldg(f + c);
-    const double rp = ldg(f + c + plane), rn = ldg(f + c - plane);
-    const double tp = ldg(f + c + kp), tn = ldg(f + c - kp);
-    const double pe = ldg(f + c + dke), pw = ldg(f + c + dkw);
-    r.a0 = rp - rn;
-    r.a1 = fma(-2.0, x, rp) + rn;
-    r.b0 = tp - tn;
-    r.b1 = fma(-2.0, x, tp) + tn;
-    r.c0 = pe - pw;
-    r.c1 = fma(-2.0, x, pe) + pw;
+__device__ __forceinline__ S7 stencil(const double* __restrict__ f, int64_t c, int64_t plane, int kp, int dkw, int dke) {
+    return S7{ldg(f + c), ldg(f + c + plane), ldg(f + c - plane), ldg(f + c + kp), ldg(f + c - kp), ldg(f + c + dke),
+              ldg(f + c + dkw)};
+}
+// neighbours minus the centre
+__device__ __forceinline__ S7 centred(const S7& f) {
+    return S7{f.c, f.rp - f.c, f.rm - f.c, f.tp - f.c, f.tm - f.c, f.pe - f.c, f.pw - f.c};
 }
 
-// Per-cell factors shared by every field: the advecting velocity times the stencil scales, and the
-// diffusion operator's coefficient per raw difference (from the column table).
-struct Fold {
-    double U, V, W, dr2, dr1, dt2, dt1, dp2;
-    __device__ __forceinline__ double transport(const R6& r) const { return fma(U, r.a0, fma(V, r.b0, W * r.c0)); }
-    __device__ __forceinline__ double diffusion(const R6& r) const {
-        return fma(dr2, r.a1, fma(dr1, r.a0, fma(dt2, r.b1, fma(dt1, r.b0, dp2 * r.c1))));
-    }
-};
+// kappa diffusion - transport of a field as one weight per stencil value (the transport's weights sum to zero
+// over the neighbours, the diffusion's centre weight is kappa l_0).
+struct Wt { double rp, rm, tp, tm, pe, pw, c; };
 
-// GB300 issues two FP64 operations per SM per cycle, and this kernel is bound by that pipe. The reference
-// scales each of a field's six differences before combining them (RHS_Sat_Turb.cpp:300-1000); here the
-// scales are folded into per-cell factors (Fold) and per-column coefficients (ColGeo), so a field costs its
-// nine differencing operations, three for transport and five for diffusion. Every term is the reference's;
-// the products are associated differently (a few ulps per term).
-template <int MODE>
-__global__ void __launch_bounds__(256) rk_stage_fp64_kernel(const KConst K, const StageIO<double> io,
-                                                            const StageParams sp) {
+__device__ __forceinline__ Wt weights(double kappa, double U, double V, double W, const StageGeo& g) {
+    return Wt{fma(kappa, g.l_rp, -U), fma(kappa, g.l_rm, U), fma(kappa, g.l_tp, -V), fma(kappa, g.l_tm, V),
+              fma(kappa, g.l_p, -W), fma(kappa, g.l_p, W), kappa * g.l_0};
+}
+
+// extra + sum over the neighbours of weight times difference to the centre
+__device__ __forceinline__ double apply_centred(const Wt& w, const S7& d, double extra) {
+    return fma(w.rp, d.rp, fma(w.rm, d.rm, fma(w.tp, d.tp, fma(w.tm, d.tm, fma(w.pe, d.pe, fma(w.pw, d.pw, extra))))));
+}
+// the same on the values themselves
+__device__ __forceinline__ double apply_values(const Wt& w, const S7& f, double extra) {
+    return fma(w.rp, f.rp, fma(w.rm, f.rm, fma(w.tp, f.tp, fma(w.tm, f.tm,
+           fma(w.pe, f.pe, fma(w.pw, f.pw, fma(w.c, f.c, extra)))))));
+}
+
+// The default switches: metric split on, no hydro-buoyancy, no legacy buoyancy, no radiation or thermal-mass-flux
+// source, no flux-form species term, and couplings of exactly 1 (whose products are the factors themselves).
+bool plain_knobs(const KConst& K) {
+    return K.metric_split && !K.hydro_buoy && !K.buoy_legacy && !K.rad_on && !K.tmf_on && !K.divu_on &&
+           K.precip_coupling == 1.0 && K.chem == 1.0 && K.turb_coupling == 1.0;
+}
+
+// Rows of 32 cells per block and blocks per SM: 4 x 128 threads at 128 registers, no spills. The two-iteration
+// step at 41x181x361 took 13.36 ms with 2 x 256, 13.21 with 4 x 128, 13.24 / 13.27 / 13.29 with 5 / 6 / 8 x 128
+// (spilling), 15.05 with 1 x 256: a few warps fill the FP64 pipe, the finer blocks even out the last wave.
+constexpr int RKS_ROWS = 4, RKS_BLOCKS = 4;
+
+// What bounds it: the FP64 pipe (two operations per SM per cycle). With the differences of each field scaled and
+// combined one by one it was 590 FP64 instructions per interior cell and 2.38 ms per launch at 41x181x361, while
+// the launch's 1.97 GB take 0.29 ms. So the kernel is written for the fewest FP64 operations: 302 per cell, 1.46 ms
+// (the two-iteration step 20.03 -> 12.68 ms; at 27x118x222 the launch 0.595 -> 0.362 ms). Transport and diffusion of
+// RHS_Sat_Turb.cpp:300-1000 together are one weight per stencil value: seven fused multiply-adds per field with
+// weights that cost seven more per diffusivity -- shared by the three phases of a species, by u, v and w, and by the
+// water and ammonia groups where their Schmidt numbers are equal. Comparisons run on the integer pipe.
+//   u, v, w always combine differences to the centre (five operations more per field): their tendencies are
+//   results (the projection's source), w's zonal differences are small against w, and differences of near-equal
+//   values are exact. So do k* and omega*: the closure floors k* to a uniform value and divides by gradients that
+//   a uniform field must leave at zero. t and the species do the same where their tendencies are asked for
+//   (CENTRED); else the tendency only enters y + dt r, and the rounding of weight times value, eps sum |weight| |f|,
+//   is there below eps |f| times dt sum |weight| -- the Courant number that a stable step keeps under 3.
+// PLAIN: the default switches (`plain_knobs`), whose branches are then left out at compile time: an instruction
+// the compiler predicates off still takes its slot of the FP64 pipe.
+template <int MODE, bool CENTRED, bool PLAIN>
+__global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kernel(const KConst K,
+                                                                                  const StageIO<double> io,
+                                                                                  const StageParams sp) {
     const int k = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 8 + threadIdx.y;
+    const int j = blockIdx.y * RKS_ROWS + threadIdx.y;
     const int i = blockIdx.z;
     if (k >= K.km || j >= K.jm) return;
     const int64_t plane = K.plane;
@@ -100,167 +150,133 @@ __global__ void __launch_bounds__(256) rk_stage_fp64_kernel(const KConst K, cons
     const int kw = (k == 0) ? K.km - 2 : k - 1;
     const int ke = (k == K.km - 2) ? 0 : k + 1;
     const int dkw = kw - k, dke = ke - k;
+    const StageGeo& g = io.geo[(int64_t)i * K.jm + j];
+    auto load = [&](int q) { return stencil(io.in[q], c, plane, kp, dkw, dke); };
 
-    const ColGeo* gp = io.geo + ((int64_t)i * K.jm + j);
-    const double inv_rm = ldg(&gp->inv_rm), inv_rm2 = ldg(&gp->inv_rm2), inv_rmsinthe = ldg(&gp->inv_rmsinthe);
-    const double cotanthe = ldg(&gp->cotanthe), costhe = ldg(&gp->costhe), v_metric = ldg(&gp->v_metric);
-
-    const double u = ldg(io.in[ATSAT_F_U] + c);
-    const double v = ldg(io.in[ATSAT_F_V] + c);
-    const double w = ldg(io.in[ATSAT_F_W] + c);
-    Fold fd;
-    fd.U = u * K.inv_2dr;
-    fd.V = v * ldg(&gp->t_the);
-    fd.W = w * ldg(&gp->t_phi);
-    fd.dr2 = K.inv_dr2;
-    fd.dr1 = ldg(&gp->d_r1);
-    fd.dt2 = ldg(&gp->d_t2);
-    fd.dt1 = ldg(&gp->d_t1);
-    fd.dp2 = ldg(&gp->d_p2);
-
-    R6 ru, rv, rw;
-    raw6(io.in[ATSAT_F_U], c, plane, kp, dkw, dke, ru);
-    raw6(io.in[ATSAT_F_V], c, plane, kp, dkw, dke, rv);
-    raw6(io.in[ATSAT_F_W], c, plane, kp, dkw, dke, rw);
-    const double dpdr = (ldg(io.p_dyn + c + plane) - ldg(io.p_dyn + c - plane)) * K.inv_2dr;
-    const double dpdthe = (ldg(io.p_dyn + c + kp) - ldg(io.p_dyn + c - kp)) * K.inv_2dthe;
-    const double dpdphi = (ldg(io.p_dyn + c + dke) - ldg(io.p_dyn + c + dkw)) * K.inv_2dphi;
+    const S7 su = load(ATSAT_F_U), sv = load(ATSAT_F_V), sw = load(ATSAT_F_W);
+    const double u = su.c, v = sv.c, w = sw.c;
+    const double U = u * K.inv_2dr, V = v * g.s_the, W = w * g.s_phi;
+    const double dpr = (ldg(io.p_dyn + c + plane) - ldg(io.p_dyn + c - plane)) * K.inv_2dr;
+    const double dpth = (ldg(io.p_dyn + c + kp) - ldg(io.p_dyn + c - kp)) * g.s_the;
+    const double dpph = (ldg(io.p_dyn + c + dke) - ldg(io.p_dyn + c + dkw)) * g.s_phi;
 
     // eddy viscosity as the momentum / scalar equations read it (RHS_Sat_Turb.cpp:577-582)
     const double nue_c = ldg(io.nue + c);
-    const double nue_t = (K.turb_coupling != 0.0 && isfinite(nue_c)) ? K.turb_coupling * smax(0.0, nue_c) : 0.0;
+    const double nue_t = finite(nue_c) ? (PLAIN ? 1.0 : K.turb_coupling) * positive(nue_c) : 0.0;
     const double nue_t_s = nue_t * K.inv_pr_t;
+    double sd = 0.0;              // flux-form factor of the species (RHS_Sat_Turb.cpp:979-1009)
 
     // ---- momentum (RHS_Sat_Turb.cpp:310-350, 388-399, 435-456, 700-714, 780-835) ----
     {
-        const double cor_rad = ldg(&gp->cor_rad) * w;
-        const double cor_the = ldg(&gp->cor_the) * w;
-        const double v_cor = v - ldg(&gp->vbar0), u_cor = u - ldg(&gp->ubar0);
-        const double cor_phi = ldg(&gp->cor_phi) * (costhe * v_cor + ldg(&gp->sinthe_true) * u_cor);
-
-        double transport_u = fd.transport(ru);
-        if (!K.metric_split) transport_u = transport_u - K.metric_on * (v * v + w * w) * inv_rm;
-        const double transport_v = fd.transport(rv) + (u * v - w * w * cotanthe) * inv_rm;
-        const double transport_w = fd.transport(rw) + (w * u + v * w * cotanthe) * inv_rm;
-        // diffusion_u: 4 du/dr / rm in place of du/dr 2 / rm, and 2 u / rm^2
-        const double diffusion_u = fma(fd.dr1, ru.a0, fd.diffusion(ru)) + 2.0 * u * inv_rm2;
-        const double x_v2 = ldg(&gp->x_v2);
-        const double diffusion_v = fd.diffusion(rv) - v_metric * v + ldg(&gp->x_v1) * ru.b0 - x_v2 * rw.c0;
-        const double diffusion_w = fd.diffusion(rw) - v_metric * w + ldg(&gp->x_w1) * ru.c0 + x_v2 * rv.c0;
+        const S7 du = centred(su), dv = centred(sv), dw = centred(sw);
+        const double visc = K.inv_re + nue_t;
+        const Wt wt = weights(visc, U, V, W, g);
+        Wt wu = wt;
+        wu.rp = fma(visc, g.lu_rp, -U);
+        wu.rm = fma(visc, g.lu_rm, U);
+        const double u_t = du.tp - du.tm, u_p = du.pe - du.pw, v_p = dv.pe - dv.pw, w_p = dw.pe - dw.pw;
 
         double buoyancy_u = 0.0;
         const double t_c = ldg(io.in[ATSAT_F_T] + c);
-        if (t_c > 0.0 && !K.hydro_buoy) {
+        if (PLAIN || !K.hydro_buoy) {
             const double ps = ldg(io.p_stat + c);
-            if (K.buoy_legacy) buoyancy_u = K.legacy_buoy * (ps + ldg(io.p_dyn + c)) / (K.rR * t_c * K.t_ref);
-            else if (in_rcp_range(t_c)) buoyancy_u = K.kbuoy * ((K.buoy_c * ps) * recip_nr(t_c) - ldg(io.buoy + i));
-            else buoyancy_u = K.kbuoy * (K.g * ps / (K.rR * t_c * K.t_ref) - ldg(io.buoy + i));
+            if ((PLAIN || !K.buoy_legacy) && in_rcp_range(t_c)) {
+                buoyancy_u = K.kbuoy * ((K.buoy_c * ps) * recip_nr(t_c) - ldg(io.buoy + i));
+            } else if (t_c > 0.0) {
+                if (!PLAIN && K.buoy_legacy) buoyancy_u = K.legacy_buoy * (ps + ldg(io.p_dyn + c)) / (K.rR * t_c * K.t_ref);
+                else buoyancy_u = K.kbuoy * (K.g * ps / (K.rR * t_c * K.t_ref) - ldg(io.buoy + i));
+            }
         }
-        const double visc = K.inv_re + nue_t;
-        const double rhs_u = -dpdr + buoyancy_u - transport_u + diffusion_u * visc
-                           - K.cor_rad_on * K.Coriolis * cor_rad + K.centrifugal * ldg(&gp->cent_rad);
-        double dpmdthe = 0.0, dpmdphi = 0.0;
-        if (K.metric_split) {
-            dpmdthe = (ldg(io.p_metric + c + kp) - ldg(io.p_metric + c - kp)) * K.inv_2dthe;
-            dpmdphi = (ldg(io.p_metric + c + dke) - ldg(io.p_metric + c + dkw)) * K.inv_2dphi;
+        double fu = fma(visc, g.u_metric * u, fma(-g.c_rad, w, g.cent_rad + buoyancy_u) - dpr);
+        if (!PLAIN && !K.metric_split) fu = fma(K.metric_on * g.inv_rm, fma(v, v, w * w), fu);
+        const double rhs_u = apply_centred(wu, du, fu);
+
+        double pth = dpth, pph = dpph;
+        if (PLAIN || K.metric_split) {
+            pth = fma(ldg(io.p_metric + c + kp) - ldg(io.p_metric + c - kp), g.s_the, pth);
+            pph = fma(ldg(io.p_metric + c + dke) - ldg(io.p_metric + c + dkw), g.s_phi, pph);
         }
-        const double rhs_v = -(dpdthe + dpmdthe) * inv_rm - transport_v + diffusion_v * visc - K.Coriolis * cor_the
-                           + K.centrifugal * ldg(&gp->cent_the);
-        const double rhs_w = -(dpdphi + dpmdphi) * inv_rmsinthe - transport_w + diffusion_w * visc
-                           - K.Coriolis * cor_phi;
+        const double wcot = w * g.cot;
+        const double mv = fma(u, v, -(w * wcot)), mw = fma(w, u, v * wcot);
+        const double xv = fma(g.x_v1, u_t, -fma(g.x_v2, w_p, g.v_metric * v));
+        const double xw = fma(g.x_w1, u_p, fma(g.x_v2, v_p, -(g.v_metric * w)));
+        const double rhs_v = apply_centred(wt, dv, fma(visc, xv, fma(-mv, g.inv_rm, fma(-g.c_the, w, g.cent_the) - pth)));
+        const double rhs_w = apply_centred(wt, dw, fma(visc, xw, fma(-mw, g.inv_rm,
+                                           fma(-g.c_v, v, fma(-g.c_u, u, g.c_0)) - pph)));
         emit<MODE>(io, sp, K, ATSAT_F_U, c, rhs_u);
         emit<MODE>(io, sp, K, ATSAT_F_V, c, rhs_v);
         emit<MODE>(io, sp, K, ATSAT_F_W, c, rhs_w);
         if (MODE != MODE_STAGE) {
-            io.aux[0][c] = rhs_u + dpdr;
-            io.aux[1][c] = rhs_v + dpdthe * inv_rm;
-            io.aux[2][c] = rhs_w + dpdphi * inv_rmsinthe;
+            io.aux[0][c] = rhs_u + dpr;
+            io.aux[1][c] = rhs_v + dpth;
+            io.aux[2][c] = rhs_w + dpph;
         }
+        if (!PLAIN && K.divu_on)
+            sd = K.species_divu * ((du.rp - du.rm) * K.inv_2dr + 2.0 * u * g.inv_rm + (dv.tp - dv.tm) * g.s_the
+                                   + v * g.cot * g.inv_rm + w_p * g.s_phi);
     }
 
-    // flux-form factor of the species (RHS_Sat_Turb.cpp:979-1009), 0 unless ATSAT_SPECIES_DIVU
-    const double sd = K.divu_on ? K.species_divu * (ru.a0 * K.inv_2dr + 2.0 * u * inv_rm + rv.b0 * ldg(&gp->t_the)
-                                                    + v * cotanthe * inv_rm + rw.c0 * ldg(&gp->t_phi))
-                                : 0.0;
+    // kappa diffusion - transport + extra of field q
+    auto tendency = [&](int q, const Wt& wt, double extra) -> double {
+        const S7 f = load(q);
+        const bool turb = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
+        return (CENTRED || turb) ? apply_centred(wt, centred(f), extra) : apply_values(wt, f, extra);
+    };
 
     // ---- temperature (RHS_Sat_Turb.cpp:368-386, 409, 435-437, 611-665, 752-759) ----
     {
-        double dpstatdr = 0.0;
+        double dps = 0.0;
         if (K.adiabatic) {
-            dpstatdr = (ldg(io.p_stat + c + plane) - ldg(io.p_stat + c - plane)) * K.inv_2dr * K.to_nd;
+            dps = (ldg(io.p_stat + c + plane) - ldg(io.p_stat + c - plane)) * K.dps_scale;
             const double rho_l = ldg(io.rho_mix + c);
-            if (K.adiabatic_rho && rho_l > 0.0 && isfinite(rho_l))
-                dpstatdr *= in_rcp_range(rho_l) ? K.r_mix * recip_nr(rho_l) : K.r_mix / rho_l;
-        }
-        const double pressure_t = K.coeff_energy_p * (u * (dpdr + dpstatdr) + v * dpdthe * inv_rm
-                                                      + w * dpdphi * inv_rmsinthe);
-        R6 rt;
-        raw6(io.in[ATSAT_F_T], c, plane, kp, dkw, dke, rt);
-        const double diffusion_t = fd.diffusion(rt);
-        double radiation_t = 0.0;
-        if (K.rad_on) {
-            const double rho_f = ldg(io.rho_mix + c);
-            const double rho = (rho_f > 0.0 && isfinite(rho_f)) ? rho_f : K.r_mix;
-            if (rho > 0.0) {
-                radiation_t = K.rad_coupling * ldg(io.q_rad + c) * K.rad_num / (rho * K.rad_den_c);
-                if (!isfinite(radiation_t)) radiation_t = 0.0;
-                else if (radiation_t > 0.5) radiation_t = 0.5;
-                else if (radiation_t < -0.5) radiation_t = -0.5;
+            if (K.adiabatic_rho) {
+                if (in_rcp_range(rho_l)) dps *= K.r_mix * recip_nr(rho_l);
+                else if (rho_l > 0.0 && isfinite(rho_l)) dps *= K.r_mix / rho_l;
             }
         }
-        double precip_t = 0.0;
-        if (K.precip_on) {
-            precip_t = K.precip_coupling * ldg(io.q_precip + c) * K.precip_num * K.precip_den;
-            if (!isfinite(precip_t)) precip_t = 0.0;
-            else if (precip_t > 0.5) precip_t = 0.5;
-            else if (precip_t < -0.5) precip_t = -0.5;
+        double r = K.coeff_energy_p * fma(u, dpr + dps, fma(v, dpth, w * dpph));
+        if (!PLAIN && K.rad_on) {
+            const double rho_f = ldg(io.rho_mix + c);
+            const double rho = (rho_f > 0.0 && isfinite(rho_f)) ? rho_f : K.r_mix;
+            if (rho > 0.0) r += clip_half(K.rad_coupling * ldg(io.q_rad + c) * K.rad_num / (rho * K.rad_den_c));
         }
-        double rhs_t = pressure_t - fd.transport(rt) + diffusion_t * (K.inv_re_pr + nue_t_s);
-        if (K.tmf_on) rhs_t = rhs_t - K.tmf_chem * ldg(io.thermalmassflux + c);
-        rhs_t = rhs_t + radiation_t + precip_t;
-        emit<MODE>(io, sp, K, ATSAT_F_T, c, rhs_t);
+        if (K.precip_on) r += clip_half(K.precip_factor * ldg(io.q_precip + c));
+        if (!PLAIN && K.tmf_on) r -= K.tmf_chem * ldg(io.thermalmassflux + c);
+        emit<MODE>(io, sp, K, ATSAT_F_T, c, tendency(ATSAT_F_T, weights(K.inv_re_pr + nue_t_s, U, V, W, g), r));
     }
 
     // ---- species (RHS_Sat_Turb.cpp:409-431, 457-491, 839-937) ----
-    const double pc = K.precip_coupling;
-#define ATSAT_SPECIES(FID, INV_SC_RE, EXTRA)                                                   \
-    {                                                                                          \
-        R6 r6;                                                                                 \
-        raw6(io.in[FID], c, plane, kp, dkw, dke, r6);                                          \
-        double r = fma(fd.diffusion(r6), (INV_SC_RE) + nue_t_s, (EXTRA) - fd.transport(r6));   \
-        if (K.divu_on) r -= sd * ldg(io.in[FID] + c);                                          \
-        emit<MODE>(io, sp, K, FID, c, r);                                                      \
-    }
-    ATSAT_SPECIES(ATSAT_F_H2O, K.inv_sc_re_h2o, pc * ldg(io.s_precip[0] + c))
-    ATSAT_SPECIES(ATSAT_F_H2O_CLOUD, K.inv_sc_re_h2o, pc * ldg(io.s_precip[1] + c))
-    ATSAT_SPECIES(ATSAT_F_H2O_ICE, K.inv_sc_re_h2o, pc * ldg(io.s_precip[2] + c))
-    ATSAT_SPECIES(ATSAT_F_H2S, K.inv_sc_re_h2s, K.chem * ldg(io.massflux_h2s + c))
-    ATSAT_SPECIES(ATSAT_F_NH3, K.inv_sc_re_nh3, K.chem * ldg(io.massflux_nh3 + c) + pc * ldg(io.s_precip[3] + c))
-    ATSAT_SPECIES(ATSAT_F_NH3_CLOUD, K.inv_sc_re_nh3, pc * ldg(io.s_precip[4] + c))
-    ATSAT_SPECIES(ATSAT_F_NH3_ICE, K.inv_sc_re_nh3, pc * ldg(io.s_precip[5] + c))
-    ATSAT_SPECIES(ATSAT_F_CH4, K.inv_sc_re_ch4, pc * ldg(io.s_precip[6] + c))
-    ATSAT_SPECIES(ATSAT_F_CH4_CLOUD, K.inv_sc_re_ch4, pc * ldg(io.s_precip[7] + c))
-    ATSAT_SPECIES(ATSAT_F_CH4_ICE, K.inv_sc_re_ch4, pc * ldg(io.s_precip[8] + c))
+    auto species = [&](int q, const Wt& wt, double extra) {
+        double r = extra;
+        if (!PLAIN && K.divu_on) r -= sd * ldg(io.in[q] + c);
+        emit<MODE>(io, sp, K, q, c, tendency(q, wt, r));
+    };
+    const double pc = PLAIN ? 1.0 : K.precip_coupling, chem = PLAIN ? 1.0 : K.chem;
+    // fma(1, a, b) is a + b bit for bit
+    Wt wt = weights(K.inv_sc_re_h2o + nue_t_s, U, V, W, g);
+    species(ATSAT_F_H2O, wt, pc * ldg(io.s_precip[0] + c));
+    species(ATSAT_F_H2O_CLOUD, wt, pc * ldg(io.s_precip[1] + c));
+    species(ATSAT_F_H2O_ICE, wt, pc * ldg(io.s_precip[2] + c));
+    if (!K.nh3_as_h2o) wt = weights(K.inv_sc_re_nh3 + nue_t_s, U, V, W, g);
+    species(ATSAT_F_NH3, wt, fma(chem, ldg(io.massflux_nh3 + c), pc * ldg(io.s_precip[3] + c)));
+    species(ATSAT_F_NH3_CLOUD, wt, pc * ldg(io.s_precip[4] + c));
+    species(ATSAT_F_NH3_ICE, wt, pc * ldg(io.s_precip[5] + c));
+    wt = weights(K.inv_sc_re_ch4 + nue_t_s, U, V, W, g);
+    species(ATSAT_F_CH4, wt, pc * ldg(io.s_precip[6] + c));
+    species(ATSAT_F_CH4_CLOUD, wt, pc * ldg(io.s_precip[7] + c));
+    species(ATSAT_F_CH4_ICE, wt, pc * ldg(io.s_precip[8] + c));
+    wt = weights(K.inv_sc_re_h2s + nue_t_s, U, V, W, g);
+    species(ATSAT_F_H2S, wt, chem * ldg(io.massflux_h2s + c));
     // nh4sh carries the flux-limiter correction (RHS_Sat_Turb.cpp:932-937)
-    ATSAT_SPECIES(ATSAT_F_NH4SH, K.inv_sc_re_nh4sh, ldg(io.fluxlim_nh4sh + c) + K.chem * ldg(io.massflux_nh4sh + c))
-#undef ATSAT_SPECIES
+    wt = weights(K.inv_sc_re_nh4sh + nue_t_s, U, V, W, g);
+    species(ATSAT_F_NH4SH, wt, fma(chem, ldg(io.massflux_nh4sh + c), ldg(io.fluxlim_nh4sh + c)));
 
     // ---- k-omega transport (RHS_Sat_Turb.cpp:511-538) ----
     if (K.turb) {
-        {
-            R6 r6;
-            raw6(io.in[ATSAT_F_TKE], c, plane, kp, dkw, dke, r6);
-            const double r = fma(fd.diffusion(r6), K.inv_re + nue_c * K.inv_sig_k,
-                                 ldg(io.tke_source + c) - fd.transport(r6));
-            emit<MODE>(io, sp, K, ATSAT_F_TKE, c, r);
-        }
-        {
-            R6 r6;
-            raw6(io.in[ATSAT_F_DIS], c, plane, kp, dkw, dke, r6);
-            const double r = fma(fd.diffusion(r6), K.inv_re + nue_c * K.inv_sig_w,
-                                 ldg(io.dis_source + c) - fd.transport(r6));
-            emit<MODE>(io, sp, K, ATSAT_F_DIS, c, r);
-        }
+        wt = weights(fma(nue_c, K.inv_sig_k, K.inv_re), U, V, W, g);
+        emit<MODE>(io, sp, K, ATSAT_F_TKE, c, tendency(ATSAT_F_TKE, wt, ldg(io.tke_source + c)));
+        wt = weights(fma(nue_c, K.inv_sig_w, K.inv_re), U, V, W, g);
+        emit<MODE>(io, sp, K, ATSAT_F_DIS, c, tendency(ATSAT_F_DIS, wt, ldg(io.dis_source + c)));
     } else if (MODE == MODE_RHS || (MODE == MODE_FINAL && sp.write_all_rhs)) {
         io.rhs[ATSAT_F_TKE][c] = 0.0;
         io.rhs[ATSAT_F_DIS][c] = 0.0;
@@ -440,11 +456,15 @@ __global__ void __launch_bounds__(256) density_kernel(const KConst K, const doub
 
 cudaError_t launch_rk_stage_fp64(const KConst& kc, const StageIO<double>& io, const StageParams& sp, int mode,
                                  cudaStream_t s) {
-    dim3 block(32, 8);
-    dim3 grid((kc.km + 31) / 32, (kc.jm + 7) / 8, kc.im);
-    if (mode == MODE_RHS) rk_stage_fp64_kernel<MODE_RHS><<<grid, block, 0, s>>>(kc, io, sp);
-    else if (mode == MODE_STAGE) rk_stage_fp64_kernel<MODE_STAGE><<<grid, block, 0, s>>>(kc, io, sp);
-    else rk_stage_fp64_kernel<MODE_FINAL><<<grid, block, 0, s>>>(kc, io, sp);
+    const dim3 block(32, RKS_ROWS), grid((kc.km + 31) / 32, (kc.jm + RKS_ROWS - 1) / RKS_ROWS, kc.im);
+    const bool plain = plain_knobs(kc);
+    auto go = [&](auto kernel) { kernel<<<grid, block, 0, s>>>(kc, io, sp); };
+    if (mode == MODE_RHS) plain ? go(rk_stage_fp64_kernel<MODE_RHS, true, true>) : go(rk_stage_fp64_kernel<MODE_RHS, true, false>);
+    else if (mode == MODE_STAGE)
+        plain ? go(rk_stage_fp64_kernel<MODE_STAGE, false, true>) : go(rk_stage_fp64_kernel<MODE_STAGE, false, false>);
+    else if (sp.write_all_rhs)
+        plain ? go(rk_stage_fp64_kernel<MODE_FINAL, true, true>) : go(rk_stage_fp64_kernel<MODE_FINAL, true, false>);
+    else plain ? go(rk_stage_fp64_kernel<MODE_FINAL, false, true>) : go(rk_stage_fp64_kernel<MODE_FINAL, false, false>);
     return cudaGetLastError();
 }
 
