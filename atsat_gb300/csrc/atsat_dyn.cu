@@ -1048,7 +1048,6 @@ bool variant_available(const atsat_dyn* h, int v) {
     }
 }
 
-int launches_per_stage(const atsat_dyn* h) { return h->variant >= ATSAT_DYN_STAGE_SPLIT ? 2 : 1; }
 
 // The tracer kernel's stream, in the order its consumers read it: the winds' point values (u, [du], v,
 // [dv], w, w's low word, [dw]) and nue; then per tracer field its y_n and increment halo boxes, its
@@ -1070,6 +1069,7 @@ TracerPlan make_plan_tracer(atsat_dyn* h, const MixedIO& io, int mode) {
     add(io.nue, 1);
     for (int q = ATSAT_F_H2O; q < NPROG; q++) {
         const bool turb = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
+        pl.first[q - ATSAT_F_H2O] = n;
         if (turb && !h->kc.turb) continue;
         add(io.yn32[q], 0);
         if (dl) add(io.dl_in[q], 0);
@@ -1091,7 +1091,7 @@ TracerPlan make_plan_tracer(atsat_dyn* h, const MixedIO& io, int mode) {
         if (turb) add(io.acc_turb[q - ATSAT_F_TKE], 1);
         else if (mode == MODE_FINAL) { add(io.dl1[q], 1); add(io.dl2[q], 1); }
     }
-    pl.n_items = n;
+    pl.n_items = pl.first[NPROG - ATSAT_F_H2O] = n;
     return pl;
 }
 
@@ -1234,11 +1234,7 @@ bool march_compact() {
 // waves of the resident blocks (measured best at 41x181x361, where the autotuner picks the same 13 levels).
 int default_march_levels(const atsat_dyn* h) {
     const KConst& K = h->kc;
-    int nsm = 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess || nsm < 1) {
-        cudaGetLastError();
-        nsm = 152;
-    }
+    const int nsm = sm_count();
     const int n_pt = 10 + (K.precip_on ? 1 : 0) + (K.rad_on ? 2 : 0) + (K.tmf_on ? 1 : 0);
     const int per_sm = (march_compact() && n_pt <= 12) ? 3 : 2;
     const int64_t tiles = (int64_t)((K.km - 1 + TILE_K - 1) / TILE_K) * ((K.jm - 4 + TILE_J - 1) / TILE_J);
@@ -1284,6 +1280,12 @@ MarchPlan make_plan_march(atsat_dyn* h, const MixedIO& io, int mode) {
     return pl;
 }
 
+// kernels of one stage without the final combine
+int launches_per_stage(atsat_dyn* h, const MixedIO& io, int mode) {
+    if (h->variant < ATSAT_DYN_STAGE_SPLIT) return 1;
+    return h->variant == ATSAT_DYN_STAGE_MARCH && stage_fusable(h->kf, make_plan_march(h, io, mode), mode) ? 1 : 2;
+}
+
 cudaError_t launch_stage(atsat_dyn* h, const MixedIO& io, const StageParams& sp, int mode) {
     const int v = (mode == MODE_RHS || !variant_available(h, h->variant)) ? ATSAT_DYN_STAGE_DIRECT : h->variant;
     switch (v) {
@@ -1315,6 +1317,7 @@ cudaError_t launch_stage(atsat_dyn* h, const MixedIO& io, const StageParams& sp,
             const TracerPlan pt = make_plan_tracer(h, io, mode);
             if (pt.n_items != tracer_plan_items(mode, io.dl_in[0] != nullptr, h->kc.turb != 0))
                 return cudaErrorInvalidValue;   // the plan and the kernel disagree: never expected
+            if (stage_fusable(h->kf, pm, mode)) return launch_rk_stage_fused(h->maps, h->kf, io, sp, pm, pt, mode, h->stream);
             const cudaError_t e = launch_rk_mom_march(h->maps, h->kf, io, sp, pm, mode, h->stream);
             if (e != cudaSuccess) return e;
             return launch_rk_tracer_tile(h->maps, h->kf, io, sp, pt, mode, h->stream);
@@ -1383,8 +1386,9 @@ int enqueue_rk4_mixed(atsat_dyn* h, bool resident) {
             io.wlo_out = h->wlo_o;
         }
         Timed t(h, ATSAT_K_RK_STAGE);
-        CK(h, launch_stage(h, io, sp, stage == 3 ? MODE_FINAL : MODE_STAGE));
-        h->launches += launches_per_stage(h);
+        const int mode = stage == 3 ? MODE_FINAL : MODE_STAGE;
+        CK(h, launch_stage(h, io, sp, mode));
+        h->launches += launches_per_stage(h, io, mode);
         // the TMA-tiled tracer kernel leaves the final stage's FP64 sum to launch_final_combine
         const int v = variant_available(h, h->variant) ? h->variant : ATSAT_DYN_STAGE_DIRECT;
         if (stage == 3 && (v == ATSAT_DYN_STAGE_SPLIT_TILED || v == ATSAT_DYN_STAGE_TILED2 || v == ATSAT_DYN_STAGE_MARCH))
@@ -1596,6 +1600,19 @@ int enqueue_clamp(atsat_dyn* h, bool resident = false) {
 }
 
 }  // namespace
+
+int atsat::sm_count() {
+    static const int n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
+            cudaGetLastError();
+            v = 152;
+        }
+        return v;
+    }();
+    return n;
+}
 
 extern "C" {
 
@@ -2872,7 +2889,7 @@ int atsat_dyn_autotune(atsat_dyn_t h, int32_t reps, int32_t* chosen, double* ms)
         for (int r = 0; r < 2 + reps; r++) {
             if (r == 2) CK(h, cudaEventRecord(ev[0], h->stream));
             CK(h, launch_stage(h, io, sp, MODE_STAGE));
-            h->launches += launches_per_stage(h);
+            h->launches += launches_per_stage(h, io, MODE_STAGE);
         }
         CK(h, cudaEventRecord(ev[1], h->stream));
         CK(h, cudaEventSynchronize(ev[1]));

@@ -350,6 +350,7 @@ struct TracerPlan {
     int n_items;
     int arr[TRACER_MAX_ITEMS];
     unsigned char kind[TRACER_MAX_ITEMS];
+    int first[NPROG - ATSAT_F_H2O + 1];   // the first item of each tracer field; the last entry: n_items
     unsigned int* err;
     long long wait_limit;          // SM clocks before a consumer's or the producer's slot wait gives up
     int withhold;                  // test hook: the producer leaves the last `withhold` items unissued
@@ -362,6 +363,8 @@ cudaError_t launch_rk_tracer_tile(const TileMaps& maps, const MixedConstF& kf, c
                                   const StageParams& sp, const TracerPlan& plan, int mode, cudaStream_t s);
 cudaError_t launch_rk_mom(const MixedConstF& kf, const MixedIO& io, const StageParams& sp, int mode, cudaStream_t s);
 int tracer_plan_items(int mode, bool has_dl, bool turb);
+int tracer_groups(int64_t tiles);   // field groups (blocks per tile) of the tracer kernel for this many tiles
+int sm_count();                     // SMs of the current device
 // the momentum / temperature equations alone, TMA-tiled (species_divu off)
 cudaError_t launch_rk_mom_tile(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                                const TracerPlan& plan, int mode, cudaStream_t s);
@@ -388,6 +391,12 @@ struct MarchPlan {
 };
 cudaError_t launch_rk_mom_march(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                                 const MarchPlan& plan, int mode, cudaStream_t s);
+
+// an intermediate stage of the march variant as one launch: its momentum blocks and the tracer blocks in one grid;
+// stage_fusable: the plan's rings fit (the compact ones)
+bool stage_fusable(const MixedConstF& kf, const MarchPlan& mp, int mode);
+cudaError_t launch_rk_stage_fused(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
+                                  const MarchPlan& mp, const TracerPlan& tp, int mode, cudaStream_t s);
 
 // standalone pressure-equation solver (poisson.cu)
 struct PoissonSolver;

@@ -1,0 +1,108 @@
+// One launch per RK stage of the march variant: the blocks of the radial-march momentum kernel (rk_march_body.cuh) and
+// those of the TMA-tiled tracer kernel (rk_tracer_body.cuh) in one grid. The two read the same stage input and write
+// different fields, so they need no order between them.
+#include "rk_march_body.cuh"
+#include "rk_tracer_body.cuh"
+
+namespace atsat {
+
+namespace {
+
+static_assert(march::THREADS == tracer::THREADS, "one block size");
+
+struct FusedGrid {
+    int nm, nt;                    // momentum blocks, tracer tiles
+    int nk, nj;
+};
+
+template <int MODE>
+struct Fused {
+    static constexpr bool CMP = MODE == MODE_STAGE;
+    static constexpr size_t SMEM = march::Shape<MODE, CMP>::SMEM > tracer::SMEM_BYTES ? march::Shape<MODE, CMP>::SMEM
+                                                                                      : tracer::SMEM_BYTES;
+};
+
+template <int MODE, bool HAS_DL, int NG>
+__global__ void __launch_bounds__(march::THREADS, Fused<MODE>::CMP ? 3 : 2)
+rk_stage_fused_kernel(const __grid_constant__ CUtensorMap plane, const __grid_constant__ CUtensorMap plane_seam,
+                      const __grid_constant__ CUtensorMap plane_pt, const __grid_constant__ CUtensorMap box,
+                      const __grid_constant__ CUtensorMap box_seam, const __grid_constant__ CUtensorMap box_pt,
+                      const MixedConstF K, const MixedIO io, const StageParams sp, const MarchPlan mp,
+                      const TracerPlan tp, const FusedGrid G) {
+    extern __shared__ __align__(128) float smem[];
+    // momentum blocks first (they are the longer ones), then the tracer tiles, their field groups side by side
+    const bool mom = (int)blockIdx.x < G.nm;
+    const int m = mom ? (int)blockIdx.x : (int)blockIdx.x - G.nm, n = mom ? m : m / NG, g = m - n * NG;
+    const int bx = n % G.nk, r = n / G.nk, by = r % G.nj, bz = r / G.nj;
+    if (mom)
+        march::block<MODE, HAS_DL, Fused<MODE>::CMP>(plane, plane_seam, plane_pt, K, io, sp, mp, smem, bx, by, bz);
+    else
+        tracer::group_block<MODE, HAS_DL, NG>(box, box_seam, box_pt, K, io, sp, tp, smem, bx, by, bz, g);
+}
+
+template <int MODE, bool HAS_DL, int NG>
+cudaError_t launch_groups(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
+                          const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
+    static bool attr = false;
+    constexpr size_t smem = Fused<MODE>::SMEM;
+    if (!attr) {
+        const cudaError_t e = cudaFuncSetAttribute(rk_stage_fused_kernel<MODE, HAS_DL, NG>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
+    auto map = [](const unsigned char* p) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(p); };
+    rk_stage_fused_kernel<MODE, HAS_DL, NG><<<G.nm + G.nt * NG, march::THREADS, smem, s>>>(
+        map(m.plane1), map(m.seam1), map(m.pt1), map(m.main4), map(m.seam4), map(m.pt4), kf, io, sp, mp, tp, G);
+    return cudaGetLastError();
+}
+
+template <int MODE, bool HAS_DL>
+cudaError_t launch_one(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
+                       const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
+    switch (tracer_groups(G.nt)) {
+        case 13: return launch_groups<MODE, HAS_DL, 13>(m, kf, io, sp, mp, tp, G, s);
+        case 4: return launch_groups<MODE, HAS_DL, 4>(m, kf, io, sp, mp, tp, G, s);
+        default: return launch_groups<MODE, HAS_DL, 1>(m, kf, io, sp, mp, tp, G, s);
+    }
+}
+
+// blocks of the momentum kernel and tiles of the tracer kernel
+FusedGrid fused_grid(int im, int jm, int km, int levels) {
+    FusedGrid G{};
+    G.nk = (km - 1 + TILE_K - 1) / TILE_K;
+    G.nj = (jm - 4 + TILE_J - 1) / TILE_J;
+    if (G.nk <= 0 || G.nj <= 0 || im < 3) return G;
+    G.nm = G.nk * G.nj * ((im - 2 + levels - 1) / levels);
+    G.nt = G.nk * G.nj * ((im - 2 + TTILE_I - 1) / TTILE_I);
+    return G;
+}
+
+}  // namespace
+
+// Up to four waves of resident blocks (three per SM) the stage's two kernels are short enough that their launch and
+// their thin last waves show: one launch takes two iterations at 10x20x36 from 275 to 241 us, 21x60x121 444 -> 422,
+// 21x91x181 608 -> 586, 31x121x241 1149 -> 1122. Beyond, a lone run still gains (41x181x361 replayed 2623 -> 2579 us,
+// 61x271x541 8001 -> 7798), but handles that run concurrently fill those waves with each other's blocks already and
+// lose (three replaying in turn at 41x181x361 2489 -> 2526 us, 81x361x721 18400 -> 18548): the launches stay apart.
+// Interleaving the momentum blocks with the tracer blocks, so that both kinds share an SM, is slower the finer it is
+// (every 3rd block: 2755 us, every 4th: 2820): the two instruction streams evict each other.
+bool stage_fusable(const MixedConstF& kf, const MarchPlan& mp, int mode) {
+    if (mode != MODE_STAGE || !mp.compact || mp.n_pt > march::Shape<MODE_STAGE, true>::NPT || mp.levels < 1) return false;
+    const FusedGrid G = fused_grid(kf.im, kf.jm, kf.km, mp.levels);
+    return G.nm + G.nt <= 4 * 3 * sm_count();
+}
+
+cudaError_t launch_rk_stage_fused(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
+                                  const MarchPlan& mp, const TracerPlan& tp, int mode, cudaStream_t s) {
+    const bool has_dl = io.dl_in[0] != nullptr;
+    if (!stage_fusable(kf, mp, mode) || kf.divu_on || kf.fsz_over_int || mp.n_halo != (has_dl ? 9 : 5) ||
+        mp.n_pt < march::N_PT_FIXED || tp.n_items > TRACER_MAX_ITEMS || mp.withhold < 0)
+        return cudaErrorInvalidValue;
+    const FusedGrid G = fused_grid(kf.im, kf.jm, kf.km, mp.levels);
+    if (G.nm + G.nt == 0) return cudaSuccess;
+    return has_dl ? launch_one<MODE_STAGE, true>(maps, kf, io, sp, mp, tp, G, s)
+                  : launch_one<MODE_STAGE, false>(maps, kf, io, sp, mp, tp, G, s);
+}
+
+}  // namespace atsat
