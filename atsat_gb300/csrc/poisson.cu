@@ -26,10 +26,13 @@
 #include <omp.h>
 
 #include "dyn_common.cuh"
+#include "poisson_spectral.cuh"
 
 namespace atsat {
 
 namespace {
+
+using namespace spectral;
 
 // ---- stencil helpers over the pitched layout ----
 template <typename T>
@@ -507,43 +510,56 @@ __global__ void unpack_kernel(const KConst K, T* __restrict__ dst, const T* __re
     dst[c + 2 * m + ((i + j + 1) & 1)] = s1[o];
 }
 
+// Sums over the interior for the norms and means: a thread adds RES_LEVELS levels of its column before the warp and
+// block reductions, whose FP64 additions otherwise outnumber the cell's own (GB300 issues two FP64 operations per SM
+// per cycle): residual 120 -> 60 us, sum 37 -> 13 us at 41x181x361 with eight levels.
+constexpr int RES_LEVELS = 8;
+
+__device__ __forceinline__ void block_add(double v, double* out) {
+    __shared__ double s[8];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) s[threadIdx.y] = v;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        double a = 0.0;
+        for (int q = 0; q < 8; q++) a += s[q];
+        atomicAdd(out, a);
+    }
+    __syncthreads();
+}
+
 // r = f - L p on the interior P cells, in FP64 (p FP64), with an FP32 copy of r and the sums
-// sum r^2 and sum f^2 (sq[0], sq[1])
+// sum r^2 (sq[0]) and, where asked (`norm_f`), sum f^2 (sq[1])
 __global__ void __launch_bounds__(256) residual_kernel(const KConst K, const ColGeo* __restrict__ geo,
                                                        const double* __restrict__ f, const double* __restrict__ p,
                                                        double* __restrict__ r, float* __restrict__ r32,
-                                                       double* __restrict__ sq) {
+                                                       double* __restrict__ sq, int norm_f) {
     const int k = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * 8 + threadIdx.y;
-    const int i = blockIdx.z;
+    const int i0 = 1 + blockIdx.z * RES_LEVELS, i1 = min(i0 + RES_LEVELS, K.im - 1);
     double rr = 0.0, ff = 0.0;
-    if (k <= K.km - 2 && j >= 1 && j <= K.jm - 2 && i >= 1 && i <= K.im - 2) {
-        const int64_t c = ((int64_t)i * K.jm + j) * K.kp + k;
+    if (k <= K.km - 2 && j >= 1 && j <= K.jm - 2) {
         const int kw = (k == 0) ? K.km - 2 : k - 1, ke = (k == K.km - 2) ? 0 : k + 1;
-        const ColGeo* g = geo + ((int64_t)i * K.jm + j);
-        const double lp = (p[c + K.plane] + p[c - K.plane]) * __ldg(&g->p_num1)
-                        + (p[c + K.kp] + p[c - K.kp]) * __ldg(&g->p_num2)
-                        + (p[c - k + ke] + p[c - k + kw]) * __ldg(&g->p_num3) - __ldg(&g->p_den) * p[c];
-        const double fc = f[c];
-        const double x = fc - lp;
-        r[c] = x;
-        if (r32) r32[c] = d2f(x);
-        rr = x * x;
-        ff = fc * fc;
+        int64_t c = ((int64_t)i0 * K.jm + j) * K.kp + k;
+        double pm = p[c - K.plane], p0 = p[c];
+#pragma unroll 4
+        for (int i = i0; i < i1; i++, c += K.plane) {
+            const ColGeo* g = geo + ((int64_t)i * K.jm + j);
+            const double pp = p[c + K.plane], fc = f[c];
+            double x = fma(__ldg(&g->p_den), p0, fc);
+            x = fma(-__ldg(&g->p_num1), pp + pm, x);
+            x = fma(-__ldg(&g->p_num2), p[c + K.kp] + p[c - K.kp], x);
+            x = fma(-__ldg(&g->p_num3), p[c - k + ke] + p[c - k + kw], x);
+            r[c] = x;
+            if (r32) r32[c] = d2f(x);
+            rr = fma(x, x, rr);
+            if (norm_f) ff = fma(fc, fc, ff);
+            pm = p0;
+            p0 = pp;
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        rr += __shfl_down_sync(0xffffffffu, rr, o);
-        ff += __shfl_down_sync(0xffffffffu, ff, o);
-    }
-    __shared__ double s[2][8];
-    if (threadIdx.x == 0) { s[0][threadIdx.y] = rr; s[1][threadIdx.y] = ff; }
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        double a = 0.0, b = 0.0;
-        for (int q = 0; q < 8; q++) { a += s[0][q]; b += s[1][q]; }
-        atomicAdd(sq, a);
-        atomicAdd(sq + 1, b);
-    }
+    block_add(rr, sq);
+    if (norm_f) block_add(ff, sq + 1);
 }
 
 // p64 += e32 on the interior P cells
@@ -568,23 +584,17 @@ __global__ void convert_kernel(const KConst K, To* __restrict__ out, const Ti* _
 }
 
 // sum of p over the interior P cells (for the zero-mean normalisation)
-template <typename T>
-__global__ void __launch_bounds__(256) sum_kernel(const KConst K, const T* __restrict__ p, double* __restrict__ out) {
+__global__ void __launch_bounds__(256) sum_kernel(const KConst K, const double* __restrict__ p, double* __restrict__ out) {
     const int k = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * 8 + threadIdx.y;
-    const int i = blockIdx.z;
+    const int i0 = 1 + blockIdx.z * RES_LEVELS, i1 = min(i0 + RES_LEVELS, K.im - 1);
     double v = 0.0;
-    if (k <= K.km - 2 && j >= 1 && j <= K.jm - 2 && i >= 1 && i <= K.im - 2)
-        v = (double)p[((int64_t)i * K.jm + j) * K.kp + k];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    __shared__ double s[8];
-    if (threadIdx.x == 0) s[threadIdx.y] = v;
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        double a = 0.0;
-        for (int q = 0; q < 8; q++) a += s[q];
-        atomicAdd(out, a);
+    if (k <= K.km - 2 && j >= 1 && j <= K.jm - 2) {
+        int64_t c = ((int64_t)i0 * K.jm + j) * K.kp + k;
+#pragma unroll 4
+        for (int i = i0; i < i1; i++, c += K.plane) v += p[c];
     }
+    block_add(v, out);
 }
 
 template <typename T>
@@ -597,138 +607,10 @@ __global__ void shift_kernel(const KConst K, T* __restrict__ p, const double* __
     p[c] = (T)((double)p[c] - sum[0] * inv_n);
 }
 
-// ---- spectral solve ----
-// spec layout: [(m * 2 + part) * NJ + jj] * NI + ii, part 0 = cosine, 1 = sine coefficients
-struct Spec {
-    int n, M, NI, NJ;     // ring length km-1, modes n/2+1, radial and polar unknowns
-};
-
-template <typename T>
-__global__ void dft_fwd_kernel(const KConst K, const Spec S, const T* __restrict__ x, const T* __restrict__ tw,
-                               T* __restrict__ spec) {
-    extern __shared__ __align__(16) unsigned char dsm[];
-    T* row = reinterpret_cast<T*>(dsm);             // n
-    T* tc = row + S.n;                              // cos table, n
-    T* ts = tc + S.n;                               // sin table, n
-    const int ii = blockIdx.x, jj = blockIdx.y;
-    const int i = ii + 1, j = jj + 1;
-    const int64_t base = ((int64_t)i * K.jm + j) * K.kp;
-    for (int k = threadIdx.x; k < S.n; k += blockDim.x) {
-        row[k] = x[base + k];
-        tc[k] = tw[k];
-        ts[k] = tw[S.n + k];
-    }
-    __syncthreads();
-    for (int m = threadIdx.x; m < S.M; m += blockDim.x) {
-        T a = 0, b = 0;
-        int idx = 0;
-        for (int k = 0; k < S.n; k++) {
-            a += row[k] * tc[idx];
-            b += row[k] * ts[idx];
-            idx += m;
-            if (idx >= S.n) idx -= S.n;
-        }
-        spec[((int64_t)(m * 2 + 0) * S.NJ + jj) * S.NI + ii] = a;
-        spec[((int64_t)(m * 2 + 1) * S.NJ + jj) * S.NI + ii] = b;
-    }
-}
-
-template <typename T>
-__global__ void dft_inv_kernel(const KConst K, const Spec S, const T* __restrict__ spec, const T* __restrict__ tw,
-                               T* __restrict__ x) {
-    extern __shared__ __align__(16) unsigned char dsm[];
-    T* a = reinterpret_cast<T*>(dsm);               // M
-    T* b = a + S.M;                                 // M
-    T* tc = b + S.M;                                // n
-    T* ts = tc + S.n;                               // n
-    const int ii = blockIdx.x, jj = blockIdx.y;
-    const int i = ii + 1, j = jj + 1;
-    for (int m = threadIdx.x; m < S.M; m += blockDim.x) {
-        a[m] = spec[((int64_t)(m * 2 + 0) * S.NJ + jj) * S.NI + ii];
-        b[m] = spec[((int64_t)(m * 2 + 1) * S.NJ + jj) * S.NI + ii];
-    }
-    for (int k = threadIdx.x; k < S.n; k += blockDim.x) { tc[k] = tw[k]; ts[k] = tw[S.n + k]; }
-    __syncthreads();
-    const bool even = (S.n & 1) == 0;
-    const int mtop = even ? S.M - 1 : S.M;          // modes with a conjugate partner: 1 .. mtop-1
-    const T inv_n = (T)1 / (T)S.n;
-    const int64_t base = ((int64_t)i * K.jm + j) * K.kp;
-    for (int k = threadIdx.x; k < S.n; k += blockDim.x) {
-        T s = 0;
-        int idx = k;                                  // (m k) mod n for m = 1
-        for (int m = 1; m < mtop; m++) {
-            s += a[m] * tc[idx] + b[m] * ts[idx];
-            idx += k;
-            if (idx >= S.n) idx -= S.n;
-        }
-        T v = a[0] + (T)2 * s;
-        if (even) v += a[S.M - 1] * ((k & 1) ? (T)-1 : (T)1);
-        x[base + k] = v * inv_n;
-    }
-}
-
-// Block Thomas for one (mode, part): g_j = f_j - b_j * (W_{j-1} g_{j-1}); x_NJ = W_NJ g_NJ;
-// x_j = W_j (g_j - c_j * x_{j+1}). W is column-major per block; b, c are the theta couplings (mode
-// independent); the zero mode pins the cell (1, 1) (its row of D_1 is the identity, its c is 0, f = 0).
-template <typename T>
-__global__ void bt_solve_kernel(const Spec S, const T* __restrict__ W, const double* __restrict__ bvec,
-                                const double* __restrict__ cvec, T* __restrict__ spec) {
-    const int m = blockIdx.x >> 1, part = blockIdx.x & 1;
-    const bool even = (S.n & 1) == 0;
-    if (part == 1 && (m == 0 || (even && m == S.M - 1))) return;   // sine part identically zero
-    const int NI = S.NI, NJ = S.NJ;
-    extern __shared__ __align__(16) unsigned char dsm[];
-    T* g = reinterpret_cast<T*>(dsm);   // NI
-    T* t = g + NI;                      // NI
-    T* f = spec + (int64_t)(m * 2 + part) * NJ * NI;
-    const T* Wm = W + (int64_t)m * NJ * NI * NI;
-    const int r = threadIdx.x;
-    const bool pin = (m == 0 && part == 0);
-    // forward
-    if (r < NI) g[r] = (pin && r == 0) ? (T)0 : f[r];
-    __syncthreads();
-    for (int jj = 1; jj < NJ; jj++) {
-        if (r < NI) {
-            const T* Wp = Wm + (int64_t)(jj - 1) * NI * NI;
-            T acc = 0;
-            for (int c = 0; c < NI; c++) acc += Wp[(int64_t)c * NI + r] * g[c];
-            t[r] = f[(int64_t)jj * NI + r] - (T)bvec[jj * NI + r] * acc;
-        }
-        __syncthreads();
-        if (r < NI) {
-            f[(int64_t)(jj - 1) * NI + r] = g[r];     // keep g_{j-1} for the backward pass
-            g[r] = t[r];
-        }
-        __syncthreads();
-    }
-    // backward: x_NJ = W_NJ g_NJ
-    {
-        const T* Wp = Wm + (int64_t)(NJ - 1) * NI * NI;
-        T acc = 0;
-        if (r < NI) for (int c = 0; c < NI; c++) acc += Wp[(int64_t)c * NI + r] * g[c];
-        __syncthreads();
-        if (r < NI) { g[r] = acc; f[(int64_t)(NJ - 1) * NI + r] = acc; }
-        __syncthreads();
-    }
-    for (int jj = NJ - 2; jj >= 0; jj--) {
-        if (r < NI) {
-            T cc = (T)cvec[jj * NI + r];
-            if (pin && jj == 0 && r == 0) cc = 0;
-            t[r] = f[(int64_t)jj * NI + r] - cc * g[r];
-        }
-        __syncthreads();
-        if (r < NI) {
-            const T* Wp = Wm + (int64_t)jj * NI * NI;
-            T acc = 0;
-            for (int c = 0; c < NI; c++) acc += Wp[(int64_t)c * NI + r] * t[c];
-            g[r] = acc;
-            f[(int64_t)jj * NI + r] = acc;
-        }
-        __syncthreads();
-    }
-}
-
 dim3 cell_grid(const KConst& K) { return dim3((K.km + 31) / 32, (K.jm + 7) / 8, K.im); }
+dim3 level_grid(const KConst& K) {
+    return dim3((K.km + 31) / 32, (K.jm + 7) / 8, (K.im - 2 + RES_LEVELS - 1) / RES_LEVELS);
+}
 
 // Gauss-Jordan inverse with partial pivoting of an n x n row-major matrix (in place into inv)
 bool invert(int n, std::vector<double>& a, std::vector<double>& inv) {
@@ -764,6 +646,10 @@ bool invert(int n, std::vector<double>& a, std::vector<double>& inv) {
 struct PoissonSolver {
     KConst K{};
     Spec S{};
+    // the transforms' stages with the row pairs per block of each precision
+    bool spectral64 = false, spectral32 = false;   // the ring fits the transforms
+    FftPlan fft64{}, fft32{};
+    BtLayout bt64{}, bt32{};
     cudaStream_t stream = nullptr;
     const ColGeo* geo = nullptr;          // device column geometry (owned by the handle)
     std::vector<double> num1, num2, num3, den;   // host, [jj * NI + ii]
@@ -775,6 +661,8 @@ struct PoissonSolver {
     std::vector<double> ynull;            // left null vector of the zero mode, [jj * NI + ii]
     void* block = nullptr;
     int64_t n_interior = 0;
+    double* host_sq = nullptr;            // page-locked: the residual's sums as the host reads them
+    double norm_f = -1.0;                 // sum f^2 of the running solve (< 0: not summed yet)
     // the checkerboard-packed SOR (even rings only): per precision both colours of p and f, the column
     // weights, the grid barrier's words, and the cooperative launch's grid
     int kh = 0;
@@ -800,6 +688,24 @@ struct PoissonSolver {
 };
 
 namespace {
+
+// The transform's blocks: a few row pairs (warps) each, so that they even out over the SMs and the stores of a mode still
+// fill a sector or more (four FP32 pairs are 64 bytes, two FP64 pairs too): FP64 at 21x91x181, 855 pairs, 53 us with
+// eight pairs per block, 25 with two; FP32 at 41x181x361 17.0 with eight, 15.6 with four. False: the ring length is
+// beyond one row pair in shared memory.
+template <typename T>
+bool plan_spectral(const Spec& S, FftPlan& F) {
+    fft_plan(S.n, F);
+    for (F.warps = sizeof(T) == 4 ? 4 : 2; F.warps > 1 && fft_smem<T>(F, S.n) > 100 * 1024; F.warps--) {}
+    if (fft_smem<T>(F, S.n) > 220 * 1024) return false;
+    auto allow = [](const void* fn) {      // the limit is the kernel's, shared by every handle
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) == cudaSuccess;
+    };
+    bool ok = allow((const void*)fft_fwd_kernel<T>) && allow((const void*)fft_inv_kernel<T, T, false>);
+    if constexpr (sizeof(T) == 4) ok = ok && allow((const void*)fft_inv_kernel<T, double, true>);
+    if (!ok) cudaGetLastError();
+    return ok;
+}
 
 // D_j(m) as a dense NI x NI row-major matrix; `pin`: the zero mode's cell (1, 1) becomes x = 0
 void build_D(const PoissonSolver& P, int m, int jj, std::vector<double>& D, bool pin = true) {
@@ -893,6 +799,11 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
     S.NI = kc.im - 2;
     S.NJ = kc.jm - 2;
     if (S.NI > 1024) { *err = "poisson: im too large"; delete P; return nullptr; }
+    S.RS = (2 * S.NI + 3) & ~3;
+    P->spectral64 = plan_spectral<double>(S, P->fft64);
+    P->spectral32 = plan_spectral<float>(S, P->fft32);
+    P->bt64 = bt_layout<double>(S.NI);
+    P->bt32 = bt_layout<float>(S.NI);
     const int NI = S.NI, NJ = S.NJ;
     P->n_interior = (int64_t)NI * NJ * S.n;
     const size_t nc = (size_t)NI * NJ;
@@ -990,14 +901,14 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
     }
     // device buffers
     const size_t fsz = (size_t)kc.fsz;
-    const size_t nspec = (size_t)S.M * 2 * nc;
-    const size_t nW = (size_t)S.M * NJ * blk;
+    const size_t nspec = (size_t)S.M * NJ * S.RS;
+    const size_t nblk = (size_t)S.M * NJ, nW64 = nblk * P->bt64.stride, nW32 = nblk * P->bt32.stride;
     size_t bytes = 0;
     auto take = [&](size_t b) { size_t o = bytes; bytes += (b + 255) & ~size_t(255); return o; };
     const size_t o_f = take(fsz * 8), o_p = take(fsz * 8), o_r = take(fsz * 8), o_sq = take(64);
-    const size_t o_W64 = take(nW * 8), o_s64 = take(nspec * 8), o_b = take(nc * 8), o_c = take(nc * 8);
+    const size_t o_W64 = take(nW64 * 8), o_s64 = take(nspec * 8), o_b = take(nc * 8), o_c = take(nc * 8);
     const size_t o_tw64 = take((size_t)2 * S.n * 8), o_p32 = take(fsz * 4), o_r32 = take(fsz * 4), o_e32 = take(fsz * 4);
-    const size_t o_W32 = take(nW * 4), o_s32 = take(nspec * 4), o_tw32 = take((size_t)2 * S.n * 4);
+    const size_t o_W32 = take(nW32 * 4), o_s32 = take(nspec * 4), o_tw32 = take((size_t)2 * S.n * 4);
     // the packed SOR's arrays (even rings): p and f of both colours in each precision, the column weights
     P->packed = (S.n % 2) == 0;
     P->kh = ((S.n / 2 + 31) / 32) * 32;
@@ -1008,6 +919,11 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
     const size_t o_tiles = take(P->packed ? TB_MAX_TILES * sizeof(TbTile) : 0);
     cudaError_t e = cudaMalloc(&P->block, bytes);
     if (e != cudaSuccess) { *err = std::string("poisson: cudaMalloc: ") + cudaGetErrorString(e); delete P; return nullptr; }
+    if ((e = cudaHostAlloc(&P->host_sq, 64, cudaHostAllocDefault)) != cudaSuccess) {
+        *err = std::string("poisson: cudaHostAlloc: ") + cudaGetErrorString(e);
+        poisson_destroy(P);
+        return nullptr;
+    }
     if ((e = cudaEventCreate(&P->sev[0])) != cudaSuccess || (e = cudaEventCreate(&P->sev[1])) != cudaSuccess) {
         *err = std::string("poisson: cudaEventCreate: ") + cudaGetErrorString(e);
         poisson_destroy(P);
@@ -1072,8 +988,17 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
             if (!(ev && std::atoi(ev) == 1)) plan_tb(P, 2, dev, nsm);
         }
     }
-    std::vector<float> W32(nW);
-    for (size_t q = 0; q < nW; q++) W32[q] = (float)W[q];
+    // the pivot blocks in the mode solve's layout
+    std::vector<double> W64(nW64, 0.0);
+    std::vector<float> W32(nW32, 0.0f);
+#pragma omp parallel for schedule(static)
+    for (size_t b = 0; b < nblk; b++)
+        for (int c = 0; c < NI; c++)
+            for (int r = 0; r < NI; r++) {
+                const double w = W[b * blk + (size_t)c * NI + r];
+                W64[b * P->bt64.stride + bt_place<double>(P->bt64, NI, r, c)] = w;
+                W32[b * P->bt32.stride + bt_place<float>(P->bt32, NI, r, c)] = (float)w;
+            }
     std::vector<double> tw(2 * S.n);
     std::vector<float> tw32(2 * S.n);
     for (int k = 0; k < S.n; k++) {
@@ -1082,8 +1007,8 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
     }
     for (int q = 0; q < 2 * S.n; q++) tw32[q] = (float)tw[q];
     if ((e = cudaMemsetAsync(P->block, 0, bytes, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(P->W64, W.data(), nW * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(P->W32, W32.data(), nW * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(P->W64, W64.data(), nW64 * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(P->W32, W32.data(), nW32 * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(P->bvec_d, P->bvec.data(), nc * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(P->cvec_d, P->cvec.data(), nc * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(P->tw64, tw.data(), 2 * S.n * 8, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
@@ -1108,6 +1033,7 @@ void poisson_destroy(PoissonSolver* P) {
     for (cudaEvent_t& ev : P->sev)
         if (ev) cudaEventDestroy(ev);
     if (P->block) cudaFree(P->block);
+    if (P->host_sq) cudaFreeHost(P->host_sq);
     delete P;
 }
 
@@ -1216,33 +1142,38 @@ cudaError_t sor_packed_run(PoissonSolver* P, const T* f, T* p, T w, int nsweeps,
     return herr ? cudaErrorLaunchTimeout : cudaSuccess;
 }
 
-// x = L^-1 rhs by the spectral block solve in precision T (rhs and x pitched; x may alias rhs)
-template <typename T>
-cudaError_t direct(PoissonSolver* P, const T* rhs, T* x, T* spec, const T* W, const T* tw) {
+template <typename T> const FftPlan& fft_of(PoissonSolver* P);
+template <> const FftPlan& fft_of<double>(PoissonSolver* P) { return P->fft64; }
+template <> const FftPlan& fft_of<float>(PoissonSolver* P) { return P->fft32; }
+
+// x = L^-1 rhs, of zero interior mean, by the spectral block solve in precision T on the interior (rhs and x pitched; x
+// may alias rhs); ADD: x += L^-1 rhs in FP64. The boundary planes are the caller's.
+template <typename T, typename To, bool ADD>
+cudaError_t direct(PoissonSolver* P, const T* rhs, To* x, T* spec, const T* W, const T* tw) {
     const KConst& K = P->K;
     const Spec& S = P->S;
-    const dim3 rows(S.NI, S.NJ);
-    dft_fwd_kernel<T><<<rows, 128, (size_t)3 * S.n * sizeof(T), P->stream>>>(K, S, rhs, tw, spec);
-    const int thr = ((S.NI + 31) / 32) * 32;
-    bt_solve_kernel<T><<<2 * S.M, thr, (size_t)2 * S.NI * sizeof(T), P->stream>>>(S, W, P->bvec_d, P->cvec_d, spec);
-    dft_inv_kernel<T><<<rows, 128, (size_t)(2 * S.M + 2 * S.n) * sizeof(T), P->stream>>>(K, S, spec, tw, x);
-    // zero interior mean (the zero mode's pinned constant), then the boundary planes
-    cudaMemsetAsync(P->sq + 2, 0, sizeof(double), P->stream);
-    sum_kernel<T><<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, x, P->sq + 2);
-    shift_kernel<T><<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, x, P->sq + 2, 1.0 / (double)P->n_interior);
-    return fold(P, x);
+    const FftPlan& F = fft_of<T>(P);
+    if (!(sizeof(T) == 8 ? P->spectral64 : P->spectral32)) return cudaErrorInvalidValue;
+    const dim3 rows(((S.NI + 1) / 2 + F.warps - 1) / F.warps, S.NJ);
+    fft_fwd_kernel<T><<<rows, 32 * F.warps, fft_smem<T>(F, S.n), P->stream>>>(K, S, F, rhs, tw, spec);
+    const cudaError_t e = launch_bt<T>(S, sizeof(T) == 8 ? P->bt64 : P->bt32, W, P->bvec_d, P->cvec_d, spec, P->stream);
+    if (e != cudaSuccess) return e;
+    fft_inv_kernel<T, To, ADD><<<rows, 32 * F.warps, fft_smem<T>(F, S.n), P->stream>>>(K, S, F, spec, tw, x);
+    return cudaGetLastError();
 }
 
-// ||f - L p|| / ||f|| with r64 (and r32) written
+// ||f - L p|| / ||f|| with r64 (and r32) written; ||f|| is summed on the first call of a solve (P->norm_f < 0).
 cudaError_t residual(PoissonSolver* P, double* rel) {
     const KConst& K = P->K;
     cudaError_t e = cudaMemsetAsync(P->sq, 0, 2 * sizeof(double), P->stream);
     if (e != cudaSuccess) return e;
-    residual_kernel<<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->geo, P->f64, P->p64, P->r64, P->r32, P->sq);
-    double h[2];
-    if ((e = cudaMemcpyAsync(h, P->sq, sizeof(h), cudaMemcpyDeviceToHost, P->stream)) != cudaSuccess) return e;
+    const bool first = P->norm_f < 0.0;
+    residual_kernel<<<level_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->geo, P->f64, P->p64, P->r64, P->r32, P->sq, first);
+    double* h = P->host_sq;
+    if ((e = cudaMemcpyAsync(h, P->sq, 2 * sizeof(double), cudaMemcpyDeviceToHost, P->stream)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(P->stream)) != cudaSuccess) return e;
-    *rel = h[1] > 0.0 ? std::sqrt(h[0] / h[1]) : std::sqrt(h[0]);
+    if (first) P->norm_f = h[1];
+    *rel = P->norm_f > 0.0 ? std::sqrt(h[0] / P->norm_f) : std::sqrt(h[0]);
     return cudaSuccess;
 }
 
@@ -1261,7 +1192,7 @@ cudaError_t poisson_run(PoissonSolver* P, int method, double tol, int max_iter, 
     if (e != cudaSuccess) return e;
     const KConst& K = P->K;
     if ((e = cudaMemsetAsync(P->sq + 2, 0, sizeof(double), P->stream)) != cudaSuccess) return e;
-    sum_kernel<double><<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->p64, P->sq + 2);
+    sum_kernel<<<level_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->p64, P->sq + 2);
     shift_kernel<double><<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->p64, P->sq + 2, 1.0 / (double)P->n_interior);
     if ((e = fold<double>(P, P->p64)) != cudaSuccess) return e;
     return cudaStreamSynchronize(P->stream);
@@ -1275,17 +1206,18 @@ cudaError_t poisson_run_inner(PoissonSolver* P, int method, double tol, int max_
     *inner_total = 0;
     P->spp = 0;
     P->sweep_ms = 0.0;
+    P->norm_f = -1.0;
     const size_t fsz = (size_t)K.fsz;
     if (method == 3) {
-        e = direct<double>(P, P->f64, P->p64, P->spec64, P->W64, P->tw64);
-        if (e != cudaSuccess) return e;
+        e = direct<double, double, false>(P, P->f64, P->p64, P->spec64, P->W64, P->tw64);
+        if (e != cudaSuccess || (e = fold<double>(P, P->p64)) != cudaSuccess) return e;
         *iters = 1;
         return residual(P, rel);
     }
     if (method == 4) {
         convert_kernel<float, double><<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->r32, P->f64);
-        e = direct<float>(P, P->r32, P->p32, P->spec32, P->W32, P->tw32);
-        if (e != cudaSuccess) return e;
+        e = direct<float, float, false>(P, P->r32, P->p32, P->spec32, P->W32, P->tw32);
+        if (e != cudaSuccess || (e = fold<float>(P, P->p32)) != cudaSuccess) return e;
         convert_kernel<double, float><<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->p64, P->p32);
         *iters = 1;
         return residual(P, rel);
@@ -1331,7 +1263,7 @@ cudaError_t poisson_run_inner(PoissonSolver* P, int method, double tol, int max_
         if ((e = residual(P, rel)) != cudaSuccess) return e;
         if (*rel <= tol || it == max_iter) break;
         if (method == 5) {
-            e = direct<float>(P, P->r32, P->e32, P->spec32, P->W32, P->tw32);
+            e = direct<float, double, true>(P, P->r32, P->p64, P->spec32, P->W32, P->tw32);
             *inner_total += 1;
         } else {
             if ((e = cudaMemsetAsync(P->e32, 0, fsz * 4, P->stream)) != cudaSuccess) return e;
@@ -1341,7 +1273,7 @@ cudaError_t poisson_run_inner(PoissonSolver* P, int method, double tol, int max_
             *inner_total += inner;
         }
         if (e != cudaSuccess) return e;
-        axpy_kernel<<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->p64, P->e32);
+        if (method != 5) axpy_kernel<<<cell_grid(K), dim3(32, 8), 0, P->stream>>>(K, P->p64, P->e32);
         if ((e = fold<double>(P, P->p64)) != cudaSuccess) return e;
         *iters = it + 1;
     }
