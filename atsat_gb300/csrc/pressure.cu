@@ -67,10 +67,16 @@ __global__ void prep_seam_kernel(const KConst K, double* const* __restrict__ six
     f[c + K.km - 1] = f[c];
 }
 
+// The projection source with its clamp and lc_old. Bound by the FP64 pipe (two operations per SM per cycle): 16
+// operations per cell -- the scales of each difference are one product from the column table, the clamp's compare runs on
+// the integer pipe (positive doubles order as integers, finiteness is an exponent test), lc_old's three second
+// differences accumulate into div by fma. LEGACY: the source div(aux - rhs); INCR: lc_old is added. They are compiled in
+// because an instruction predicated off still takes its slot of that pipe: 98 -> 88 us at 41x181x361
+// (the operations alone are 64).
+template <bool LEGACY, bool INCR>
 __global__ void __launch_bounds__(256) press_source_kernel(
         const KConst K, const ColGeo* __restrict__ geo, const double* __restrict__ su,
-        const double* __restrict__ sv, const double* __restrict__ sw, const double* __restrict__ aux_u,
-        const double* __restrict__ aux_v, const double* __restrict__ aux_w, const double* __restrict__ rhs_u,
+        const double* __restrict__ sv, const double* __restrict__ sw, const double* __restrict__ rhs_u,
         const double* __restrict__ rhs_v, const double* __restrict__ rhs_w, const double* __restrict__ p,
         double* __restrict__ src, unsigned long long* __restrict__ nclamp) {
     const int k = blockIdx.x * 32 + threadIdx.x;
@@ -84,16 +90,13 @@ __global__ void __launch_bounds__(256) press_source_kernel(
         const int ke = (k == K.km - 2) ? 0 : k + 1;
         const int64_t cw = c - k + kw, ce = c - k + ke;
         const ColGeo* g = geo + ((int64_t)i * K.jm + j);
-        // GB300 issues two FP64 operations per SM per cycle: the scales of each difference are one
-        // product from the column table, the clamp one compare (finiteness is an exponent test), and
-        // lc_old's three second differences accumulate into div by fma (17 operations per cell)
         double dr_, dthe_, dphi_;
-        if (K.press_src == 0) {     // legacy div(aux - rhs), PressureSolver.h:373-381
-            dr_ = (ldg(aux_u + c + P) - ldg(aux_u + c - P)) - (ldg(rhs_u + c + P) - ldg(rhs_u + c - P));
-            dthe_ = (ldg(aux_v + c + kp) - ldg(aux_v + c - kp)) - (ldg(rhs_v + c + kp) - ldg(rhs_v + c - kp));
-            dphi_ = (ldg(aux_w + ce) - ldg(aux_w + cw)) - (ldg(rhs_w + ce) - ldg(rhs_w + cw));
+        if (LEGACY) {               // div(aux - rhs), PressureSolver.h:373-381; su, sv, sw are the aux fields
+            dr_ = (ldg(su + c + P) - ldg(su + c - P)) - (ldg(rhs_u + c + P) - ldg(rhs_u + c - P));
+            dthe_ = (ldg(sv + c + kp) - ldg(sv + c - kp)) - (ldg(rhs_v + c + kp) - ldg(rhs_v + c - kp));
+            dphi_ = (ldg(sw + ce) - ldg(sw + cw)) - (ldg(rhs_w + ce) - ldg(rhs_w + cw));
         } else {                    // projection source, rigid-lid zero of S_u on the radial walls (:246-248)
-            const bool wall0 = K.press_incr && K.rigid_lid;
+            const bool wall0 = INCR && K.rigid_lid;
             const double sup = (wall0 && i + 1 == K.im - 1) ? 0.0 : ldg(su + c + P);
             const double sdn = (wall0 && i - 1 == 0) ? 0.0 : ldg(su + c - P);
             dr_ = sup - sdn;
@@ -102,11 +105,13 @@ __global__ void __launch_bounds__(256) press_source_kernel(
         }
         double div = fma(dphi_, ldg(&g->src_phi), fma(dthe_, ldg(&g->src_the), dr_ * ldg(&g->src_r)));
         const double src_max = ldg(&g->p_den) * K.pdyn_cap;
-        uint32_t lo, hi;
-        split_f64(div, lo, hi);
-        if (((hi >> 20) & 0x7FFu) == 0x7FFu) { div = 0.0; clamped = true; }
-        else if (fabs(div) > src_max) { div = (div > src_max) ? src_max : -src_max; clamped = true; }
-        if (K.press_incr) {         // lc_old = Lc(p_dyn) before the sweep (:249-282)
+        const long long bits = __double_as_longlong(div), mag = bits & 0x7FFFFFFFFFFFFFFFll;
+        if (mag >= 0x7FF0000000000000ll) { div = 0.0; clamped = true; }
+        else if (mag > __double_as_longlong(src_max)) {      // src_max > 0
+            div = __longlong_as_double(__double_as_longlong(src_max) | (bits & (long long)0x8000000000000000ull));
+            clamped = true;
+        }
+        if (INCR) {                 // lc_old = Lc(p_dyn) before the sweep (:249-282)
             const double p0 = ldg(p + c);      // fma(-2, p0, s) == s - 2 p0: the product is exact
             div = fma(ldg(&g->lc_num1), fma(-2.0, p0, ldg(p + c + P) + ldg(p + c - P)), div);
             div = fma(ldg(&g->lc_num2), fma(-2.0, p0, ldg(p + c + kp) + ldg(p + c - kp)), div);
@@ -226,8 +231,12 @@ cudaError_t launch_press_source(const KConst& kc, const ColGeo* geo, const doubl
                                 const double* rhs_u, const double* rhs_v, const double* rhs_w, const double* p,
                                 double* src, unsigned long long* nclamp, cudaStream_t s) {
     dim3 block(32, 8), grid((kc.km - 1 + 31) / 32, (kc.jm + 7) / 8, kc.im);
-    press_source_kernel<<<grid, block, 0, s>>>(kc, geo, su, sv, sw, aux_u, aux_v, aux_w, rhs_u, rhs_v, rhs_w, p,
-                                               src, nclamp);
+    if (kc.press_src == 0)          // press_incr is off then
+        press_source_kernel<true, false><<<grid, block, 0, s>>>(kc, geo, aux_u, aux_v, aux_w, rhs_u, rhs_v, rhs_w, p, src, nclamp);
+    else if (kc.press_incr)
+        press_source_kernel<false, true><<<grid, block, 0, s>>>(kc, geo, su, sv, sw, rhs_u, rhs_v, rhs_w, p, src, nclamp);
+    else
+        press_source_kernel<false, false><<<grid, block, 0, s>>>(kc, geo, su, sv, sw, rhs_u, rhs_v, rhs_w, p, src, nclamp);
     return cudaGetLastError();
 }
 
