@@ -822,25 +822,25 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
             P->bvec[q] = P->num2[q] * (jj == NJ - 1 ? 1.0 - kc.c13 : 1.0);   // coefficient of x_{j-1}
             P->cvec[q] = P->num2[q] * (jj == 0 ? 1.0 - kc.c13 : 1.0);        // coefficient of x_{j+1}
         }
-    // the inverse pivot blocks of every mode (FP64), then an FP32 copy
-    const size_t blk = (size_t)NI * NI;
-    std::vector<double> W((size_t)S.M * NJ * blk);
+    // the inverse pivot blocks of every mode, FP64 and FP32, in the mode solve's layouts
+    const size_t blk = (size_t)NI * NI, nblk = (size_t)S.M * NJ;
+    const size_t nW64 = nblk * P->bt64.stride, nW32 = nblk * P->bt32.stride;
+    std::vector<double> W64(nW64);
+    std::vector<float> W32(nW32);
     bool ok = true;
 #pragma omp parallel for schedule(dynamic)
     for (int m = 0; m < S.M; m++) {
-        std::vector<double> D, Sm, inv;
-        double* Wm = W.data() + (size_t)m * NJ * blk;
+        std::vector<double> D, Sm, inv, prev(blk);          // prev: W_{j-1}, column-major
         for (int jj = 0; jj < NJ; jj++) {
             build_D(*P, m, jj, D);
             Sm = D;
             if (jj > 0) {
-                const double* Wp = Wm + (size_t)(jj - 1) * blk;     // column-major W_{j-1}
                 for (int r = 0; r < NI; r++) {
                     const double b = P->bvec[(size_t)jj * NI + r];
                     for (int c = 0; c < NI; c++) {
                         double cc = P->cvec[(size_t)(jj - 1) * NI + c];
                         if (m == 0 && jj - 1 == 0 && c == 0) cc = 0.0;
-                        Sm[(size_t)r * NI + c] -= b * Wp[(size_t)c * NI + r] * cc;
+                        Sm[(size_t)r * NI + c] -= b * prev[(size_t)c * NI + r] * cc;
                     }
                 }
             }
@@ -849,9 +849,16 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
                 ok = false;
                 break;
             }
-            double* Wj = Wm + (size_t)jj * blk;
-            for (int r = 0; r < NI; r++)
-                for (int c = 0; c < NI; c++) Wj[(size_t)c * NI + r] = inv[(size_t)r * NI + c];
+            const size_t b = (size_t)m * NJ + jj;
+            double* w64 = W64.data() + b * P->bt64.stride;
+            float* w32 = W32.data() + b * P->bt32.stride;
+            for (int c = 0; c < NI; c++)
+                for (int r = 0; r < NI; r++) {
+                    const double w = inv[(size_t)r * NI + c];
+                    prev[(size_t)c * NI + r] = w;
+                    w64[bt_place<double>(P->bt64, NI, r, c)] = w;
+                    w32[bt_place<float>(P->bt32, NI, r, c)] = (float)w;
+                }
         }
     }
     if (!ok) { *err = "poisson: singular pivot block"; delete P; return nullptr; }
@@ -902,7 +909,6 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
     // device buffers
     const size_t fsz = (size_t)kc.fsz;
     const size_t nspec = (size_t)S.M * NJ * S.RS;
-    const size_t nblk = (size_t)S.M * NJ, nW64 = nblk * P->bt64.stride, nW32 = nblk * P->bt32.stride;
     size_t bytes = 0;
     auto take = [&](size_t b) { size_t o = bytes; bytes += (b + 255) & ~size_t(255); return o; };
     const size_t o_f = take(fsz * 8), o_p = take(fsz * 8), o_r = take(fsz * 8), o_sq = take(64);
@@ -988,17 +994,6 @@ PoissonSolver* poisson_create(const KConst& kc, const ColGeo* geo_dev, const std
             if (!(ev && std::atoi(ev) == 1)) plan_tb(P, 2, dev, nsm);
         }
     }
-    // the pivot blocks in the mode solve's layout
-    std::vector<double> W64(nW64, 0.0);
-    std::vector<float> W32(nW32, 0.0f);
-#pragma omp parallel for schedule(static)
-    for (size_t b = 0; b < nblk; b++)
-        for (int c = 0; c < NI; c++)
-            for (int r = 0; r < NI; r++) {
-                const double w = W[b * blk + (size_t)c * NI + r];
-                W64[b * P->bt64.stride + bt_place<double>(P->bt64, NI, r, c)] = w;
-                W32[b * P->bt32.stride + bt_place<float>(P->bt32, NI, r, c)] = (float)w;
-            }
     std::vector<double> tw(2 * S.n);
     std::vector<float> tw32(2 * S.n);
     for (int k = 0; k < S.n; k++) {
