@@ -47,8 +47,8 @@ struct atsat_dyn {
     double* stage[NPROG] = {};
     double* acc[NPROG] = {};
     double* src = nullptr;
-    // PRESS_LINE / PRESS_BAROTROPIC: forward-sweep scratch of the line pass, interior-mean partials and
-    // the means on entry and after a sweep, the barotropic tables and scratch (one allocation)
+    // PRESS_LINE / PRESS_BAROTROPIC: the line pass's elimination table and forward-sweep scratch, interior-mean
+    // partials and the means on entry and after a sweep, the barotropic tables and scratch (one allocation)
     double* pv_buf = nullptr;
     // the turbulence closure: its knobs, one allocation for P_k (fsz), u_tau (jm x kp) and the tables
     atsat_dyn_turb_params tp{};
@@ -59,7 +59,8 @@ struct atsat_dyn {
     double* clamp_added = nullptr;
     unsigned long long* clamp_cells = nullptr;
     double* clamp_partial = nullptr;     // the floor's per-block sums
-    double *line_cp = nullptr, *line_dp = nullptr, *imean_partial = nullptr, *pmean = nullptr;
+    LineGeo* line_tab = nullptr;
+    double *line_dp = nullptr, *imean_partial = nullptr, *pmean = nullptr;
     BaroTables baro{};
     double* p_baro = nullptr;            // null unless set
     double* partial = nullptr;
@@ -1433,7 +1434,7 @@ int enqueue_pressure(atsat_dyn* h, int sweeps) {
             for (int colour = 0; colour < 2; colour++) {
                 Timed t(h, ATSAT_K_PRESS_SWEEP);
                 int n = 0;
-                CK(h, launch_line_pass(K, h->geo, h->src, pd, h->line_cp, h->line_dp, colour, h->stream, &n));
+                CK(h, launch_line_pass(K, h->line_tab, h->src, pd, h->line_dp, colour, h->stream, &n));
                 h->launches += n;
             }
         }
@@ -1724,33 +1725,35 @@ int setup_press_variants(atsat_dyn* h) {
     if (!line && !baro) return ATSAT_DYN_OK;
     constexpr double PI = 3.14159265358979323846;
     const int N = K.km - 1, J = K.jm - 2, NM = N / 2;
-    const int64_t n_line = line ? 2 * K.fsz : 0;
+    const int64_t NU = ((int64_t)NM + 1 + 31) / 32 * 32;
+    const int64_t n_line = line ? K.fsz + (int64_t)K.im * K.jm * (int64_t)(sizeof(LineGeo) / 8) : 0;
     const int64_t n_mean = line ? interior_mean_partials(K) + 2 : 0;
-    const int64_t n_tab = baro ? 2LL * (NM + 1) * N + (NM + 1) + K.jm + J : 0;
-    const int64_t n_scr = baro ? (int64_t)J * N + J + 4LL * (NM + 1) * J : 0;
+    const int64_t n_tab = baro ? 2LL * N + (NM + 1) + K.jm + J : 0;
+    const int64_t n_scr = baro ? (int64_t)J * N + 5 * (int64_t)J * NU + 2 : 0;
     const int64_t total = n_line + n_mean + n_tab + n_scr + 64;
     cudaError_t e = cudaMalloc(&h->pv_buf, (size_t)total * 8);
     if (e != cudaSuccess) { h->pv_buf = nullptr; return fail(h, ATSAT_DYN_E_NOMEM, "pressure variants: %s", cudaGetErrorString(e)); }
     double* q = h->pv_buf;
     if (line) {
-        h->line_cp = q; q += K.fsz;
+        h->line_tab = reinterpret_cast<LineGeo*>(q); q += (int64_t)K.im * K.jm * (int64_t)(sizeof(LineGeo) / 8);
         h->line_dp = q; q += K.fsz;
         h->pmean = q; q += 2;
         h->imean_partial = q; q += interior_mean_partials(K);
+        CK(h, launch_line_table(K, h->geo, h->line_tab, h->stream));
     }
     if (baro) {
         std::vector<double> tab((size_t)n_tab);
         double* ct = tab.data();
-        double* st = ct + (size_t)(NM + 1) * N;
-        double* lam = st + (size_t)(NM + 1) * N;
+        double* st = ct + N;
+        double* lam = st + N;
         double* sinthe = lam + (NM + 1);
         double* abs_sin = sinthe + K.jm;
+        for (int k = 0; k < N; k++) {
+            const double a = 2.0 * PI * (double)k / N;
+            ct[k] = std::cos(a);
+            st[k] = std::sin(a);
+        }
         for (int mm = 0; mm <= NM; mm++) {
-            for (int k = 0; k < N; k++) {
-                const double a = 2.0 * PI * (double)((long)mm * k % N) / N;
-                ct[(size_t)mm * N + k] = std::cos(a);
-                st[(size_t)mm * N + k] = std::sin(a);
-            }
             const double sl = std::sin(PI * mm / N);
             lam[mm] = 4.0 * sl * sl * K.inv_dphi2;
         }
@@ -1770,19 +1773,19 @@ int setup_press_variants(atsat_dyn* h) {
         e = cudaMemcpy(dtab, tab.data(), (size_t)n_tab * 8, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return fail(h, ATSAT_DYN_E_CUDA, "pressure variant tables: %s", cudaGetErrorString(e));
         BaroTables& T = h->baro;
+        T.N = N; T.NM = NM; T.J = J; T.NU = (int)NU;
         T.A2 = A2;
         T.ct = dtab;
-        T.st = dtab + (size_t)(NM + 1) * N;
-        T.lam = T.st + (size_t)(NM + 1) * N;
+        T.st = dtab + N;
+        T.lam = T.st + N;
         T.sinthe = T.lam + (NM + 1);
         T.abs_sin = T.sinthe + K.jm;
         T.R = q; q += (int64_t)J * N;
-        T.ra = q; q += J;
-        T.Ac = q; q += (int64_t)(NM + 1) * J;
-        T.As = q; q += (int64_t)(NM + 1) * J;
-        T.cp = q; q += (int64_t)(NM + 1) * J;
-        T.dp = q; q += (int64_t)(NM + 1) * J;
+        for (double** t : {&T.cp, &T.ar, &T.rdn, &T.Ac, &T.As}) { *t = q; q += (int64_t)J * NU; }
+        T.sums = q; q += 2;
+        CK(h, launch_baro_table(K, T, h->stream));
     }
+    CK(h, cudaStreamSynchronize(h->stream));
     return ATSAT_DYN_OK;
 }
 

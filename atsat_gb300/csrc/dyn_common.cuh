@@ -450,14 +450,23 @@ cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const 
                               int* launches);
 
 // PRESS_LINE / PRESS_BAROTROPIC (press_variants.cu)
+// the elimination of the line pass's radial tridiagonal per (i, j)
+struct alignas(16) LineGeo { double num1, num2, num3, a, dn, rdn, cp, pad; };
 struct BaroTables {
+    int N, NM, J, NU;                             // meridians, N / 2, polar rows, modes per row of a table (NM + 1, padded)
     double A2;                                    // sum over i = 1..im-2 of 1 / rm^2
-    const double *ct, *st;                        // (N/2 + 1) x N: cos, sin(2 pi (m k mod N) / N)
+    const double *ct, *st;                        // N: cos, sin(2 pi k / N)
     const double *lam, *sinthe, *abs_sin;         // per mode; the solver's sine table (jm); |sin(theta_j+1)|
-    double *R, *ra, *Ac, *As, *cp, *dp;           // scratch
+    double *cp, *ar, *rdn;                        // J x NU: each mode's elimination (launch_baro_table)
+    double *sums;                                 // mode 0's weight sums
+    double *R, *Ac, *As;                          // scratch: J x N, and J x NU cosine and sine sums
 };
-cudaError_t launch_line_pass(const KConst& kc, const ColGeo* geo, const double* src, double* p, double* cpb,
-                             double* dpb, int colour, cudaStream_t s, int* launches);
+cudaError_t launch_line_table(const KConst& kc, const ColGeo* geo, LineGeo* tab, cudaStream_t s);
+cudaError_t launch_baro_table(const KConst& kc, const BaroTables& T, cudaStream_t s);
+cudaError_t launch_baro_forward(const BaroTables& T, cudaStream_t s);    // R -> Ac, As (press_baro_fft.cu)
+cudaError_t launch_baro_inverse(const BaroTables& T, cudaStream_t s);    // Ac, As -> R
+cudaError_t launch_line_pass(const KConst& kc, const LineGeo* tab, const double* src, double* p, double* dpb, int colour,
+                             cudaStream_t s, int* launches);
 cudaError_t launch_interior_mean(const KConst& kc, const double* p, double* partial, double* out, cudaStream_t s,
                                  int* launches);
 int interior_mean_partials(const KConst& kc);

@@ -76,9 +76,10 @@ __device__ __forceinline__ void butterfly(Cx<T>* a) {
 }
 
 template <typename T, int R>
-__device__ __forceinline__ void stage(const Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, int s, uint32_t mag, int lane) {
+__device__ __forceinline__ void stage(const Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, int s, uint32_t mag, int lane,
+                                      int step) {
     const int items = n / R;
-    for (int e = lane; e < items; e += 32) {
+    for (int e = lane; e < items; e += step) {
         const int p = s == 1 ? e : (int)__umulhi((uint32_t)e, mag), q = e - p * s;
         Cx<T> a[R];
 #pragma unroll
@@ -97,16 +98,16 @@ __device__ __forceinline__ void stage(const Cx<T>* x, Cx<T>* y, const Cx<T>* tw,
 // any other radix: a lane per output value
 template <typename T>
 __device__ __forceinline__ void stage_any(const Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, int R, int s, uint32_t mag,
-                                          int lane) {
+                                          int lane, int step) {
     const int items = n / R;
     int u = lane / items, e = lane - u * items;
-    const int du = 32 / items, de = 32 - du * items;
-    for (int w = lane; w < n; w += 32) {
-        const int p = s == 1 ? e : (int)__umulhi((uint32_t)e, mag), q = e - p * s, step = u * items;
+    const int du = step / items, de = step - du * items;
+    for (int w = lane; w < n; w += step) {
+        const int p = s == 1 ? e : (int)__umulhi((uint32_t)e, mag), q = e - p * s, turn_by = u * items;
         Cx<T> b = x[e];
         int idx = 0;
         for (int t = 1; t < R; t++) {
-            idx += step;                                             // t u (n / R) mod n
+            idx += turn_by;                                          // t u (n / R) mod n
             if (idx >= n) idx -= n;
             const Cx<T> c = tw[idx];
             b = b + turn(x[e + t * items], c.re, c.im);
@@ -118,23 +119,29 @@ __device__ __forceinline__ void stage_any(const Cx<T>* x, Cx<T>* y, const Cx<T>*
     }
 }
 
-// One warp transforms the complex sequence in `x`; returns the buffer that holds the result in natural order.
-template <typename T>
-__device__ __forceinline__ Cx<T>* fft_warp(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, const FftPlan& F, int lane) {
+// Transforms the complex sequence in `x` with `step` threads (`lane` this one's index; `sync` orders their shared-memory
+// accesses); returns the buffer that holds the result in natural order.
+template <typename T, class Sync>
+__device__ __forceinline__ Cx<T>* fft(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, const FftPlan& F, int lane, int step,
+                                      Sync sync) {
     for (int st = 0; st < F.stages; st++) {
         const int R = F.radix[st], s = F.s[st];
         const uint32_t mag = F.mag[st];
         switch (R) {
-            case 2: stage<T, 2>(x, y, tw, n, s, mag, lane); break;
-            case 3: stage<T, 3>(x, y, tw, n, s, mag, lane); break;
-            case 4: stage<T, 4>(x, y, tw, n, s, mag, lane); break;
-            case 5: stage<T, 5>(x, y, tw, n, s, mag, lane); break;
-            default: stage_any<T>(x, y, tw, n, R, s, mag, lane); break;
+            case 2: stage<T, 2>(x, y, tw, n, s, mag, lane, step); break;
+            case 3: stage<T, 3>(x, y, tw, n, s, mag, lane, step); break;
+            case 4: stage<T, 4>(x, y, tw, n, s, mag, lane, step); break;
+            case 5: stage<T, 5>(x, y, tw, n, s, mag, lane, step); break;
+            default: stage_any<T>(x, y, tw, n, R, s, mag, lane, step); break;
         }
-        __syncwarp();
+        sync();
         Cx<T>* z = x; x = y; y = z;
     }
     return x;
+}
+template <typename T>
+__device__ __forceinline__ Cx<T>* fft_warp(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, const FftPlan& F, int lane) {
+    return fft(x, y, tw, n, F, lane, 32, [] { __syncwarp(); });
 }
 
 template <typename T>

@@ -4,16 +4,19 @@
 // PRESS_LINE: per colour ((j + k) & 1) every (j, k) column is relaxed exactly in r -- a Thomas solve over
 // i = 1..im-2 with the theta / phi neighbours lagged and both radial ends folded (p0 = c43 p1 - c13 p2) --
 // and after the boundary pass the interior mean of p_dyn is held at its value on entry. One thread per
-// column; the forward coefficients go to two scratch fields at the column's own cells. The columns of one
+// column; the matrix does not depend on k, so its elimination is tabulated once per (i, j) (LineGeo). The columns of one
 // colour read only the other colour, except across an odd periodic seam where k = 0 and k = km-2 share a
 // colour: as in a single thread's visit of the reference's loop, k = km-2 is solved after k = 0 (a second
 // launch) and reads its new values.
 //
 // PRESS_BAROTROPIC: the column residual R(j, k) = sum_i (src - Lc(p)) / sum_i 1/rm^2, its real DFT over
-// the N = km-1 meridians (sequential sums, modes below 1e-12 of the row's sum |R| dropped), per mode a
-// tridiagonal in theta (mode 0 made consistent, pinned at j = 1, shifted to zero sin-weighted mean), and
-// the correction q(j, k) added to every level of the column. The cos / sin tables, the modes' eigenvalue
-// factors and the sine tables come from the host, formed with the reference's own expressions.
+// the N = km-1 meridians (press_baro_fft.cu; modes below 1e-12 of the row's sum |R| dropped), per mode a
+// tridiagonal in theta (mode 0 made consistent, pinned at j = 1, shifted to zero sin-weighted mean; its elimination
+// tabulated too), and the correction q(j, k) added to every level of the column.
+//
+// Rounding. The residual is a sum of nearly cancelling terms and the theta solve amplifies its rounding, so this file is
+// compiled without multiply-add contraction and every value is the one the reference's expressions round to: quotients
+// by a tabulated divisor are formed from its reciprocal and corrected to the division's own rounding (div_tab).
 //
 // Weights: lc_num1..3 of ColGeo are the line pass's num1, num2, num3 expression for expression.
 #include "dyn_common.cuh"
@@ -23,80 +26,118 @@ namespace {
 
 __device__ __forceinline__ double ldg(const double* p) { return __ldg(p); }
 
-// PressureSolver.h:506-567 for one column
-__device__ void line_column(const KConst& K, const ColGeo* __restrict__ geo, const double* __restrict__ src,
-                            double* __restrict__ p, double* __restrict__ cpb, double* __restrict__ dpb, int j, int k) {
+// isfinite on the integer pipe
+__device__ __forceinline__ bool finite_bits(double x) {
+    uint32_t lo, hi;
+    split_f64(x, lo, hi);
+    return (hi & 0x7FF00000u) != 0x7FF00000u;
+}
+
+// x / d from y = 1 / d (rounded): two corrections by the exact residual give the correctly rounded quotient where
+// nothing over- or underflows (P. Markstein, IA-64 and Elementary Functions, 2000, ch. 8); the division elsewhere. Five
+// FP64 operations in a chain instead of about a dozen and a call.
+__device__ __forceinline__ double div_tab(double x, double d, double y) {
+    double q = x * y;
+    uint32_t lo, hi;
+    split_f64(q, lo, hi);
+    if (((hi >> 20) & 0x7FFu) - 200u < 1600u) {
+        q = fma(fma(-q, d, x), y, q);
+        return fma(fma(-q, d, x), y, q);
+    }
+    return x / d;
+}
+
+// The elimination of a column's matrix per (i, j): the coupling to the row above as eliminated (a), the pivot and its
+// reciprocal, and cp (PressureSolver.h:506-567 with the fold of both ends).
+__global__ void line_table_kernel(const KConst K, const ColGeo* __restrict__ geo, LineGeo* __restrict__ tab) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < 1 || j > K.jm - 2) return;
+    const int lo = 1, hi = K.im - 2;
+    const bool fold = hi > lo;
+    double cprev = 0.0;
+    for (int i = lo; i <= hi; i++) {
+        const ColGeo* g = geo + ((int64_t)i * K.jm + j);
+        const double num1 = g->lc_num1, num2 = g->lc_num2, num3 = g->lc_num3;
+        double a = -num1, b = 2.0 * (num1 + num2 + num3), cc = -num1;
+        if (i == lo && fold) { b += a * K.c43; cc -= a * K.c13; }
+        if (i == hi && fold) { b += cc * K.c43; a -= cc * K.c13; }
+        const double dn = i == lo ? b : b - a * cprev;
+        LineGeo& t = tab[(int64_t)i * K.jm + j];
+        t.num1 = num1; t.num2 = num2; t.num3 = num3;
+        t.a = a; t.dn = dn; t.rdn = 1.0 / dn;
+        t.cp = cprev = cc / dn;
+        t.pad = 0.0;
+    }
+}
+
+// One column. Bound by the FP64 pipe: 15 operations per cell, where forming the elimination in every column took about
+// 45 and two divisions (151 us per colour at 41x181x361; 39 dependent steps per thread, the loads of LINE_AHEAD levels
+// issued ahead; 4 to 13 measured alike): 64 us.
+constexpr int LINE_AHEAD = 4;
+
+__device__ void line_column(const KConst& K, const LineGeo* __restrict__ tab, const double* __restrict__ src,
+                            double* __restrict__ p, double* __restrict__ dpb, int j, int k) {
     const int64_t P = K.plane, kp = K.kp;
     const int kw = (k == 0) ? K.km - 2 : k - 1;
     const int ke = (k == K.km - 2) ? 0 : k + 1;
     const int lo = 1, hi = K.im - 2;
-    const bool fold = hi > lo;
-    double cprev = 0.0, dprev = 0.0;
-    for (int i = lo; i <= hi; i++) {
-        const int64_t c = ((int64_t)i * K.jm + j) * kp + k;
-        const ColGeo* g = geo + ((int64_t)i * K.jm + j);
-        const double num1 = ldg(&g->lc_num1), num2 = ldg(&g->lc_num2), num3 = ldg(&g->lc_num3);
-        const double acc_h = num2 * (p[c + kp] + p[c - kp]) + num3 * (p[c - k + ke] + p[c - k + kw]);
-        double a = -num1, b = 2.0 * (num1 + num2 + num3), cc = -num1;
-        double d = acc_h - ldg(src + c);
-        if (i == lo) {
-            if (fold) { b += a * K.c43; cc -= a * K.c13; }
-            else d -= a * p[c - P];
+    double dprev = 0.0;
+    const int64_t c1 = ((int64_t)lo * K.jm + j) * kp + k;
+    for (int i0 = lo; i0 <= hi; i0 += LINE_AHEAD) {
+        double n[LINE_AHEAD], s[LINE_AHEAD], e[LINE_AHEAD], w[LINE_AHEAD], f[LINE_AHEAD];
+#pragma unroll
+        for (int u = 0; u < LINE_AHEAD; u++) {
+            const int64_t c = c1 + (int64_t)(i0 - lo + u) * P;
+            if (i0 + u <= hi) {
+                n[u] = p[c - kp]; s[u] = p[c + kp]; e[u] = p[c - k + ke]; w[u] = p[c - k + kw]; f[u] = ldg(src + c);
+            }
         }
-        if (i == hi) {
-            if (fold) { b += cc * K.c43; a -= cc * K.c13; }
-            else d -= cc * p[c + P];
+#pragma unroll
+        for (int u = 0; u < LINE_AHEAD; u++) {
+            const int i = i0 + u;
+            if (i > hi) break;
+            const LineGeo& t = tab[(int64_t)i * K.jm + j];
+            const double d = t.num2 * (s[u] + n[u]) + t.num3 * (e[u] + w[u]) - f[u];
+            dprev = div_tab(i == lo ? d : d - t.a * dprev, t.dn, t.rdn);
+            dpb[c1 + (int64_t)(i - lo) * P] = dprev;
         }
-        double cpi, dpi;
-        if (i == lo) {
-            cpi = cc / b;
-            dpi = d / b;
-        } else {
-            const double dn = b - a * cprev;
-            cpi = cc / dn;
-            dpi = (d - a * dprev) / dn;
-        }
-        cpb[c] = cpi;
-        dpb[c] = dpi;
-        cprev = cpi;
-        dprev = dpi;
     }
     double x = dprev;
-    {
-        const int64_t c = ((int64_t)hi * K.jm + j) * kp + k;
-        if (isfinite(x)) p[c] = x;
-    }
+    int64_t c = c1 + (int64_t)(hi - lo) * P;
+    if (finite_bits(x)) p[c] = x;
+#pragma unroll 4
     for (int i = hi - 1; i >= lo; i--) {
-        const int64_t c = ((int64_t)i * K.jm + j) * kp + k;
-        x = dpb[c] - cpb[c] * x;
-        if (isfinite(x)) p[c] = x;
+        c -= P;
+        x = dpb[c] - tab[(int64_t)i * K.jm + j].cp * x;
+        if (finite_bits(x)) p[c] = x;
     }
 }
 
-__global__ void __launch_bounds__(128) line_kernel(const KConst K, const ColGeo* __restrict__ geo,
+constexpr int LINE_THREADS = 64;   // 181 columns of a colour and row are 3 x 64: the blocks even out over the SMs
+
+__global__ void __launch_bounds__(LINE_THREADS) line_kernel(const KConst K, const LineGeo* __restrict__ tab,
                                                    const double* __restrict__ src, double* __restrict__ p,
-                                                   double* __restrict__ cpb, double* __restrict__ dpb, int colour) {
+                                                   double* __restrict__ dpb, int colour) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     if (j > K.jm - 2) return;
     const int k = 2 * m + ((colour - j) & 1);
     if (k > K.km - 2) return;
     if (k == K.km - 2 && k > 0 && ((K.km - 1) & 1)) return;     // after its seam partner k = 0
-    line_column(K, geo, src, p, cpb, dpb, j, k);
+    line_column(K, tab, src, p, dpb, j, k);
 }
 
-__global__ void line_seam_kernel(const KConst K, const ColGeo* __restrict__ geo, const double* __restrict__ src,
-                                 double* __restrict__ p, double* __restrict__ cpb, double* __restrict__ dpb,
-                                 int colour) {
+__global__ void line_seam_kernel(const KConst K, const LineGeo* __restrict__ tab, const double* __restrict__ src,
+                                 double* __restrict__ p, double* __restrict__ dpb, int colour) {
     const int j = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     if (j > K.jm - 2) return;
     const int k = K.km - 2;
     if (((j + k) & 1) != colour) return;
-    line_column(K, geo, src, p, cpb, dpb, j, k);
+    line_column(K, tab, src, p, dpb, j, k);
 }
 
 // ---- interior mean (PressureSolver.h:310-316): per level partial sums over row chunks, then in order ----
-constexpr int IM_CHUNKS = 8;
+constexpr int IM_CHUNKS = 16;
 
 __global__ void __launch_bounds__(128) imean_partial_kernel(const KConst K, const double* __restrict__ p,
                                                             double* __restrict__ partial) {
@@ -107,6 +148,7 @@ __global__ void __launch_bounds__(128) imean_partial_kernel(const KConst K, cons
     double s = 0.0;
     for (int j = j0 + warp; j < j1; j += 4) {
         const double* row = p + ((int64_t)i * K.jm + j) * K.kp;
+#pragma unroll 4
         for (int k = lane; k <= K.km - 2; k += 32) s += ldg(row + k);
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
@@ -117,10 +159,10 @@ __global__ void __launch_bounds__(128) imean_partial_kernel(const KConst K, cons
 }
 
 __global__ void imean_final_kernel(const double* __restrict__ partial, int n, double count, double* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double s = 0.0;
-    for (int q = 0; q < n; q++) s += partial[q];
-    *out = s / count;
+    for (int q = threadIdx.x; q < n; q += 32) s += partial[q];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *out = s / count;
 }
 
 // p -= mean_now - mean_entry on every cell (PressureSolver.h:750-755)
@@ -135,18 +177,42 @@ __global__ void __launch_bounds__(256) mean_shift_kernel(const KConst K, double*
 }
 
 // ---- PRESS_BAROTROPIC (PressureSolver.h:573-708) ----
-// the column residual of PressureSolver.h:581-604, end rows read as the boundary pass sets them
-__device__ __forceinline__ double pb_i(const KConst& K, const double* p, int i, int j, int k) {
-    const int64_t row = (int64_t)j * K.kp + k;
-    if (i == 0) return K.c43 * p[K.plane + row] - K.c13 * p[2 * K.plane + row];
-    if (i == K.im - 1) return K.c43 * p[(K.im - 2) * K.plane + row] - K.c13 * p[(K.im - 3) * K.plane + row];
-    return p[(int64_t)i * K.plane + row];
-}
-__device__ __forceinline__ double pb_j(const KConst& K, const double* p, int i, int j, int k) {
-    const int64_t base = (int64_t)i * K.plane + k;
-    if (j == 0) return K.c43 * p[base + K.kp] - K.c13 * p[base + 2 * K.kp];
-    if (j == K.jm - 1) return K.c43 * p[base + (int64_t)(K.jm - 2) * K.kp] - K.c13 * p[base + (int64_t)(K.jm - 3) * K.kp];
-    return p[base + (int64_t)j * K.kp];
+// the column residual of PressureSolver.h:581-604, end rows read as the boundary pass sets them. 13 FP64 operations per
+// cell, each rounded as the reference's ((x + y) - 2 p0 as one fma: the product is exact); the column marches in i with
+// its radial neighbours in registers, and the polar rows' folds and the lid are branches of
+// their own, not predicated instructions that would take the pipe's slots: 183 -> 86 us at 41x181x361 (the operations
+// alone are 52).
+template <bool NORTH, bool SOUTH>
+__device__ __forceinline__ double column_residual(const KConst& K, const ColGeo* __restrict__ geo,
+                                                  const double* __restrict__ src, const double* __restrict__ p, int j, int k) {
+    const int N = K.km - 1;
+    const int kw = (k == 0) ? N - 1 : k - 1;
+    const int ke = (k == N - 1) ? 0 : k + 1;
+    const int64_t P = K.plane, kp = K.kp;
+    int64_t c = ((int64_t)K.jm + j) * kp + k;
+    double s = 0.0, p0 = p[c], pn = p[c + P];
+    double pm = K.c43 * p0 - K.c13 * pn;                     // i = 0
+    const ColGeo* g = geo + ((int64_t)K.jm + j);
+    auto term = [&](double pip) {
+        const double pjp = SOUTH ? K.c43 * p0 - K.c13 * p[c - kp] : p[c + kp];
+        const double pjm = NORTH ? K.c43 * p0 - K.c13 * p[c + kp] : p[c - kp];
+        const double lc = ldg(&g->lc_num1) * fma(-2.0, p0, pip + pm)
+                        + ldg(&g->lc_num2) * fma(-2.0, p0, pjp + pjm)
+                        + ldg(&g->lc_num3) * fma(-2.0, p0, p[c - k + ke] + p[c - k + kw]);
+        s += ldg(src + c) - lc;
+    };
+#pragma unroll 4
+    for (int i = 1; i < K.im - 2; i++) {
+        const double ahead = p[c + 2 * P];                   // level i + 2: an interior level or the lid (not used)
+        term(pn);
+        pm = p0;
+        p0 = pn;
+        pn = ahead;
+        c += P;
+        g += K.jm;
+    }
+    term(K.c43 * p0 - K.c13 * pm);                           // the level below the lid
+    return s;
 }
 
 __global__ void __launch_bounds__(128) baro_resid_kernel(const KConst K, const ColGeo* __restrict__ geo,
@@ -156,149 +222,159 @@ __global__ void __launch_bounds__(128) baro_resid_kernel(const KConst K, const C
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y;
     if (k >= N || j > K.jm - 2) return;
-    const int kw = (k == 0) ? N - 1 : k - 1;
-    const int ke = (k == N - 1) ? 0 : k + 1;
-    double s = 0.0;
-    for (int i = 1; i < K.im - 1; i++) {
-        const ColGeo* g = geo + ((int64_t)i * K.jm + j);
-        const int64_t c = ((int64_t)i * K.jm + j) * K.kp + k;
-        const double p0 = p[c];
-        const double lc = ldg(&g->lc_num1) * (pb_i(K, p, i + 1, j, k) + pb_i(K, p, i - 1, j, k) - 2.0 * p0)
-                        + ldg(&g->lc_num2) * (pb_j(K, p, i, j + 1, k) + pb_j(K, p, i, j - 1, k) - 2.0 * p0)
-                        + ldg(&g->lc_num3) * (p[c - k + ke] + p[c - k + kw] - 2.0 * p0);
-        s += ldg(src + c) - lc;
-    }
+    const double s = j == 1 ? column_residual<true, false>(K, geo, src, p, j, k)
+                   : j == K.jm - 2 ? column_residual<false, true>(K, geo, src, p, j, k)
+                                   : column_residual<false, false>(K, geo, src, p, j, k);
     R[(int64_t)(j - 1) * N + k] = s / A2;
 }
 
-// sum_k |R(j, k)| per row, in order
-__global__ void baro_rowabs_kernel(int J, int N, const double* __restrict__ R, double* __restrict__ ra) {
-    const int jj = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jj >= J) return;
-    double s = 0.0;
-    for (int k = 0; k < N; k++) s += fabs(R[(int64_t)jj * N + k]);
-    ra[jj] = s;
-}
-
-// Ac[m][j] = sum_k R cos(2 pi m k / N), As likewise with sin; one thread per (mode, row), sums in k order
-__global__ void __launch_bounds__(128) baro_dft_kernel(int J, int N, int NM, const double* __restrict__ R,
-                                                       const double* __restrict__ ct, const double* __restrict__ st,
-                                                       const double* __restrict__ ra, double* __restrict__ Ac,
-                                                       double* __restrict__ As) {
-    const int jj = blockIdx.x * blockDim.x + threadIdx.x;
-    const int mm = blockIdx.y;
-    if (jj >= J || mm > NM) return;
-    const double* r_ = R + (int64_t)jj * N;
-    const double* c_ = ct + (int64_t)mm * N;
-    const double* s_ = st + (int64_t)mm * N;
-    double sc = 0.0, ss = 0.0;
-    for (int k = 0; k < N; k++) {
-        const double r = ldg(r_ + k);
-        sc += r * ldg(c_ + k);
-        ss += r * ldg(s_ + k);
-    }
-    if (mm > 0) {
-        const double tol = 1.0e-12 * ra[jj];
-        if (fabs(sc) < tol) sc = 0.0;
-        if (fabs(ss) < tol) ss = 0.0;
-    }
-    Ac[(int64_t)mm * J + jj] = sc;
-    As[(int64_t)mm * J + jj] = ss;
-}
-
-struct BaroModes {
-    int J, N, NM;
-    double e, c43, c13;
-    const double* lam;         // NM+1: 4 sin^2(pi m / N) / dphi^2
-    const double* sinthe;      // jm: the solver's guarded sine table
-    const double* abs_sin;     // J: |sin(the_z[jj+1])|
-    double *Ac, *As, *cp, *dp; // cp, dp: (NM+1) x J scratch
-};
-
-// PressureSolver.h:638-680: one thread per mode, both parts
-__global__ void baro_modes_kernel(const BaroModes B) {
+// The elimination of each mode's tridiagonal in theta (PressureSolver.h:638-680): cp, the pivot's reciprocal and the
+// coupling times it at [jj * NU + mode]; mode 0's weight sums.
+__global__ void baro_table_kernel(const BaroTables B, double e, double c43, double c13) {
     const int mm = blockIdx.x * blockDim.x + threadIdx.x;
     if (mm > B.NM) return;
     const int J = B.J;
-    const double e = B.e, lam = B.lam[mm];
-    auto coef = [&](int jj, double& a, double& b, double& c) {
+    const double lam = B.lam[mm];
+    double cprev = 0.0;
+    for (int jj = 0; jj < J; jj++) {
         const double s_ = B.sinthe[jj + 1];
-        a = e;
-        c = e;
-        b = -2.0 * e - lam / (s_ * s_);
-        if (jj == 0) { a = 0.0; b += B.c43 * e; c -= B.c13 * e; }
-        if (jj == J - 1) { c = 0.0; b += B.c43 * e; a -= B.c13 * e; }
-    };
-    double* cp = B.cp + (int64_t)mm * J;
-    double* dp = B.dp + (int64_t)mm * J;
-    for (int part = 0; part < 2; part++) {
-        if (mm == 0 && part == 1) continue;
-        if (2 * mm == B.N && part == 1) continue;
-        double* d = (part == 0 ? B.Ac : B.As) + (int64_t)mm * J;
-        double a0, b0, c0;
-        coef(0, a0, b0, c0);
-        if (mm == 0) {
-            double yr = 0.0, ys = 0.0;
-            for (int jj = 0; jj < J; jj++) {
-                const double y = (jj == 0 || jj == J - 1) ? 1.5 : 1.0;
-                yr += y * d[jj];
-                ys += y * B.abs_sin[jj];
-            }
-            for (int jj = 0; jj < J; jj++) d[jj] -= yr / ys * B.abs_sin[jj];
-            b0 = 1.0;
-            c0 = 0.0;
-            d[0] = 0.0;
+        double a = e, b = -2.0 * e - lam / (s_ * s_), c = e;
+        if (jj == 0) { a = 0.0; b += c43 * e; c -= c13 * e; }
+        if (jj == J - 1) { c = 0.0; b += c43 * e; a -= c13 * e; }
+        if (mm == 0 && jj == 0) { b = 1.0; c = 0.0; }
+        const double dn = jj == 0 ? b : b - a * cprev;
+        const int64_t o = (int64_t)jj * B.NU + mm;
+        B.rdn[o] = 1.0 / dn;
+        B.ar[o] = a / dn;
+        B.cp[o] = cprev = c / dn;
+    }
+    if (mm == 0) {
+        double ys = 0.0, sw = 0.0;
+        for (int jj = 0; jj < J; jj++) {
+            ys += ((jj == 0 || jj == J - 1) ? 1.5 : 1.0) * B.abs_sin[jj];
+            sw += B.abs_sin[jj];
         }
-        cp[0] = c0 / b0;
-        dp[0] = d[0] / b0;
-        for (int jj = 1; jj < J; jj++) {
-            double a, b, c;
-            coef(jj, a, b, c);
-            const double dn = b - a * cp[jj - 1];
-            cp[jj] = c / dn;
-            dp[jj] = (d[jj] - a * dp[jj - 1]) / dn;
-        }
-        d[J - 1] = dp[J - 1];
-        for (int jj = J - 2; jj >= 0; jj--) d[jj] = dp[jj] - cp[jj] * d[jj + 1];
-        if (mm == 0) {
-            double sq = 0.0, sw = 0.0;
-            for (int jj = 0; jj < J; jj++) {
-                sq += B.abs_sin[jj] * d[jj];
-                sw += B.abs_sin[jj];
-            }
-            for (int jj = 0; jj < J; jj++) d[jj] -= sq / sw;
-        }
+        B.sums[0] = ys;
+        B.sums[1] = sw;
     }
 }
 
-// PressureSolver.h:684-697: q(j, k) back in phi, added to every level of the column
-__global__ void __launch_bounds__(128) baro_apply_kernel(const KConst K, int J, int N, int NM,
-                                                         const double* __restrict__ Ac, const double* __restrict__ As,
-                                                         const double* __restrict__ ct, const double* __restrict__ st,
-                                                         double* __restrict__ p) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int jj = blockIdx.y;
-    if (k >= N || jj >= J) return;
-    double q = 0.0;
-    for (int mm = 0; mm <= NM; mm++) {
-        const bool real = (mm == 0 || 2 * mm == N);
-        const double w_ = real ? 1.0 : 2.0;
-        q += w_ * (ldg(Ac + (int64_t)mm * J + jj) * ldg(ct + (int64_t)mm * N + k)
-                   + (real ? 0.0 : ldg(As + (int64_t)mm * J + jj) * ldg(st + (int64_t)mm * N + k)));
+// One lane per (mode, part), block 0 mode 0 alone: its sums over theta are chains of their own. What counts is the chain,
+// one fma a row each way; what it reads is loaded a batch of MODES_AHEAD rows ahead, side by side over the modes. With
+// the elimination formed in the chain (two divisions a row) and a mode's rows read one by one it took 809 us at
+// 41x181x361, with tabulated divisors and quotients rounded as the division's 163 us; now 70 us, most
+// of it mode 0's.
+constexpr int MODES_AHEAD = 8;
+
+__global__ void __launch_bounds__(32) baro_modes_kernel(const BaroTables B) {
+    const int J = B.J, NM = B.NM;
+    const int lane = threadIdx.x;
+    const int u = ((int)blockIdx.x - 1) * 32 + lane;         // modes 1 .. NM of part 0, then of part 1
+    const bool zero = blockIdx.x == 0;
+    const int mm = zero ? 0 : (u < NM ? u + 1 : u - NM + 1), part = zero || u < NM ? 0 : 1;
+    if (!zero && (u >= 2 * NM || (part == 1 && 2 * mm == B.N))) return;
+    double* __restrict__ d = (part == 0 ? B.Ac : B.As) + mm;
+    const double* __restrict__ ar = B.ar + mm;
+    const double* __restrict__ rdn = B.rdn + mm;
+    const double* __restrict__ cp = B.cp + mm;
+    const int NU = B.NU;
+    auto warp_sum = [](double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    if (zero) {                                              // the whole warp; then lane 0 solves
+        double yr = 0.0;
+        for (int jj = lane; jj < J; jj += 32) yr += ((jj == 0 || jj == J - 1) ? 1.5 : 1.0) * d[(int64_t)jj * NU];
+        const double f = warp_sum(yr) / B.sums[0];
+        for (int jj = lane; jj < J; jj += 32) {
+            const int64_t o = (int64_t)jj * NU;
+            d[o] = jj == 0 ? 0.0 : d[o] - f * B.abs_sin[jj];
+        }
+        __syncwarp();
     }
-    q /= N;
-    for (int i = 0; i < K.im; i++) p[((int64_t)i * K.jm + (jj + 1)) * K.kp + k] += q;
+    double dprev = 0.0;
+    double x[MODES_AHEAD], c[MODES_AHEAD];
+    auto forward = [&](int j0) {
+#pragma unroll
+        for (int q = 0; q < MODES_AHEAD; q++)
+            if (j0 + q < J) {
+                const int64_t o = (int64_t)(j0 + q) * NU;
+                x[q] = d[o] * rdn[o];
+                c[q] = ar[o];
+            }
+    };
+    const int Jn = zero && lane ? 0 : J;                     // rows this lane solves
+    if (Jn) forward(0);
+    for (int j0 = 0; j0 < Jn; j0 += MODES_AHEAD) {
+        double y[MODES_AHEAD], b[MODES_AHEAD];
+#pragma unroll
+        for (int q = 0; q < MODES_AHEAD; q++) { y[q] = x[q]; b[q] = c[q]; }
+        forward(j0 + MODES_AHEAD);
+#pragma unroll
+        for (int q = 0; q < MODES_AHEAD; q++) {
+            if (j0 + q >= J) break;
+            dprev = fma(-b[q], dprev, y[q]);
+            d[(int64_t)(j0 + q) * NU] = dprev;
+        }
+    }
+    auto backward = [&](int j0) {
+#pragma unroll
+        for (int q = 0; q < MODES_AHEAD; q++)
+            if (j0 - q >= 0) {
+                const int64_t o = (int64_t)(j0 - q) * NU;
+                x[q] = d[o];
+                c[q] = cp[o];
+            }
+    };
+    if (Jn) backward(J - 2);
+    for (int j0 = Jn - 2; j0 >= 0; j0 -= MODES_AHEAD) {
+        double y[MODES_AHEAD], b[MODES_AHEAD];
+#pragma unroll
+        for (int q = 0; q < MODES_AHEAD; q++) { y[q] = x[q]; b[q] = c[q]; }
+        backward(j0 - MODES_AHEAD);
+#pragma unroll
+        for (int q = 0; q < MODES_AHEAD; q++) {
+            if (j0 - q < 0) break;
+            dprev = fma(-b[q], dprev, y[q]);
+            d[(int64_t)(j0 - q) * NU] = dprev;
+        }
+    }
+    if (zero) {
+        __syncwarp();
+        double sq = 0.0;
+        for (int jj = lane; jj < J; jj += 32) sq += B.abs_sin[jj] * d[(int64_t)jj * NU];
+        const double f = warp_sum(sq) / B.sums[1];
+        for (int jj = lane; jj < J; jj += 32) d[(int64_t)jj * NU] -= f;
+    }
+}
+
+// q(j, k) added to every level of the column (PressureSolver.h:684-697)
+__global__ void __launch_bounds__(256) baro_add_kernel(const KConst K, int N, const double* __restrict__ q,
+                                                       double* __restrict__ p) {
+    const int k = blockIdx.x * 32 + threadIdx.x;
+    const int j = 1 + blockIdx.y * 8 + threadIdx.y;
+    if (k >= N || j > K.jm - 2) return;
+    const double v = ldg(q + (int64_t)(j - 1) * N + k);
+    const int i0 = blockIdx.z * 4;
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (i0 + u < K.im) p[((int64_t)(i0 + u) * K.jm + j) * K.kp + k] += v;
 }
 
 }  // namespace
 
-cudaError_t launch_line_pass(const KConst& kc, const ColGeo* geo, const double* src, double* p, double* cpb,
-                             double* dpb, int colour, cudaStream_t s, int* launches) {
+cudaError_t launch_line_table(const KConst& kc, const ColGeo* geo, LineGeo* tab, cudaStream_t s) {
+    line_table_kernel<<<(kc.jm + 63) / 64, 64, 0, s>>>(kc, geo, tab);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_line_pass(const KConst& kc, const LineGeo* tab, const double* src, double* p, double* dpb, int colour,
+                             cudaStream_t s, int* launches) {
     const int nm = (kc.km - 1 + 1) / 2 + 1;
-    line_kernel<<<dim3((nm + 127) / 128, kc.jm - 2), 128, 0, s>>>(kc, geo, src, p, cpb, dpb, colour);
+    line_kernel<<<dim3((nm + LINE_THREADS - 1) / LINE_THREADS, kc.jm - 2), LINE_THREADS, 0, s>>>(kc, tab, src, p, dpb, colour);
     *launches += 1;
     if (((kc.km - 1) & 1) && kc.km - 2 > 0) {
-        line_seam_kernel<<<(kc.jm - 2 + 127) / 128, 128, 0, s>>>(kc, geo, src, p, cpb, dpb, colour);
+        line_seam_kernel<<<(kc.jm - 2 + 127) / 128, 128, 0, s>>>(kc, tab, src, p, dpb, colour);
         *launches += 1;
     }
     return cudaGetLastError();
@@ -322,15 +398,20 @@ cudaError_t launch_mean_shift(const KConst& kc, double* p, const double* mean, c
     return cudaGetLastError();
 }
 
+cudaError_t launch_baro_table(const KConst& kc, const BaroTables& T, cudaStream_t s) {
+    baro_table_kernel<<<(T.NM + 1 + 31) / 32, 32, 0, s>>>(T, kc.inv_dthe2, kc.c43, kc.c13);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_barotropic(const KConst& kc, const ColGeo* geo, const double* src, double* p, const BaroTables& T,
                               cudaStream_t s, int* launches) {
-    const int N = kc.km - 1, J = kc.jm - 2, NM = N / 2;
+    const int N = T.N, J = T.J;
     baro_resid_kernel<<<dim3((N + 127) / 128, J), 128, 0, s>>>(kc, geo, src, p, T.A2, T.R);
-    baro_rowabs_kernel<<<(J + 127) / 128, 128, 0, s>>>(J, N, T.R, T.ra);
-    baro_dft_kernel<<<dim3((J + 127) / 128, NM + 1), 128, 0, s>>>(J, N, NM, T.R, T.ct, T.st, T.ra, T.Ac, T.As);
-    BaroModes B{J, N, NM, kc.inv_dthe2, kc.c43, kc.c13, T.lam, T.sinthe, T.abs_sin, T.Ac, T.As, T.cp, T.dp};
-    baro_modes_kernel<<<(NM + 1 + 63) / 64, 64, 0, s>>>(B);
-    baro_apply_kernel<<<dim3((N + 127) / 128, J), 128, 0, s>>>(kc, J, N, NM, T.Ac, T.As, T.ct, T.st, p);
+    cudaError_t e = launch_baro_forward(T, s);
+    if (e != cudaSuccess) return e;
+    baro_modes_kernel<<<1 + (2 * T.NM + 31) / 32, 32, 0, s>>>(T);
+    if ((e = launch_baro_inverse(T, s)) != cudaSuccess) return e;
+    baro_add_kernel<<<dim3((N + 31) / 32, (J + 7) / 8, (kc.im + 3) / 4), dim3(32, 8), 0, s>>>(kc, N, T.R, p);
     *launches += 5;
     return cudaGetLastError();
 }
