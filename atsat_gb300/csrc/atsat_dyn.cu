@@ -1795,7 +1795,7 @@ int setup_turbulence(atsat_dyn* h) {
     const atsat_dyn_params& p = h->p;
     const atsat_dyn_grid& g = h->g;
     const int im = K.im, jm = K.jm;
-    const int64_t n_tab = 5LL * im + 2LL * jm + (int64_t)im * jm;
+    const int64_t n_tab = 6LL * im + 2LL * jm + (int64_t)im * jm;
     const int64_t total = K.fsz + (int64_t)jm * K.kp + n_tab + 16;
     cudaError_t e = cudaMalloc(&h->turb_buf, (size_t)total * 8);
     if (e != cudaSuccess) { h->turb_buf = nullptr; return fail(h, ATSAT_DYN_E_NOMEM, "turbulence: %s", cudaGetErrorString(e)); }
@@ -1813,6 +1813,7 @@ int setup_turbulence(atsat_dyn* h) {
     double* sinthe = thick + im;
     double* cot = sinthe + jm;
     double* irs = cot + jm;
+    double* tref_dz = irs + (size_t)im * jm;
     const float hl = (float)(p.L_atm * g.dr);           // the model's float layer spacing, km
     const double inv_2dthe = 1.0 / (2.0 * g.dthe), inv_2dphi = 1.0 / (2.0 * g.dphi);
     for (int i = 0; i < im; i++) {
@@ -1830,12 +1831,17 @@ int setup_turbulence(atsat_dyn* h) {
     }
     for (int i = 0; i < im; i++)
         for (int j = 0; j < jm; j++) irs[(size_t)i * jm + j] = inv_2dphi / (rm[i] * sinthe[j]);
+    for (int i = 0; i < im; i++) {
+        const double dz = i > 0 && i < im - 1 ? height[i + 1] - height[i - 1] : 0.0;
+        tref_dz[i] = dz > 0.0 ? p.t_ref / dz : 0.0;
+    }
     double* d = q;
     e = cudaMemcpy(d, t.data(), (size_t)n_tab * 8, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail(h, ATSAT_DYN_E_CUDA, "turbulence tables: %s", cudaGetErrorString(e));
     TurbTables& T = h->ttab;
     T.rm = d; T.inv_rm = d + im; T.inv_rm2dthe = d + 2 * im; T.height_m = d + 3 * im; T.thick_m = d + 4 * im;
     T.sinthe = d + 5 * im; T.cotanthe = d + 5 * im + jm; T.inv_rmsinthe2dphi = d + 5 * im + 2 * jm;
+    T.tref_dz = d + 5 * im + 2 * jm + (int64_t)im * jm;
     T.dr = g.dr; T.dthe = g.dthe; T.dphi = g.dphi;
     return ATSAT_DYN_OK;
 }

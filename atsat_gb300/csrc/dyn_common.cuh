@@ -443,6 +443,7 @@ struct TurbTables {
     const double *rm, *inv_rm, *inv_rm2dthe, *height_m, *thick_m;   // im
     const double *sinthe, *cotanthe;                                // jm: exact-zero guard, no floor
     const double* inv_rmsinthe2dphi;                                // im x jm
+    const double* tref_dz;     // im: t_ref over the distance of the levels above and below (0 where there is none)
     double dr, dthe, dphi, taper_dz;
 };
 cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const atsat_dyn_turb_params& tp,

@@ -2,13 +2,14 @@
 // floors of k* and omega*, the sources of the chosen closure (k-omega SST by default, k-omega, k-epsilon) with
 // the production P_k of the curvature-corrected velocity-gradient tensor and the moist buoyancy sink of k, the
 // floors and caps after the source loop, the zero-gradient copy at i = 0, the eddy-viscosity cap, the seam
-// copy and the two lid corners -- pass for pass in the reference's order, one kernel per pass. ATSAT has no
+// copy and the two lid corners -- in the reference's order of passes. ATSAT has no
 // solid body (cSaturnModel.h:254-255), so the land branches are constant.
 //
 // Per-level and per-row factors come from the host (TurbTables) with the reference's expressions: the model's
 // float layer-height table (cSaturnModel.h:1062-1074), the closure's own sine (exact-zero guard, no floor),
 // inv_2dthe / rm and inv_2dphi / (rm sin). The sources loop reads only the other cells' k* and omega*, which
-// no thread of it writes (the floors run as separate passes), so its result does not depend on the order.
+// no thread of it writes (the floors run as separate passes), so its result does not depend on the order. The default
+// closure (SST) has a source kernel of its own that applies the floors and caps where it reads and writes (sst_kernel).
 #include "dyn_common.cuh"
 
 namespace atsat {
@@ -26,7 +27,10 @@ struct TurbArgs {
     double u_0, t_ref, g, cp_mix, r_mix, R_mix, L_m, nue_air, re_turb, nue_max, k_bg_nd, vel_star_max;
     double dr, dthe, dphi, inv_2dr, abl_height, taper_dz;
     // quotients of constants, formed once on the host
-    double inv_L_m, nue_air_nd, gam_ad, tL2_pr, inv_R_mix, inv_cpR;
+    double inv_L_m, nue_air_nd, gam_ad, tL2_pr, inv_R_mix, inv_cpR, inv_2dr2;
+    double la[3], lb[3], sa[3], sb[3];   // L / R_mix and ep L^2 / (cp R_mix) over liquid and over ice
+    float inv_ys_free_f, nue_air_nd_f;
+    int sst_bound_ok;                // the constants of the FP32 bounds are in range
     double ep[3], lv[3], ls[3], t_0[3];
     TurbTables tab;
     double *u, *v, *w, *t, *rho, *tke, *dis, *tken, *disn, *nue, *tks, *dss, *prod, *vel_star;
@@ -65,6 +69,7 @@ __global__ void __launch_bounds__(256) turb_clamp_in_kernel(const TurbArgs A) {
     A.dis[c] = dmax(DIS_MIN, A.dis[c]);
 }
 
+// k-omega and k-epsilon (SST: sst_kernel)
 __device__ void sources_cell(const TurbArgs& A, int i, int j, int k) {
     const TurbTables& T = A.tab;
     const int64_t c = cidx(A, i, j, k);
@@ -121,43 +126,7 @@ __device__ void sources_cell(const TurbArgs& A, int i, int j, int k) {
     const double Omega = sqrt(W12 * W12 + W13 * W13 + W23 * W23);
     const double L_m = A.L_m;
     double nue, tks, dss;
-    if (A.model == 2) {            // compute_k_omega_SST (Turbulence.h:1020-1106)
-        // GB300 issues two FP64 operations per SM per cycle and a division costs about a dozen: the
-        // quotients here are products with 1 / omega, 1 / y*, 1 / CD and 1 / k (four divisions per cell
-        // instead of fifteen), and those reciprocals are Newton-refined FP32 ones (qdiv) where in range
-        const double a1 = 0.31, bet_star = 0.09, bet1 = 0.0333, bet2 = 0.0368, gam1 = 0.413, gam2 = 0.2, sig_w2 = 1.168;
-        const double inv_bet_star = 1.0 / 0.09;
-        const double nue_air_nd = A.nue_air_nd;
-        const double dz_layer = dmax(1.0, T.thick_m[i - 1 > 0 ? i - 1 : 0]);
-        const double y_phys = A.turb_free ? 1.0e20 : dmax(T.height_m[i] - T.height_m[0], dz_layer);
-        const double y_star = y_phys * A.inv_L_m;
-        const double inv_ys = qdiv(1.0, y_star), inv_ys2 = inv_ys * inv_ys;
-        const double dtkedthe = (tk[c + kp] - tk[c - kp]) * inv_rm2dthe;
-        const double ddisdthe = (ds[c + kp] - ds[c - kp]) * inv_rm2dthe;
-        const double dtkedphi = (tk[ce] - tk[cw]) * inv_rmsinthe2dphi;
-        const double ddisdphi = (ds[ce] - ds[cw]) * inv_rmsinthe2dphi;
-        const double grad_dot = dtkedr * ddisdr + dtkedthe * ddisdthe + dtkedphi * ddisdphi;
-        const double dis_safe = dmax(dsc, 1.0e-20);
-        const double inv_dis = qdiv(1.0, dis_safe);
-        const double CD_kw = dmax(2.0 * sig_w2 * inv_dis * grad_dot, 1.0e-20);
-        const double sq_k = sqrt(tkc);
-        const double t_a = sq_k * inv_bet_star * inv_dis * inv_ys;         // sqrt(k) / (beta* omega y*)
-        const double t_b = 500.0 * nue_air_nd * inv_ys2 * inv_dis;         // 500 nu / (y*^2 omega)
-        const double arg1 = dmin(dmax(t_a, t_b), qdiv(4.0 * sig_w2 * tkc * inv_ys2, CD_kw));
-        const double arg2 = dmax(2.0 * t_a, t_b);
-        const double a1sq = arg1 * arg1;
-        const double F1 = tanh(a1sq * a1sq);
-        const double F2 = tanh(arg2 * arg2);
-        nue = qdiv(a1 * tkc, dmax(a1 * dis_safe, Omega * F2));
-        const double tke_safe = dmax(tkc, 1.0e-20);
-        const double P_k = dmin(prod, 20.0 * bet_star * tke_safe * dis_safe);
-        const double Y_k = bet_star * tke_safe * dis_safe;
-        const double P_w = qdiv((F1 * gam1 + (1.0 - F1) * gam2) * P_k * dis_safe, tke_safe);
-        const double Y_w = (F1 * bet1 + (1.0 - F1) * bet2) * dis_safe * dis_safe;
-        const double D_w = 2.0 * (1.0 - F1) * sig_w2 * inv_dis * grad_dot;
-        tks = P_k - Y_k;
-        dss = P_w - Y_w + D_w;
-    } else if (A.model == 1) {     // compute_k_omega (Turbulence.h:929-1017)
+    if (A.model == 1) {            // compute_k_omega (Turbulence.h:929-1017)
         const double bet_star = 0.09, gam = 0.52, C_lim = 0.875, bet_0 = 0.0708;
         // the reference's quotients by rm 2 dthe, rm sin 2 dphi and 2 dr (rm + 1) as products with the
         // column's reciprocals (one division per cell)
@@ -243,6 +212,236 @@ __device__ void sources_cell(const TurbArgs& A, int i, int j, int k) {
     A.nue[c] = nue;
     A.tks[c] = tks;
     A.dss[c] = dss;
+}
+
+// ---- the SST closure (Turbulence.h:1020-1106 with 628-650, 800-881) ----
+// Comparisons on the integer pipe (a DSETP takes a slot of the FP64 pipe like an addition): non-negative doubles order
+// as their bit patterns.
+__device__ __forceinline__ unsigned long long bits_of(double x) { return (unsigned long long)__double_as_longlong(x); }
+constexpr unsigned long long INF_BITS = 0x7FF0000000000000ull, SIGN_BIT = 0x8000000000000000ull;
+// (lo < x) ? x : lo for lo >= 0 (NaN: lo)
+__device__ __forceinline__ double floor_at(double x, double lo) {
+    const unsigned long long b = bits_of(x);
+    return b > bits_of(lo) && b <= INF_BITS ? x : lo;
+}
+// (hi < x) ? hi : x for x, hi >= 0 or NaN
+__device__ __forceinline__ double cap_at(double x, double hi) {
+    const unsigned long long b = bits_of(x);
+    return b > bits_of(hi) && b <= INF_BITS ? hi : x;
+}
+// clamp3(x, -s, s), s >= 0
+__device__ __forceinline__ double clip_to(double x, double s) {
+    const unsigned long long b = bits_of(x), m = b & ~SIGN_BIT;
+    return m > bits_of(s) && m <= INF_BITS ? __longlong_as_double((long long)(bits_of(s) | (b & SIGN_BIT))) : x;
+}
+// clamp3(x, 0, hi)
+__device__ __forceinline__ double clip_positive(double x, double hi) {
+    const unsigned long long b = bits_of(x);
+    if (b & SIGN_BIT) return b > SIGN_BIT && b <= (SIGN_BIT | INF_BITS) ? 0.0 : x;
+    return cap_at(x, hi);
+}
+__device__ __forceinline__ bool finite_double(double x) { return (bits_of(x) & INF_BITS) != INF_BITS; }
+
+// Menter's blending where it is not negligible: F1, F2 and the eddy viscosity's denominator
+struct SstBlend { double F1, nue; };
+__device__ __noinline__ SstBlend sst_blend(double tkc, double dsc, double inv_dis, double inv_ys, double nue_air_nd,
+                                           double grad_dot, double W2) {
+    const double a1 = 0.31, inv_bet_star = 1.0 / 0.09, sig_w2 = 1.168;
+    const double inv_ys2 = inv_ys * inv_ys;
+    const double CD_kw = dmax(2.0 * sig_w2 * inv_dis * grad_dot, 1.0e-20);
+    const double t_a = sqrt(tkc) * inv_bet_star * inv_dis * inv_ys;        // sqrt(k) / (beta* omega y*)
+    const double t_b = 500.0 * nue_air_nd * inv_ys2 * inv_dis;             // 500 nu / (y*^2 omega)
+    const double arg1 = dmin(dmax(t_a, t_b), qdiv(4.0 * sig_w2 * tkc * inv_ys2, CD_kw));
+    const double arg2 = dmax(2.0 * t_a, t_b);
+    const double a1sq = arg1 * arg1;
+    const double F2 = tanh(arg2 * arg2);
+    return {tanh(a1sq * a1sq), qdiv(a1 * tkc, dmax(a1 * dsc, sqrt(W2) * F2))};
+}
+
+// k* at its background after the source loop (Turbulence.h:634-643)
+__device__ __forceinline__ double sst_floor(const TurbArgs& A, double tk, int j, int k) {
+    double k_bg = A.k_bg_nd;
+    if (!A.turb_free) {
+        const double vs = A.vel_star[(int64_t)j * A.kp + k];
+        k_bg = 0.01 * vs * vs / (sqrt(C_NUE) * A.u_0 * A.u_0);
+    }
+    return dmax(k_bg, tk);
+}
+
+// The sources, the production and the eddy viscosity of one cell, floors and caps included: k* and omega* enter floored
+// (neighbours in the interior too, as the reference's pass before the loop leaves them) and are not written here
+// (turb_floor_kernel does, after every cell has read its neighbours).
+//
+// Bound by the FP64 pipe (two operations per SM per cycle): SST_OPS operations per cell where the reference's expressions
+// term by term, with a pass per floor, took 337 and 1347 us at 41x181x361 (1.50 ms with the passes around them). What
+// went: the tensor products sum to cnue (2 (rr^2 + tt^2 + pp^2) - 2/3 S^2 + (rt + tr)^2 + (rp + pr)^2 + (tp + pt)^2)
+// - 2/3 k S; scales are fused into the differences; quotients share 1 / omega, 1 / k, 1 / rho, 1 / T; comparisons are
+// integer; and the blending functions are evaluated only where FP32 bounds with a margin do not already settle them
+// (F1 < 1e-18 leaves 1 - F1 = 1 and the blended constants at their second values to the last bit, Omega F2 < a1 omega
+// the viscosity's maximum): away from walls, with the closure's y* of 1e20 m, nowhere. SST_NOW
+__global__ void __launch_bounds__(128, 4) sst_kernel(const TurbArgs A) {
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y, i = blockIdx.z;
+    if (!interior(A, i, j, k)) return;
+    const TurbTables& T = A.tab;
+    const int64_t c = cidx(A, i, j, k), P = A.plane, kp = A.kp;
+    const int N = A.km - 1;
+    const int64_t cw = c - k + (A.periodic ? (k == 0 ? N - 1 : k - 1) : k - 1);
+    const int64_t ce = c - k + (A.periodic ? (k == N - 1 ? 0 : k + 1) : k + 1);
+    const double inv_rm = A.curv ? T.inv_rm[i] : 0.0;
+    const double s_r = A.inv_2dr, s_t = T.inv_rm2dthe[i], s_p = T.inv_rmsinthe2dphi[(int64_t)i * A.jm + j];
+
+    // k*, omega* and their gradients' product
+    const double tkc = floor_at(A.tke[c], 0.0), dsc = floor_at(A.dis[c], DIS_MIN);
+    double grad_dot;
+    {
+        const bool up = i < A.im - 2, dn = i > 1, so = j < A.jm - 2, no = j > 1;
+        auto tk = [&](int64_t n, bool in) { const double x = A.tke[n]; return in ? floor_at(x, 0.0) : x; };
+        auto ds = [&](int64_t n, bool in) { const double x = A.dis[n]; return in ? floor_at(x, DIS_MIN) : x; };
+        const double gr = (tk(c + P, up) - tk(c - P, dn)) * (ds(c + P, up) - ds(c - P, dn));
+        const double gt = (tk(c + kp, so) - tk(c - kp, no)) * (ds(c + kp, so) - ds(c - kp, no));
+        const bool edge_e = !A.periodic && k == N - 1, edge_w = !A.periodic && k == 1;
+        const double gp = (tk(ce, !edge_e) - tk(cw, !edge_w)) * (ds(ce, !edge_e) - ds(cw, !edge_w));
+        grad_dot = fma(gr, A.inv_2dr2, fma(gt, s_t * s_t, gp * (s_p * s_p)));
+    }
+    const double inv_dis = in_rcp_range(dsc) ? recip_nr(dsc) : 1.0 / dsc;
+    const double k_over_d = tkc * inv_dis;
+
+    // the velocity-gradient tensor and the production
+    double prod;
+    float W2f;
+    {
+        const double *u = A.u, *v = A.v, *w = A.w;
+        const double u_r = u[c] * inv_rm, v_r = v[c] * inv_rm, w_r = w[c] * inv_rm, cot = T.cotanthe[j];
+        const double rr = (u[c + P] - u[c - P]) * s_r, tr = (v[c + P] - v[c - P]) * s_r, pr = (w[c + P] - w[c - P]) * s_r;
+        const double rt = fma(u[c + kp] - u[c - kp], s_t, -v_r), rp = fma(u[ce] - u[cw], s_p, -w_r);
+        const double tt = fma(v[c + kp] - v[c - kp], s_t, u_r), tp = fma(v[ce] - v[cw], s_p, -(w_r * cot));
+        const double pt = (w[c + kp] - w[c - kp]) * s_t, pp = fma(w[ce] - w[cw], s_p, fma(v_r, cot, u_r));
+        const double S = rr + tt + pp, h = 0.66667 * S;
+        const double a = rt + tr, b = rp + pr, d = tp + pt;
+        const double diag = fma(rr, rr, fma(tt, tt, pp * pp)), off = fma(a, a, fma(b, b, d * d));
+        const double cnue = cap_at(k_over_d, A.nue_max);
+        prod = floor_at(fma(cnue, fma(2.0, diag, fma(-h, S, off)), -(h * tkc)), 0.0);
+        // an upper bound of the rotation rate's square, free of cancellation
+        const float w12 = fabsf(d2f(rt)) + fabsf(d2f(tr)), w13 = fabsf(d2f(rp)) + fabsf(d2f(pr));
+        const float w23 = fabsf(d2f(tp)) + fabsf(d2f(pt));
+        W2f = w12 * w12 + w13 * w13 + w23 * w23;
+    }
+    A.prod[c] = prod;
+
+    const double bet_star = 0.09, bet1 = 0.0333, bet2 = 0.0368, gam1 = 0.413, gam2 = 0.2, sig_w2 = 1.168;
+    double gam = gam2, bet = bet2, d_w = 2.0 * sig_w2, nue = k_over_d;
+    {
+        double y_phys = 1.0e20;
+        if (!A.turb_free)
+            y_phys = dmax(T.height_m[i] - T.height_m[0], dmax(1.0, T.thick_m[i - 1 > 0 ? i - 1 : 0]));
+        // upper bounds of max(t_a, t_b) and of Omega F2 (tanh x <= x), one percent above FP32's rounding
+        const float kf = d2f(tkc), df = d2f(dsc), iyf = A.turb_free ? A.inv_ys_free_f : 1.0f / d2f(y_phys * A.inv_L_m);
+        const float ta = 1.01f * sqrtf(kf) * (1.0f / 0.09f) * iyf / df, tb = 1.01f * 500.0f * A.nue_air_nd_f * iyf * iyf / df;
+        const float m2 = fmaxf(2.0f * ta, tb);
+        const bool settled = fmaxf(ta, tb) < 1.0e-5f && 1.02f * sqrtf(W2f) * m2 * m2 < 0.3f * df && W2f < 1.0e30f &&
+                             df < 1.0e30f && kf < 1.0e30f && A.sst_bound_ok;
+        if (!settled) {
+            // the exact rotation rate, formed again
+            const double *u = A.u, *v = A.v, *w = A.w;
+            const double v_r = v[c] * inv_rm, w_r = w[c] * inv_rm, cot = T.cotanthe[j];
+            const double W12 = fma(u[c + kp] - u[c - kp], s_t, -v_r) - (v[c + P] - v[c - P]) * s_r;
+            const double W13 = fma(u[ce] - u[cw], s_p, -w_r) - (w[c + P] - w[c - P]) * s_r;
+            const double W23 = fma(v[ce] - v[cw], s_p, -(w_r * cot)) - (w[c + kp] - w[c - kp]) * s_t;
+            const SstBlend B = sst_blend(tkc, dsc, inv_dis, qdiv(1.0, y_phys * A.inv_L_m), A.nue_air_nd, grad_dot,
+                                         fma(W12, W12, fma(W13, W13, W23 * W23)));
+            gam = B.F1 * gam1 + (1.0 - B.F1) * gam2;
+            bet = B.F1 * bet1 + (1.0 - B.F1) * bet2;
+            d_w = 2.0 * (1.0 - B.F1) * sig_w2;
+            nue = B.nue;
+        }
+    }
+    const double tke_safe = floor_at(tkc, 1.0e-20);
+    const double kd = tke_safe * dsc, Y_k = bet_star * kd;
+    const double P_k = cap_at(prod, 20.0 * Y_k);
+    const double inv_k = in_rcp_range(tke_safe) ? recip_nr(tke_safe) : 1.0 / tke_safe;
+    double tks = P_k - Y_k;
+    const double P_w = gam * P_k * (dsc * inv_k);
+    const double dss = fma(d_w * inv_dis, grad_dot, fma(-(bet * dsc), dsc, P_w));
+
+    // the buoyancy sink of k (Turbulence.h:800-835): B = -nu_t N^2 / Pr_t, moist N^2 in saturated cells
+    if (A.buoy != 0) {
+        const double Tc = A.t[c] * A.t_ref, tref_dz = T.tref_dz[i];
+        const bool fast_T = in_rcp_range(Tc);
+        if (fast_T || Tc > 0.0) {
+            const double inv_T = fast_T ? recip_nr(Tc) : 1.0 / Tc;
+            double Gam = A.gam_ad, fac = 1.0;
+            if (A.buoy == 3) {
+                double rho = A.r_mix;
+                if (A.local_rho) {
+                    const double r_ = A.rho[c];
+                    if (in_rcp_range(r_) || (r_ > 0.0 && isfinite(r_))) rho = r_;
+                }
+                const double inv_rho = in_rcp_range(rho) ? recip_nr(rho) : 1.0 / rho;
+                const double inv_rT = inv_rho * inv_T;
+                double a = 0.0, b = 0.0;
+                bool moist = false;
+                if (A.r_mix > 0.0 || rho > 0.0) {
+#pragma unroll
+                    for (int n = 0; n < 3; n++) {
+                        const double qc = (floor_at(A.gc[n][c], 0.0) + floor_at(A.gi[n][c], 0.0)) * inv_rho;
+                        if (!(bits_of(qc) > bits_of(1.0e-9) && bits_of(qc) <= INF_BITS)) continue;
+                        const bool liquid = Tc >= A.t_0[n];
+                        const double q = floor_at(A.gv[n][c], 0.0) * inv_rT;
+                        a = fma(liquid ? A.la[n] : A.sa[n], q, a);
+                        b = fma(liquid ? A.lb[n] : A.sb[n], q * inv_T, b);
+                        moist = true;
+                    }
+                }
+                if (moist && finite_double(a + b)) {
+                    fac = 1.0 + a;
+                    Gam = Gam * fac * qdiv(1.0, 1.0 + b);
+                }
+            }
+            if (tref_dz > 0.0) {
+                const double N2 = A.g * inv_T * fma(A.t[c + P] - A.t[c - P], tref_dz, Gam) * fac;
+                const unsigned long long nb = bits_of(N2);
+                const bool positive = nb > 0ull && nb < INF_BITS;
+                if (positive || (A.buoy == 2 && finite_double(N2))) tks = fma(-(floor_at(nue, 0.0) * N2), A.tL2_pr, tks);
+            }
+        }
+    }
+    // the caps after the source loop, from the floored k* (its background) and omega*
+    const double tk_out = sst_floor(A, tkc, j, k);
+    A.nue[c] = clip_positive(nue, A.nue_max);
+    const double d20 = 20.0 * dsc;
+    A.dss[c] = clip_to(dss, d20 * dsc);
+    A.tks[c] = clip_to(tks, d20 * tk_out);
+}
+
+// k* and omega* at their floors (the passes before and after the source loop together)
+__global__ void __launch_bounds__(256) turb_floor_kernel(const TurbArgs A) {
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
+    if (!interior(A, i, j, k)) return;
+    const int64_t c = cidx(A, i, j, k);
+    A.tke[c] = sst_floor(A, floor_at(A.tke[c], 0.0), j, k);
+    A.dis[c] = floor_at(A.dis[c], DIS_MIN);
+}
+
+// The wall copy at i = 0 and the cap of nue on the cells the source kernel leaves alone (no taper: the cap is then
+// idempotent there). blockIdx.z: the planes i = 0 and im-1; the rows j = 0 and jm-1; the meridian km-1, and k = 0 where
+// the seam is not periodic.
+__global__ void __launch_bounds__(128) turb_edges_kernel(const TurbArgs A) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, im = A.im, jm = A.jm, km = A.km;
+    int i, j, k;
+    switch (blockIdx.z) {
+        case 0: case 1: i = blockIdx.z ? im - 1 : 0; j = y; k = x; break;
+        case 2: case 3: i = 1 + y; j = blockIdx.z == 3 ? jm - 1 : 0; k = x; break;
+        default: i = 1 + y; j = 1 + x; k = blockIdx.z == 5 ? 0 : km - 1; break;
+    }
+    if (k >= km || j >= jm || (blockIdx.z >= 2 && i > im - 2) || (blockIdx.z >= 4 && j > jm - 2)) return;
+    const int64_t c = cidx(A, i, j, k);
+    double nue = A.nue[c];
+    if (i == 0) {
+        A.tke[c] = A.tke[c + A.plane];
+        A.dis[c] = A.dis[c + A.plane];
+        nue = A.nue[c + A.plane];
+    }
+    A.nue[c] = clip_positive(nue, A.nue_max);
 }
 
 __global__ void __launch_bounds__(128) turb_sources_kernel(const TurbArgs A) {
@@ -357,9 +556,19 @@ cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const 
     A.tL2_pr = (A.L_m / A.u_0) * (A.L_m / A.u_0) / 0.9;
     A.inv_R_mix = 1.0 / p.R_mix;
     A.inv_cpR = 1.0 / (p.cp_mix * p.R_mix);
+    A.inv_2dr2 = A.inv_2dr * A.inv_2dr;
+    A.inv_ys_free_f = (float)(1.0 / (1.0e20 * A.inv_L_m));
+    A.nue_air_nd_f = (float)A.nue_air_nd;
+    A.sst_bound_ok = A.inv_ys_free_f > 1.0e-30f && A.inv_ys_free_f < 1.0e30f && A.nue_air_nd_f >= 0.0f && A.nue_air_nd_f < 1.0e30f;
     A.abl_height = tp.abl_height;
     A.taper_dz = tab.taper_dz;
     for (int n = 0; n < 3; n++) { A.ep[n] = tp.ep[n]; A.lv[n] = tp.lv[n]; A.ls[n] = tp.ls[n]; A.t_0[n] = tp.t_0[n]; }
+    for (int n = 0; n < 3; n++) {
+        A.la[n] = tp.lv[n] * A.inv_R_mix;
+        A.sa[n] = tp.ls[n] * A.inv_R_mix;
+        A.lb[n] = tp.ep[n] * tp.lv[n] * tp.lv[n] * A.inv_cpR;
+        A.sb[n] = tp.ep[n] * tp.ls[n] * tp.ls[n] * A.inv_cpR;
+    }
     A.tab = tab;
     A.u = f[ATSAT_F_U]; A.v = f[ATSAT_F_V]; A.w = f[ATSAT_F_W]; A.t = f[ATSAT_F_T]; A.rho = f[ATSAT_F_RHO_MIX];
     A.tke = f[ATSAT_F_TKE]; A.dis = f[ATSAT_F_DIS]; A.tken = f[ATSAT_F_TKEN]; A.disn = f[ATSAT_F_DISN];
@@ -373,12 +582,28 @@ cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const 
     const dim3 b8(32, 8), g8((K.km + 31) / 32, (K.jm + 7) / 8, K.im);
     const dim3 b4(32, 4), g4((K.km + 31) / 32, (K.jm + 3) / 4, K.im);
     turb_vel_star_kernel<<<dim3((K.km + 127) / 128, K.jm), 128, 0, s>>>(A);
-    turb_clamp_in_kernel<<<g8, b8, 0, s>>>(A);
-    turb_sources_kernel<<<g4, b4, 0, s>>>(A);
-    turb_clamp_out_kernel<<<g8, b8, 0, s>>>(A);
-    turb_wall_kernel<<<dim3((K.km + 127) / 128, K.jm), 128, 0, s>>>(A);
-    turb_nue_cap_kernel<<<g8, b8, 0, s>>>(A);
-    *launches += 6;
+    const dim3 gw((K.km + 127) / 128, K.jm);
+    if (tp.model == ATSAT_TURB_K_OMEGA_SST) {
+        sst_kernel<<<g4, b4, 0, s>>>(A);
+        turb_floor_kernel<<<g8, b8, 0, s>>>(A);
+        *launches += 3;
+        if (tp.abl_taper) {
+            turb_wall_kernel<<<gw, 128, 0, s>>>(A);
+            turb_nue_cap_kernel<<<g8, b8, 0, s>>>(A);
+            *launches += 2;
+        } else {
+            const int width = K.km > K.jm ? K.km : K.jm, rows = K.jm > K.im ? K.jm : K.im;
+            turb_edges_kernel<<<dim3((width + 127) / 128, rows, p.phi_periodic ? 5 : 6), 128, 0, s>>>(A);
+            *launches += 1;
+        }
+    } else {
+        turb_clamp_in_kernel<<<g8, b8, 0, s>>>(A);
+        turb_sources_kernel<<<g4, b4, 0, s>>>(A);
+        turb_clamp_out_kernel<<<g8, b8, 0, s>>>(A);
+        turb_wall_kernel<<<gw, 128, 0, s>>>(A);
+        turb_nue_cap_kernel<<<g8, b8, 0, s>>>(A);
+        *launches += 6;
+    }
     if (p.phi_periodic) {
         turb_seam_kernel<<<(K.im * K.jm * 8 + 255) / 256, 256, 0, s>>>(A);
         *launches += 1;
