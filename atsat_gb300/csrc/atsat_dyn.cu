@@ -1795,7 +1795,7 @@ int setup_turbulence(atsat_dyn* h) {
     const atsat_dyn_params& p = h->p;
     const atsat_dyn_grid& g = h->g;
     const int im = K.im, jm = K.jm;
-    const int64_t n_tab = 6LL * im + 2LL * jm + (int64_t)im * jm;
+    const int64_t n_tab = 7LL * im + 2LL * jm + 2LL * im * jm;
     const int64_t total = K.fsz + (int64_t)jm * K.kp + n_tab + 16;
     cudaError_t e = cudaMalloc(&h->turb_buf, (size_t)total * 8);
     if (e != cudaSuccess) { h->turb_buf = nullptr; return fail(h, ATSAT_DYN_E_NOMEM, "turbulence: %s", cudaGetErrorString(e)); }
@@ -1814,6 +1814,8 @@ int setup_turbulence(atsat_dyn* h) {
     double* cot = sinthe + jm;
     double* irs = cot + jm;
     double* tref_dz = irs + (size_t)im * jm;
+    double* s_t2 = tref_dz + im;
+    double* s_p2 = s_t2 + im;
     const float hl = (float)(p.L_atm * g.dr);           // the model's float layer spacing, km
     const double inv_2dthe = 1.0 / (2.0 * g.dthe), inv_2dphi = 1.0 / (2.0 * g.dphi);
     for (int i = 0; i < im; i++) {
@@ -1834,6 +1836,8 @@ int setup_turbulence(atsat_dyn* h) {
     for (int i = 0; i < im; i++) {
         const double dz = i > 0 && i < im - 1 ? height[i + 1] - height[i - 1] : 0.0;
         tref_dz[i] = dz > 0.0 ? p.t_ref / dz : 0.0;
+        s_t2[i] = inv_rm2dthe[i] * inv_rm2dthe[i];
+        for (int j = 0; j < jm; j++) s_p2[(size_t)i * jm + j] = irs[(size_t)i * jm + j] * irs[(size_t)i * jm + j];
     }
     double* d = q;
     e = cudaMemcpy(d, t.data(), (size_t)n_tab * 8, cudaMemcpyHostToDevice);
@@ -1842,6 +1846,8 @@ int setup_turbulence(atsat_dyn* h) {
     T.rm = d; T.inv_rm = d + im; T.inv_rm2dthe = d + 2 * im; T.height_m = d + 3 * im; T.thick_m = d + 4 * im;
     T.sinthe = d + 5 * im; T.cotanthe = d + 5 * im + jm; T.inv_rmsinthe2dphi = d + 5 * im + 2 * jm;
     T.tref_dz = d + 5 * im + 2 * jm + (int64_t)im * jm;
+    T.s_t2 = T.tref_dz + im;
+    T.s_p2 = T.s_t2 + im;
     T.dr = g.dr; T.dthe = g.dthe; T.dphi = g.dphi;
     return ATSAT_DYN_OK;
 }

@@ -443,6 +443,7 @@ struct TurbTables {
     const double *rm, *inv_rm, *inv_rm2dthe, *height_m, *thick_m;   // im
     const double *sinthe, *cotanthe;                                // jm: exact-zero guard, no floor
     const double* inv_rmsinthe2dphi;                                // im x jm
+    const double *s_t2, *s_p2; // the squares of inv_rm2dthe and inv_rmsinthe2dphi
     const double* tref_dz;     // im: t_ref over the distance of the levels above and below (0 where there is none)
     double dr, dthe, dphi, taper_dz;
 };

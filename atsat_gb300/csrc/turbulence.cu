@@ -30,6 +30,7 @@ struct TurbArgs {
     double inv_L_m, nue_air_nd, gam_ad, tL2_pr, inv_R_mix, inv_cpR, inv_2dr2;
     double la[3], lb[3], sa[3], sb[3];   // L / R_mix and ep L^2 / (cp R_mix) over liquid and over ice
     float inv_ys_free_f, nue_air_nd_f;
+    int kbg_pos, t0_pos, rmix_pos;   // constants whose signs allow integer comparisons
     int sst_bound_ok;                // the constants of the FP32 bounds are in range
     double ep[3], lv[3], ls[3], t_0[3];
     TurbTables tab;
@@ -265,20 +266,21 @@ __device__ __forceinline__ double sst_floor(const TurbArgs& A, double tk, int j,
         const double vs = A.vel_star[(int64_t)j * A.kp + k];
         k_bg = 0.01 * vs * vs / (sqrt(C_NUE) * A.u_0 * A.u_0);
     }
-    return dmax(k_bg, tk);
+    return A.kbg_pos ? floor_at(tk, k_bg) : dmax(k_bg, tk);
 }
 
 // The sources, the production and the eddy viscosity of one cell, floors and caps included: k* and omega* enter floored
 // (neighbours in the interior too, as the reference's pass before the loop leaves them) and are not written here
 // (turb_floor_kernel does, after every cell has read its neighbours).
 //
-// Bound by the FP64 pipe (two operations per SM per cycle): SST_OPS operations per cell where the reference's expressions
+// Bound by the FP64 pipe (two operations per SM per cycle): about 110 operations per cell where the reference's expressions
 // term by term, with a pass per floor, took 337 and 1347 us at 41x181x361 (1.50 ms with the passes around them). What
 // went: the tensor products sum to cnue (2 (rr^2 + tt^2 + pp^2) - 2/3 S^2 + (rt + tr)^2 + (rp + pr)^2 + (tp + pt)^2)
 // - 2/3 k S; scales are fused into the differences; quotients share 1 / omega, 1 / k, 1 / rho, 1 / T; comparisons are
 // integer; and the blending functions are evaluated only where FP32 bounds with a margin do not already settle them
 // (F1 < 1e-18 leaves 1 - F1 = 1 and the blended constants at their second values to the last bit, Omega F2 < a1 omega
-// the viscosity's maximum): away from walls, with the closure's y* of 1e20 m, nowhere. SST_NOW
+// the viscosity's maximum): away from walls, with the closure's y* of 1e20 m, nowhere. Now 580 us, 0.63 ms a run
+// (four to eight blocks per SM measured alike).
 __global__ void __launch_bounds__(128, 4) sst_kernel(const TurbArgs A) {
     const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y, i = blockIdx.z;
     if (!interior(A, i, j, k)) return;
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(128, 4) sst_kernel(const TurbArgs A) {
         const double gt = (tk(c + kp, so) - tk(c - kp, no)) * (ds(c + kp, so) - ds(c - kp, no));
         const bool edge_e = !A.periodic && k == N - 1, edge_w = !A.periodic && k == 1;
         const double gp = (tk(ce, !edge_e) - tk(cw, !edge_w)) * (ds(ce, !edge_e) - ds(cw, !edge_w));
-        grad_dot = fma(gr, A.inv_2dr2, fma(gt, s_t * s_t, gp * (s_p * s_p)));
+        grad_dot = fma(gr, A.inv_2dr2, fma(gt, T.s_t2[i], gp * T.s_p2[(int64_t)i * A.jm + j]));
     }
     const double inv_dis = in_rcp_range(dsc) ? recip_nr(dsc) : 1.0 / dsc;
     const double k_over_d = tkc * inv_dis;
@@ -380,12 +382,12 @@ __global__ void __launch_bounds__(128, 4) sst_kernel(const TurbArgs A) {
                 const double inv_rT = inv_rho * inv_T;
                 double a = 0.0, b = 0.0;
                 bool moist = false;
-                if (A.r_mix > 0.0 || rho > 0.0) {
+                if (A.rmix_pos || rho > 0.0) {
 #pragma unroll
                     for (int n = 0; n < 3; n++) {
                         const double qc = (floor_at(A.gc[n][c], 0.0) + floor_at(A.gi[n][c], 0.0)) * inv_rho;
                         if (!(bits_of(qc) > bits_of(1.0e-9) && bits_of(qc) <= INF_BITS)) continue;
-                        const bool liquid = Tc >= A.t_0[n];
+                        const bool liquid = A.t0_pos ? bits_of(Tc) >= bits_of(A.t_0[n]) : Tc >= A.t_0[n];   // Tc > 0
                         const double q = floor_at(A.gv[n][c], 0.0) * inv_rT;
                         a = fma(liquid ? A.la[n] : A.sa[n], q, a);
                         b = fma(liquid ? A.lb[n] : A.sb[n], q * inv_T, b);
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(128, 4) sst_kernel(const TurbArgs A) {
                     Gam = Gam * fac * qdiv(1.0, 1.0 + b);
                 }
             }
-            if (tref_dz > 0.0) {
+            if (bits_of(tref_dz) != 0ull) {
                 const double N2 = A.g * inv_T * fma(A.t[c + P] - A.t[c - P], tref_dz, Gam) * fac;
                 const unsigned long long nb = bits_of(N2);
                 const bool positive = nb > 0ull && nb < INF_BITS;
@@ -559,6 +561,9 @@ cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const 
     A.inv_2dr2 = A.inv_2dr * A.inv_2dr;
     A.inv_ys_free_f = (float)(1.0 / (1.0e20 * A.inv_L_m));
     A.nue_air_nd_f = (float)A.nue_air_nd;
+    A.kbg_pos = A.k_bg_nd >= 0.0;
+    A.rmix_pos = p.r_mix > 0.0;
+    A.t0_pos = tp.t_0[0] > 0.0 && tp.t_0[1] > 0.0 && tp.t_0[2] > 0.0;
     A.sst_bound_ok = A.inv_ys_free_f > 1.0e-30f && A.inv_ys_free_f < 1.0e30f && A.nue_air_nd_f >= 0.0f && A.nue_air_nd_f < 1.0e30f;
     A.abl_height = tp.abl_height;
     A.taper_dz = tab.taper_dz;
