@@ -147,9 +147,22 @@ __global__ void __launch_bounds__(256) rk_tracer_kernel(const MixedConstF K, con
     }
 }
 
+// B p_stat / t - buoy for t, p_stat outside the fast quotient's range (t > 0): 1/t refined by one
+// Newton-Raphson step times B p. Called, not inlined: inlined it was if-converted, and its four FP64
+// operations took their slots of the FP64 pipe in every cell.
+__device__ __noinline__ double anomaly_rare(double t, double ps, double r0, double bnum, double buoy) {
+    const double r = fma(r0, fma(-t, r0, 1.0), r0);
+    return ps * bnum * r - buoy;
+}
+
 // Once per step: the FP32 copies of y_n (and w's low word), the stage-0 increment live - y_n, the FP32
-// copies of changed point inputs, and the frozen FP64 terms of the momentum equations.
+// copies of changed point inputs, and the frozen FP64 terms of the momentum equations. PLAIN: the default
+// switches (split metric, no radial Coriolis term, the level-mean buoyancy), compiled in for the same reason
+// as anomaly_rare: 17.1 -> 11.9 FP64 slots a cell, 92.6 -> 76.7 us at 41x181x361 (50 us of FP64 issue, 33 us of
+// memory traffic at the copy rate).
+template <bool PLAIN>
 __global__ void __launch_bounds__(256) mixed_prepare_kernel(const KConst K, const MixedPrep pr) {
+    const bool split = PLAIN || K.metric_split, cor_rad = !PLAIN && pr.cor_rad, legacy = !PLAIN && K.buoy_legacy;
     const int k = blockIdx.x * 32 + threadIdx.x;
     const int j = blockIdx.y * 8 + threadIdx.y;
     const int i = blockIdx.z;
@@ -225,7 +238,7 @@ __global__ void __launch_bounds__(256) mixed_prepare_kernel(const KConst K, cons
     // meridional balance (three fmas) and the buoyancy anomaly (three), twelve operations per cell
     double dpm_the = 0.0;          // the p_metric difference along theta
     float dpmdphi = 0.0f;
-    if (K.metric_split) {
+    if (split) {
         dpm_the = __ldg(pr.p_metric + c + kp) - __ldg(pr.p_metric + c - kp);
         dpmdphi = d2f(__ldg(pr.p_metric + ce) - __ldg(pr.p_metric + cw)) * __ldg(&g->s_phi_f);
     }
@@ -245,7 +258,7 @@ __global__ void __launch_bounds__(256) mixed_prepare_kernel(const KConst K, cons
     const float tf = d2f(t);
     float bps_f;
     double ban = 0.0;
-    if (K.buoy_legacy) {
+    if (legacy) {
         const double bps = (ps + __ldg(p + c)) * pr.bnum;
         bps_f = d2f(bps);
         if (tf > 0.0f) {
@@ -268,22 +281,21 @@ __global__ void __launch_bounds__(256) mixed_prepare_kernel(const KConst K, cons
                 const double q0 = f2d(psf * rf);
                 ban = fma(pr.bnum, fma(fma(-t, q0, ps), r0, q0), -buoy_i);
             } else {
-                const double r = fma(r0, fma(-t, r0, 1.0), r0);
-                ban = ps * pr.bnum * r - buoy_i;
+                ban = anomaly_rare(t, ps, r0, pr.bnum, buoy_i);
             }
         }
     }
     // frozen parts of rhs_u, rhs_v, rhs_w at y_n (RHS_Sat_Turb.cpp:310-350, 388-399, 780-835)
     const double wn = __ldg(pr.yn64[ATSAT_F_W] + c);
     double gu = __ldg(&g->cent_rad_c);
-    if (!K.metric_split) {
+    if (!split) {
         const double vn = __ldg(pr.yn64[ATSAT_F_V] + c);
         // + metric (v^2 + w^2) / rm: rhs_u subtracts transport_u, which carries - metric (RHS_Sat_Turb.cpp:391-395)
         gu += (vn * vn + wn * wn) * __ldg(&g->metric_inv_rm);
     }
-    if (pr.cor_rad) gu -= __ldg(&g->cor_rad_c) * wn;
+    if (cor_rad) gu -= __ldg(&g->cor_rad_c) * wn;
     // w (w cot / r) - Coriolis cor_the w, the centrifugal and the p_metric gradient
-    const double rest = K.metric_split ? fma(-dpm_the, __ldg(&g->s_the), __ldg(&g->cent_the_c)) : __ldg(&g->cent_the_c);
+    const double rest = split ? fma(-dpm_the, __ldg(&g->s_the), __ldg(&g->cent_the_c)) : __ldg(&g->cent_the_c);
     const double gv = fma(wn, fma(wn, __ldg(&g->cot_rm), -__ldg(&g->cor_the_c)), rest);
     pr.fz[FZ_DPR][c] = dpdr;
     pr.fz[FZ_DPTH][c] = dpdthe;
@@ -379,7 +391,9 @@ cudaError_t launch_final_combine(const MixedConstF& kf, const MixedIO& io, int q
 
 cudaError_t launch_mixed_prepare(const KConst& kc, const MixedPrep& pr, cudaStream_t s) {
     dim3 block(32, 8), grid((kc.km + 31) / 32, (kc.jm + 7) / 8, kc.im);
-    mixed_prepare_kernel<<<grid, block, 0, s>>>(kc, pr);
+    const bool plain = kc.metric_split && !pr.cor_rad && !kc.buoy_legacy;
+    plain ? mixed_prepare_kernel<true><<<grid, block, 0, s>>>(kc, pr)
+          : mixed_prepare_kernel<false><<<grid, block, 0, s>>>(kc, pr);
     return cudaGetLastError();
 }
 
