@@ -302,11 +302,20 @@ __device__ __forceinline__ bool cell_buoyancy(const KConst& K, double tc, double
     return isfinite(b);
 }
 
-// |x| < 2^512 (zero and subnormals included), finite: an exponent test on the integer pipe
-__device__ __forceinline__ bool moderate(double x) {
+// rest + the cell's buoyancy, and whether the cell counts. A call that does the sum too: inlined, or with the sum in
+// the caller, it was if-converted, and its FP64 operations took their slots of the FP64 pipe in every cell.
+struct RareSum { double rest; int counts; };
+__device__ __noinline__ RareSum add_buoyancy_rare(const KConst& K, double tc, double pc, double rest) {
+    double b;
+    if (!cell_buoyancy(K, tc, pc, b)) return {rest, 0};
+    return {rest + b, 1};
+}
+
+// |x| < 2^e (zero and subnormals included), finite: an exponent test on the integer pipe
+__device__ __forceinline__ bool below_pow2(double x, uint32_t e) {
     uint32_t lo, hi;
     split_f64(x, lo, hi);
-    return ((hi >> 20) & 0x7FFu) < 1023u + 512u;
+    return ((hi >> 20) & 0x7FFu) < 1023u + e;
 }
 
 // GB300 issues two FP64 operations per SM per cycle, so the per-cell work is three of them: each lane
@@ -315,6 +324,8 @@ __device__ __forceinline__ bool moderate(double x) {
 // weight sum sin(theta_j) * (cells counted). Cells with t outside the reciprocal's range or a huge p
 // ("rest") take the reference's own expression and skip rule. With |p| < 2^512, 1/t < 2^127 and
 // |bc| < 2^256 every fast-path term and sum is finite, as the reference's isfinite test needs.
+// Measured at 41x181x361: 33.8 -> 28 us with the rare path called (5.1 -> 3.9 FP64 slots a cell); two or three warps
+// of a block sharing a running sum's rows changed nothing (28, 27 us), four filled two waves (42 us).
 __global__ void __launch_bounds__(LM_THREADS) level_mean_partial_kernel(const KConst K, const double* __restrict__ t,
                                                                          const double* __restrict__ ps,
                                                                          const double* __restrict__ sin_j,
@@ -322,7 +333,7 @@ __global__ void __launch_bounds__(LM_THREADS) level_mean_partial_kernel(const KC
     const int i = blockIdx.x, chunk = blockIdx.y;
     const int j0 = (int)((int64_t)K.jm * chunk / LM_CHUNKS), j1 = (int)((int64_t)K.jm * (chunk + 1) / LM_CHUNKS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool bc_ok = fabs(K.buoy_c) < 0x1p256;
+    const bool bc_ok = below_pow2(K.buoy_c, 256);
     double sum = 0.0, wsum = 0.0;
     for (int j = j0 + warp; j < j1; j += LM_THREADS / 32) {
         const int64_t row = ((int64_t)i * K.jm + j) * K.kp;
@@ -339,15 +350,13 @@ __global__ void __launch_bounds__(LM_THREADS) level_mean_partial_kernel(const KC
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 if (k0 + q * 32 + lane >= K.km) continue;
-                if (bc_ok && in_rcp_range(tv[q]) && moderate(pv[q])) {
+                if (bc_ok && in_rcp_range(tv[q]) && below_pow2(pv[q], 512)) {
                     rs = fma(pv[q], recip_nr(tv[q]), rs);
                     cnt++;
                 } else {
-                    double b;
-                    if (cell_buoyancy(K, tv[q], pv[q], b)) {
-                        rest += b;
-                        cnt++;
-                    }
+                    const RareSum r = add_buoyancy_rare(K, tv[q], pv[q], rest);
+                    rest = r.rest;
+                    cnt += r.counts;
                 }
             }
         }
@@ -386,8 +395,11 @@ __global__ void level_mean_final_kernel(const KConst K, const double* __restrict
 // 1 / rm(i) (a product instead of the reference's quotient: at most one rounding apart). Six FP64 operations
 // per cell (seven with p_baro): f = (v^2 + w^2) / rm + cor w as two products and two fmas, and the
 // trapezoid acc += dr/2 (f_{i-1} + f_i) as one add and one fma.
+// The next eight levels' loads are in flight while these are summed, and p_baro is a switch of the code: 45.5 -> 39.7 us
+// at 41x181x361 (26 us of FP64 issue).
 constexpr int MS_BATCH = 8;
 
+template <bool BARO>
 __global__ void __launch_bounds__(128) metric_scan_kernel(const KConst K, const double* __restrict__ v,
                                                           const double* __restrict__ w,
                                                           const double* __restrict__ inv_rm,
@@ -399,25 +411,38 @@ __global__ void __launch_bounds__(128) metric_scan_kernel(const KConst K, const 
     if (k >= K.km || j >= K.jm) return;
     const double cor = __ldg(cor_j + j);
     const int64_t c0 = (int64_t)j * K.kp + k;
-    double f_prev = 0.0, acc = 0.0;
-    for (int i0 = 0; i0 < K.im; i0 += MS_BATCH) {
-        double vv[MS_BATCH], ww[MS_BATCH], pb[MS_BATCH];
+    double vv[MS_BATCH], ww[MS_BATCH], pb[MS_BATCH];
+    auto load = [&](int i0) {
 #pragma unroll
         for (int q = 0; q < MS_BATCH; q++) {
             const int64_t c = c0 + (int64_t)(i0 + q) * K.plane;
             const bool in = i0 + q < K.im;
             vv[q] = in ? __ldg(v + c) : 0.0;
             ww[q] = in ? __ldg(w + c) : 0.0;
-            pb[q] = (in && p_baro) ? __ldg(p_baro + c) : 0.0;
+            if (BARO) pb[q] = in ? __ldg(p_baro + c) : 0.0;
         }
+    };
+    const double v0 = __ldg(v + c0), w0 = __ldg(w + c0);
+    load(1);
+    double f_prev = fma(fma(w0, w0, v0 * v0), __ldg(inv_rm), cor * w0), acc = 0.0;
+    pm[c0] = BARO ? acc + __ldg(p_baro + c0) : acc;
+    for (int i0 = 1; i0 < K.im; i0 += MS_BATCH) {
+        double cv[MS_BATCH], cw[MS_BATCH], cb[MS_BATCH];
+#pragma unroll
+        for (int q = 0; q < MS_BATCH; q++) {
+            cv[q] = vv[q];
+            cw[q] = ww[q];
+            if (BARO) cb[q] = pb[q];
+        }
+        load(i0 + MS_BATCH);
 #pragma unroll
         for (int q = 0; q < MS_BATCH; q++) {
             const int i = i0 + q;
             if (i >= K.im) break;
-            const double f = fma(fma(ww[q], ww[q], vv[q] * vv[q]), __ldg(inv_rm + i), cor * ww[q]);
-            if (i > 0) acc = fma(half_dr, f_prev + f, acc);
+            const double f = fma(fma(cw[q], cw[q], cv[q] * cv[q]), __ldg(inv_rm + i), cor * cw[q]);
+            acc = fma(half_dr, f_prev + f, acc);
             f_prev = f;
-            pm[c0 + (int64_t)i * K.plane] = p_baro ? acc + pb[q] : acc;
+            pm[c0 + (int64_t)i * K.plane] = BARO ? acc + cb[q] : acc;
         }
     }
 }
@@ -478,7 +503,8 @@ cudaError_t launch_level_mean(const KConst& kc, const double* t, const double* p
 cudaError_t launch_metric_scan(const KConst& kc, const double* v, const double* w, const double* inv_rm,
                                const double* cor_j, const double* p_baro, double* p_metric, cudaStream_t s) {
     dim3 block(32, 4), grid((kc.km + 31) / 32, (kc.jm + 3) / 4);
-    metric_scan_kernel<<<grid, block, 0, s>>>(kc, v, w, inv_rm, cor_j, p_baro, p_metric, 0.5 * kc.dr);
+    auto kernel = p_baro ? metric_scan_kernel<true> : metric_scan_kernel<false>;
+    kernel<<<grid, block, 0, s>>>(kc, v, w, inv_rm, cor_j, p_baro, p_metric, 0.5 * kc.dr);
     return cudaGetLastError();
 }
 
