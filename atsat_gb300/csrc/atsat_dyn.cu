@@ -539,15 +539,15 @@ bool make_tile_maps(atsat_dyn* h) {
     const CUresult r2 = enc(reinterpret_cast<CUtensorMap*>(h->maps.seam), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
                             dims, strides, box_seam, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const cuuint32_t box_main4[4] = {TILE_BX, TILE_BY, TTILE_BZ, 1};
-    const cuuint32_t box_seam4[4] = {TILE_SEAM_X, TILE_J, TTILE_I, 1};
+    const cuuint32_t box_main4[4] = {TTILE_BX, TTILE_BY, TTILE_BZ, 1};
+    const cuuint32_t box_seam4[4] = {TILE_SEAM_X, TTILE_J, TTILE_I, 1};
     const CUresult r3 = enc(reinterpret_cast<CUtensorMap*>(h->maps.main4), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
                             dims, strides, box_main4, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     const CUresult r4 = enc(reinterpret_cast<CUtensorMap*>(h->maps.seam4), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
                             dims, strides, box_seam4, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const cuuint32_t box_pt4[4] = {TILE_K, TILE_J, TTILE_I, 1};
+    const cuuint32_t box_pt4[4] = {TTILE_K, TTILE_J, TTILE_I, 1};
     const CUresult r5 = enc(reinterpret_cast<CUtensorMap*>(h->maps.pt4), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
                             dims, strides, box_pt4, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1064,13 +1064,29 @@ TracerPlan make_plan_tracer(atsat_dyn* h, const MixedIO& io, int mode) {
         n++;
     };
     const bool dl = io.dl_in[0] != nullptr;
+    pl.first[0] = n;
     add(io.yn32[ATSAT_F_U], 1); if (dl) add(io.dl_in[ATSAT_F_U], 1);
+    pl.first[1] = n;
     add(io.yn32[ATSAT_F_V], 1); if (dl) add(io.dl_in[ATSAT_F_V], 1);
-    add(io.yn32[ATSAT_F_W], 1); add(io.wlo, 1); if (dl) add(io.dl_in[ATSAT_F_W], 1);
     add(io.nue, 1);
+    pl.first[2] = n;
+    add(io.yn32[ATSAT_F_W], 1); add(io.wlo, 1); if (dl) add(io.dl_in[ATSAT_F_W], 1);
+    const MixedConstF& K = h->kf;
+    const float pc = K.precip_coupling, chem = K.chem;
     for (int q = ATSAT_F_H2O; q < NPROG; q++) {
         const bool turb = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
-        pl.first[q - ATSAT_F_H2O] = n;
+        pl.first[TRACER_WIND_GROUPS + q - ATSAT_F_H2O] = n;
+        // the field's diffusivity and source weights (RHS_Sat_Turb.cpp:580-1000 via mixed_physics.cuh)
+        TracerField& F = pl.fld[q - ATSAT_F_H2O];
+        switch (q) {
+            case ATSAT_F_H2O: case ATSAT_F_H2O_CLOUD: case ATSAT_F_H2O_ICE: F = {K.inv_sc_re_h2o, pc, 0.0f, 0.0f}; break;
+            case ATSAT_F_H2S: F = {K.inv_sc_re_h2s, chem, 0.0f, 0.0f}; break;
+            case ATSAT_F_NH3: F = {K.inv_sc_re_nh3, chem, pc, 0.0f}; break;
+            case ATSAT_F_NH3_CLOUD: case ATSAT_F_NH3_ICE: F = {K.inv_sc_re_nh3, pc, 0.0f, 0.0f}; break;
+            case ATSAT_F_CH4: case ATSAT_F_CH4_CLOUD: case ATSAT_F_CH4_ICE: F = {K.inv_sc_re_ch4, pc, 0.0f, 0.0f}; break;
+            case ATSAT_F_NH4SH: F = {K.inv_sc_re_nh4sh, chem, 1.0f, 0.0f}; break;
+            default: F = {K.inv_re, 1.0f, 0.0f, q == ATSAT_F_TKE ? K.inv_sig_k : K.inv_sig_w}; break;
+        }
         if (turb && !h->kc.turb) continue;
         add(io.yn32[q], 0);
         if (dl) add(io.dl_in[q], 0);
@@ -1085,14 +1101,14 @@ TracerPlan make_plan_tracer(atsat_dyn* h, const MixedIO& io, int mode) {
             case ATSAT_F_CH4: add(io.s_precip[6], 1); break;
             case ATSAT_F_CH4_CLOUD: add(io.s_precip[7], 1); break;
             case ATSAT_F_CH4_ICE: add(io.s_precip[8], 1); break;
-            case ATSAT_F_NH4SH: add(io.fluxlim_nh4sh, 1); add(io.massflux_nh4sh, 1); break;
+            case ATSAT_F_NH4SH: add(io.massflux_nh4sh, 1); add(io.fluxlim_nh4sh, 1); break;
             case ATSAT_F_TKE: add(io.tke_source, 1); break;
             default: add(io.dis_source, 1); break;
         }
         if (turb) add(io.acc_turb[q - ATSAT_F_TKE], 1);
         else if (mode == MODE_FINAL) { add(io.dl1[q], 1); add(io.dl2[q], 1); }
     }
-    pl.n_items = pl.first[NPROG - ATSAT_F_H2O] = n;
+    pl.n_items = pl.first[TRACER_WIND_GROUPS + NPROG - ATSAT_F_H2O] = n;
     return pl;
 }
 
@@ -1390,10 +1406,6 @@ int enqueue_rk4_mixed(atsat_dyn* h, bool resident) {
         const int mode = stage == 3 ? MODE_FINAL : MODE_STAGE;
         CK(h, launch_stage(h, io, sp, mode));
         h->launches += launches_per_stage(h, io, mode);
-        // the TMA-tiled tracer kernel leaves the final stage's FP64 sum to launch_final_combine
-        const int v = variant_available(h, h->variant) ? h->variant : ATSAT_DYN_STAGE_DIRECT;
-        if (stage == 3 && (v == ATSAT_DYN_STAGE_SPLIT_TILED || v == ATSAT_DYN_STAGE_TILED2 || v == ATSAT_DYN_STAGE_MARCH))
-            h->launches += 1;
     }
     return ATSAT_DYN_OK;
 }

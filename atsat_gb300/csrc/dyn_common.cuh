@@ -220,7 +220,7 @@ struct MixedIO {
     const float* wlo;              // y_n(w) - yn32(w)
     const float* dl_in[NPROG];     // stage increments; null entries: Y_s = y_n
     float* dl_out[NPROG];          // stages 0..2
-    float* dl1[NPROG];       // final stage: dl_1 and dl_2
+    const float* dl1[NPROG]; // final stage: dl_1 and dl_2
     const float* dl2[NPROG];
     float* acc_turb[2];            // tke, dis
     const double* yn64[NPROG];
@@ -296,8 +296,9 @@ constexpr long long TILE_WAIT_LIMIT = 1LL << 31;   // SM clocks (about a second)
 constexpr int TILE_BX = TILE_K + 8, TILE_BY = TILE_J + 2, TILE_BZ = TILE_I + 2;
 constexpr int TILE_SEAM_X = 4;
 constexpr int TILE_MAX_ITEMS = 2 * NPROG + 1;
-// the tracer kernel's taller tile: four radial levels per thread
-constexpr int TTILE_I = 4, TTILE_BZ = TTILE_I + 2;
+// the tracer kernel's tile: 256 columns, four radial levels per thread
+constexpr int TTILE_K = 64, TTILE_J = 4, TTILE_I = 4;
+constexpr int TTILE_BX = TTILE_K + 8, TTILE_BY = TTILE_J + 2, TTILE_BZ = TTILE_I + 2;
 struct TilePlan {
     int n_items;
     int item[TILE_MAX_ITEMS];
@@ -334,23 +335,29 @@ cudaError_t launch_rk_split(const MixedConstF& kf, const MixedIO& io, const Stag
 struct TileMaps {
     alignas(64) unsigned char main[128];    // box TILE_BX x TILE_BY x TILE_BZ
     alignas(64) unsigned char seam[128];    // box TILE_SEAM_X x TILE_J x TILE_I
-    alignas(64) unsigned char main4[128];   // box TILE_BX x TILE_BY x TTILE_BZ
-    alignas(64) unsigned char seam4[128];   // box TILE_SEAM_X x TILE_J x TTILE_I
-    alignas(64) unsigned char pt4[128];     // box TILE_K x TILE_J x TTILE_I (point values, no halo)
+    alignas(64) unsigned char main4[128];   // box TTILE_BX x TTILE_BY x TTILE_BZ
+    alignas(64) unsigned char seam4[128];   // box TILE_SEAM_X x TTILE_J x TTILE_I
+    alignas(64) unsigned char pt4[128];     // box TTILE_K x TTILE_J x TTILE_I (point values, no halo)
     alignas(64) unsigned char pt2[128];     // box TILE_K x TILE_J x TILE_I (point values, no halo)
     alignas(64) unsigned char plane1[128];  // box TILE_BX x TILE_BY x 1: one radial plane with its halo
     alignas(64) unsigned char seam1[128];   // box TILE_SEAM_X x TILE_J x 1
     alignas(64) unsigned char pt1[128];     // box TILE_K x TILE_J x 1
 };
 
-// The tracer kernel's stream: every array it reads, in consumption order, each either a halo box
-// (kind 0) or a point box (kind 1).
+// A stream of the split stage kernels: every array the kernel reads, in consumption order, each either a halo box
+// (kind 0) or a point box (kind 1). The tracer kernel takes its items in groups, the wind groups and then one per
+// tracer field, a group's halo boxes first.
 constexpr int TRACER_MAX_ITEMS = 96;
+constexpr int TRACER_WIND_GROUPS = 3;
+struct TracerField {
+    float kap0, w0, w1, inv_sig;   // diffusivity, source weights, 1 / sigma of tke or dis
+};
 struct TracerPlan {
     int n_items;
     int arr[TRACER_MAX_ITEMS];
     unsigned char kind[TRACER_MAX_ITEMS];
-    int first[NPROG - ATSAT_F_H2O + 1];   // the first item of each tracer field; the last entry: n_items
+    int first[TRACER_WIND_GROUPS + NPROG - ATSAT_F_H2O + 1];   // the first item of each group; the last entry: n_items
+    TracerField fld[NPROG - ATSAT_F_H2O];
     unsigned int* err;
     long long wait_limit;          // SM clocks before a consumer's or the producer's slot wait gives up
     int withhold;                  // test hook: the producer leaves the last `withhold` items unissued
@@ -433,7 +440,6 @@ cudaError_t launch_clamp_species(const KConst& kc, double* const f[11], float* c
                                  unsigned long long* cells, double* partial, cudaStream_t s);
 
 // the final stage's FP64 half of fields q0..q1 after a tiled stage kernel (rk_mixed.cu)
-cudaError_t launch_final_combine(const MixedConstF& kf, const MixedIO& io, int q0, int q1, cudaStream_t s);
 cudaError_t launch_nonfinite_fields(const KConst& kc, const double* const* f, int n, unsigned long long* count,
                                     cudaStream_t s);
 

@@ -12,7 +12,8 @@ static_assert(march::THREADS == tracer::THREADS, "one block size");
 
 struct FusedGrid {
     int nm, nt;                    // momentum blocks, tracer tiles
-    int nk, nj;
+    int nk, nj, tk, tj;            // their tiles along k and j
+    int ng;                        // field groups per tracer tile
 };
 
 template <int MODE>
@@ -22,7 +23,7 @@ struct Fused {
                                                                                       : tracer::SMEM_BYTES;
 };
 
-template <int MODE, bool HAS_DL, int NG>
+template <int MODE, bool HAS_DL>
 __global__ void __launch_bounds__(march::THREADS, Fused<MODE>::CMP ? 3 : 2)
 rk_stage_fused_kernel(const __grid_constant__ CUtensorMap plane, const __grid_constant__ CUtensorMap plane_seam,
                       const __grid_constant__ CUtensorMap plane_pt, const __grid_constant__ CUtensorMap box,
@@ -32,39 +33,31 @@ rk_stage_fused_kernel(const __grid_constant__ CUtensorMap plane, const __grid_co
     extern __shared__ __align__(128) float smem[];
     // momentum blocks first (they are the longer ones), then the tracer tiles, their field groups side by side
     const bool mom = (int)blockIdx.x < G.nm;
-    const int m = mom ? (int)blockIdx.x : (int)blockIdx.x - G.nm, n = mom ? m : m / NG, g = m - n * NG;
-    const int bx = n % G.nk, r = n / G.nk, by = r % G.nj, bz = r / G.nj;
+    const int m = mom ? (int)blockIdx.x : (int)blockIdx.x - G.nm, n = mom ? m : m / G.ng, g = m - n * G.ng;
+    const int nk = mom ? G.nk : G.tk, nj = mom ? G.nj : G.tj;
+    const int bx = n % nk, r = n / nk, by = r % nj, bz = r / nj;
     if (mom)
         march::block<MODE, HAS_DL, Fused<MODE>::CMP>(plane, plane_seam, plane_pt, K, io, sp, mp, smem, bx, by, bz);
     else
-        tracer::group_block<MODE, HAS_DL, NG>(box, box_seam, box_pt, K, io, sp, tp, smem, bx, by, bz, g);
-}
-
-template <int MODE, bool HAS_DL, int NG>
-cudaError_t launch_groups(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
-                          const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
-    static bool attr = false;
-    constexpr size_t smem = Fused<MODE>::SMEM;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_stage_fused_kernel<MODE, HAS_DL, NG>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
-    auto map = [](const unsigned char* p) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(p); };
-    rk_stage_fused_kernel<MODE, HAS_DL, NG><<<G.nm + G.nt * NG, march::THREADS, smem, s>>>(
-        map(m.plane1), map(m.seam1), map(m.pt1), map(m.main4), map(m.seam4), map(m.pt4), kf, io, sp, mp, tp, G);
-    return cudaGetLastError();
+        tracer::block<MODE, HAS_DL>(box, box_seam, box_pt, K, io, sp, tp, smem, bx, by, bz, tracer::group_q0(G.ng, g),
+                                    tracer::group_q0(G.ng, g + 1));
 }
 
 template <int MODE, bool HAS_DL>
 cudaError_t launch_one(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
-    switch (tracer_groups(G.nt)) {
-        case 13: return launch_groups<MODE, HAS_DL, 13>(m, kf, io, sp, mp, tp, G, s);
-        case 4: return launch_groups<MODE, HAS_DL, 4>(m, kf, io, sp, mp, tp, G, s);
-        default: return launch_groups<MODE, HAS_DL, 1>(m, kf, io, sp, mp, tp, G, s);
+    static bool attr = false;
+    constexpr size_t smem = Fused<MODE>::SMEM;
+    if (!attr) {
+        const cudaError_t e = cudaFuncSetAttribute(rk_stage_fused_kernel<MODE, HAS_DL>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        attr = true;
     }
+    auto map = [](const unsigned char* p) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(p); };
+    rk_stage_fused_kernel<MODE, HAS_DL><<<G.nm + G.nt * G.ng, march::THREADS, smem, s>>>(
+        map(m.plane1), map(m.seam1), map(m.pt1), map(m.main4), map(m.seam4), map(m.pt4), kf, io, sp, mp, tp, G);
+    return cudaGetLastError();
 }
 
 // blocks of the momentum kernel and tiles of the tracer kernel
@@ -73,20 +66,23 @@ FusedGrid fused_grid(int im, int jm, int km, int levels) {
     G.nk = (km - 1 + TILE_K - 1) / TILE_K;
     G.nj = (jm - 4 + TILE_J - 1) / TILE_J;
     if (G.nk <= 0 || G.nj <= 0 || im < 3) return G;
+    G.tk = (km - 1 + TTILE_K - 1) / TTILE_K;
+    G.tj = (jm - 4 + TTILE_J - 1) / TTILE_J;
     G.nm = G.nk * G.nj * ((im - 2 + levels - 1) / levels);
-    G.nt = G.nk * G.nj * ((im - 2 + TTILE_I - 1) / TTILE_I);
+    G.nt = G.tk * G.tj * ((im - 2 + TTILE_I - 1) / TTILE_I);
+    G.ng = tracer_groups(G.nt);
     return G;
 }
 
 }  // namespace
 
 // Up to four waves of resident blocks (three per SM) the stage's two kernels are short enough that their launch and
-// their thin last waves show: one launch takes two iterations at 10x20x36 from 275 to 241 us, 21x60x121 444 -> 422,
-// 21x91x181 608 -> 586, 31x121x241 1149 -> 1122. Beyond, a lone run still gains (41x181x361 replayed 2623 -> 2579 us,
-// 61x271x541 8001 -> 7798), but handles that run concurrently fill those waves with each other's blocks already and
-// lose (three replaying in turn at 41x181x361 2489 -> 2526 us, 81x361x721 18400 -> 18548): the launches stay apart.
+// their thin last waves show: one launch takes two iterations at 10x20x36 from 247 to 214 us, 21x60x121 395 -> 361,
+// 21x91x181 575 -> 549, 31x121x241 1063 -> 1018. Beyond, a lone run still gains (41x181x361 replayed 2408 -> 2351 us,
+// 61x271x541 7457 -> 7238), but handles that run concurrently fill those waves with each other's blocks already and
+// lose (three replaying in turn at 41x181x361 2193 -> 2203 us): the launches stay apart.
 // Interleaving the momentum blocks with the tracer blocks, so that both kinds share an SM, is slower the finer it is
-// (every 3rd block: 2755 us, every 4th: 2820): the two instruction streams evict each other.
+// (with the unrolled tracer code, 2489 us apart: every 3rd block 2755, every 4th 2820).
 bool stage_fusable(const MixedConstF& kf, const MarchPlan& mp, int mode) {
     if (mode != MODE_STAGE || !mp.compact || mp.n_pt > march::Shape<MODE_STAGE, true>::NPT || mp.levels < 1) return false;
     const FusedGrid G = fused_grid(kf.im, kf.jm, kf.km, mp.levels);

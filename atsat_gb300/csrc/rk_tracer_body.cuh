@@ -2,16 +2,23 @@
 // stage handling of RungeKutta_Sat_Turb.cpp:250-375), run after the momentum / temperature kernel of the
 // split variant (rk_mixed.cu) when species_divu is off.
 //
-// A block owns 32 x 8 x 4 cells (k, j, i). A producer warp streams every array the tracers read, in the
-// order the consumers use them, with tensor copies: the halo boxes (40 x 10 x 6 floats) of each field's
-// y_n copy and stage increment into a 4-slot ring, and point boxes (32 x 8 x 4 floats, no halo) of the
-// advecting winds, the eddy viscosity, the sources, the tke/dis running sums and, at the final stage, the
-// increments dl_1 and dl_2 into a 6-slot ring. At the final stage the kernel writes the FP32 increment of
-// y_{n+1} in place of dl_1 and launch_final_combine (rk_mixed.cu) adds it to y_n in FP64: the FP64 loads, adds and stores
-// then stream in a kernel of their own instead of stalling the stencil kernel. Eight consumer warps (row j,
-// lane k, four radial levels per lane) read everything from shared memory, so they never wait on a global
-// load. A field holds at most two halo and four point slots, so a block needs 67 KB of
-// shared memory and three blocks fit on an SM.
+// A block owns 64 x 4 x 4 cells (k, j, i). A producer warp streams every array the tracers read with tensor
+// copies, in groups: the advecting winds and the eddy viscosity (three groups of point boxes, 64 x 4 x 4 floats,
+// no halo), then one group per field: the halo boxes (72 x 6 x 6 floats) of its y_n copy and stage increment and
+// the point boxes of its sources, the tke/dis running sum and, at the final stage, dl_1 and dl_2. A group has one
+// "full" barrier for all of its copies and one "empty" barrier; with increments two groups are in flight, without
+// four. Eight consumer warps (half a row j, lane k, four radial levels per lane) read the boxes from shared memory;
+// at the final stage each lane loads its y_n (FP64) before it waits for the field's boxes and forms y_{n+1} there.
+// A block needs 73 KB of shared memory and 72 registers a thread: three blocks fit on an SM.
+//
+// What bounds it: memory (HBM at 88-93 % of a plain copy's rate at 41x181x361) and, close behind, issue (60 %).
+// Launches at 41x181x361, before -> now: intermediate with increments 144 -> 134 us, final stage with its FP64 half
+// 184 + 118 -> 258 us. 32 x 8 cells per tile read a halo a fifth larger per cell (2221 us a step pair against 2193).
+// Prefetching the next groups into L2 did not help (2209-2240).
+//
+// The fields run through three copies of the code (one source, two sources, tke / dis) in a loop that is not
+// unrolled. With one copy per field the program was 90 KB: at the final stage a warp in eight waited for instructions,
+// and with the FP64 half in it most did (419 us at 41x181x361), which is why that half was a kernel of its own.
 //
 // The arithmetic is mixed_physics.cuh's scalar() with its constant factors folded: with the raw
 // differences a0..a5 of the field (each part differenced on its own),
@@ -26,6 +33,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "mixed_physics.cuh"
 #include "tma_pipe.cuh"
 
@@ -36,141 +45,167 @@ using namespace mixed;
 using namespace tma;
 
 constexpr int TI = TTILE_I;                               // 4 radial levels per thread
-constexpr int PL = TILE_BX * TILE_BY;                     // 400 floats per plane of a halo box
-constexpr int BOX_F = PL * TTILE_BZ;                      // 2400
-constexpr int SEAM_F = TILE_SEAM_X * TILE_J * TI;         // 128
-constexpr int HSLOT_F = BOX_F + SEAM_F;                   // 2528 floats = 10112 bytes (79 x 128)
-constexpr int PSLOT_F = TILE_K * TILE_J * TI;             // 1024 floats = 4096 bytes
+constexpr int PL = TTILE_BX * TTILE_BY;                   // floats per plane of a halo box
+constexpr int BOX_F = PL * TTILE_BZ;
+constexpr int SEAM_F = TILE_SEAM_X * TTILE_J * TI;
+constexpr int HSLOT_F = (BOX_F + SEAM_F + 31) / 32 * 32;
+constexpr int PSLOT_F = TTILE_K * TTILE_J * TI;           // 1024 floats = 4096 bytes
 constexpr uint32_t BOX_BYTES = BOX_F * 4, SEAM_BYTES = SEAM_F * 4, PT_BYTES = PSLOT_F * 4;
-constexpr int NHS = 4, NPS = 6;                           // halo and point slots
-constexpr int NCW = TILE_J;
+constexpr int NHS = 4, NPS = 7;                           // halo and point slots
+constexpr int WPR = TTILE_K / 32;                         // warps per row
+constexpr int NCW = WPR * TTILE_J;
 constexpr int THREADS = (NCW + 1) * 32;
-constexpr int GEO_F = TI * TILE_J * 16;                   // ColGeoF of the block's columns
-constexpr int COEF_F = TI * TILE_J * 4;                   // the four per-column diffusion factors
+constexpr int GEO_F = TI * NCW * 16;                      // ColGeoF of each warp's four columns
+constexpr int COEF_F = TI * NCW * 4;                      // their four diffusion factors
 constexpr size_t SMEM_BYTES = (size_t)NHS * HSLOT_F * 4 + (size_t)NPS * PSLOT_F * 4 + (size_t)(GEO_F + COEF_F) * 4
-                            + 2 * (NHS + NPS) * 8;
+                            + 2 * NHS * 8;
 
 static_assert((HSLOT_F * 4) % 128 == 0 && (PSLOT_F * 4) % 128 == 0 && (BOX_F * 4) % 128 == 0, "slot alignment");
 
 // ---- the stream layout (the host builds the same, make_plan_tracer) ----
+constexpr int NTRACER = NPROG - ATSAT_F_H2O;
 __host__ __device__ constexpr bool turb_field(int q) { return q == ATSAT_F_TKE || q == ATSAT_F_DIS; }
 __host__ __device__ constexpr int n_src(int q) { return (q == ATSAT_F_NH3 || q == ATSAT_F_NH4SH) ? 2 : 1; }
-template <int MODE>
-__host__ __device__ constexpr int n_pt(int q) {
-    return n_src(q) + (turb_field(q) ? 1 : 0) + ((MODE == MODE_FINAL && !turb_field(q)) ? 2 : 0);
+__host__ __device__ constexpr int n_pt(int mode, int q) {
+    return n_src(q) + (turb_field(q) ? 1 : 0) + ((mode == MODE_FINAL && !turb_field(q)) ? 2 : 0);
 }
-template <bool HAS_DL>
-__host__ __device__ constexpr int n_state() { return HAS_DL ? 8 : 5; }   // u, [du], v, [dv], w, wlo, [dw], nue
+// the wind groups' point boxes: u, [du] | v, [dv], nue | w, wlo, [dw]
+constexpr int NWIND = TRACER_WIND_GROUPS;
+__host__ __device__ constexpr int n_wind(bool dl, int g) { return (g == 0 ? 1 : 2) + (dl ? 1 : 0); }
+__host__ __device__ constexpr int n_state(bool dl) { return n_wind(dl, 0) + n_wind(dl, 1) + n_wind(dl, 2); }
+__host__ __device__ constexpr int groups_ahead(bool dl) { return dl ? 2 : 4; }   // NHS halo boxes
+// Field group g of ng: the tracers [group_q0(g), group_q0(g + 1)).
+__host__ __device__ constexpr int group_q0(int ng, int g) { return ATSAT_F_H2O + NTRACER * g / ng; }
+
+// Point slots are handed out in stream order, and a group waits for the release of the group groups_ahead before it:
+// so any groups_ahead consecutive groups of a block's stream must fit the point slots.
+constexpr bool slots_fit(int mode, bool dl, int ng) {
+    for (int g = 0; g < ng; g++) {
+        int n[NWIND + NTRACER] = {}, m = 0;
+        for (int w = 0; w < NWIND; w++) n[m++] = n_wind(dl, w);
+        for (int q = group_q0(ng, g); q < group_q0(ng, g + 1); q++) n[m++] = n_pt(mode, q);
+        for (int a = 0; a < m; a++) {
+            int s = 0;
+            for (int b = a; b < m && b < a + groups_ahead(dl); b++) s += n[b];
+            if (s > NPS) return false;
+        }
+    }
+    return true;
+}
+static_assert(slots_fit(MODE_STAGE, false, 1) && slots_fit(MODE_STAGE, false, 4) && slots_fit(MODE_STAGE, false, 13) &&
+              slots_fit(MODE_STAGE, true, 1) && slots_fit(MODE_STAGE, true, 4) && slots_fit(MODE_STAGE, true, 13) &&
+              slots_fit(MODE_FINAL, true, 1) && slots_fit(MODE_FINAL, true, 4) && slots_fit(MODE_FINAL, true, 13),
+              "point slots");
+
+// One array's stencil of a lane's column of TI cells: the centre values at i-1 and i stay in registers from cell to
+// cell, so a cell costs five shared loads instead of seven.
+struct Column {
+    float rn, x;                   // the values at i-1 and i
+
+    __device__ __forceinline__ void start(const float* s, int o) {
+        rn = s[o - PL];
+        x = s[o];
+    }
+    // the raw differences of cell i; returns its centre value and moves on to i+1
+    __device__ __forceinline__ float d7(const float* s, int o, int ow, int oe, float* e) {
+        const float rp = s[o + PL];
+        const float tp = s[o + TTILE_BX], tn = s[o - TTILE_BX];
+        const float pe = s[oe], pw = s[ow];
+        const float c = x;
+        e[0] = rp - rn;
+        e[1] = rp - 2.0f * c + rn;
+        e[2] = tp - tn;
+        e[3] = tp - 2.0f * c + tn;
+        e[4] = pe - pw;
+        e[5] = pe - 2.0f * c + pw;
+        rn = c;
+        x = rp;
+        return c;
+    }
+};
+
+// A global store that the compiler may move shared loads across (a plain one could alias them as far as it knows, and
+// each cell's loads would wait for the stores of the cell before); it stays ahead of the slot's release, which is
+// volatile too.
+__device__ __forceinline__ void store(float* p, float x) {
+    asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(x));
+}
+__device__ __forceinline__ void store(double* p, double x) {
+    asm volatile("st.global.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(x));
+}
+
+// the tracers [q0, q1) of tile (bx, by, bz): the winds' groups, then those fields' groups of the plan
 template <int MODE, bool HAS_DL>
-__host__ __device__ constexpr int pt0(int q) {
-    int n = n_state<HAS_DL>();
-    for (int r = ATSAT_F_H2O; r < q; r++) n += n_pt<MODE>(r);
-    return n;
-}
-template <bool HAS_DL>
-__host__ __device__ constexpr int h0(int q) { return (q - ATSAT_F_H2O) * (HAS_DL ? 2 : 1); }
-
-template <int NS>
-__device__ __forceinline__ bool wait_items(const Ring& rg, int n0, int n1, long long limit) {
-    bool ok = true;
-#pragma unroll
-    for (int n = n0; n < n1; n++) ok = ok && mbar_wait(rg.full(n % NS), (uint32_t)((n / NS) & 1), limit);
-    return !__any_sync(0xffffffffu, !ok);
-}
-
-__device__ __forceinline__ void d7(const float* s, int o, int ow, int oe, float* e) {
-    const float x = s[o];
-    const float rp = s[o + PL], rn = s[o - PL];
-    const float tp = s[o + TILE_BX], tn = s[o - TILE_BX];
-    const float pe = s[oe], pw = s[ow];
-    e[0] = rp - rn;
-    e[1] = rp - 2.0f * x + rn;
-    e[2] = tp - tn;
-    e[3] = tp - 2.0f * x + tn;
-    e[4] = pe - pw;
-    e[5] = pe - 2.0f * x + pw;
-}
-
-// Field group g of NG: the tracers [group_q0(g), group_q0(g + 1)).
-constexpr int NTRACER = NPROG - ATSAT_F_H2O;
-template <int NG>
-__host__ __device__ constexpr int group_q0(int g) { return ATSAT_F_H2O + NTRACER * g / NG; }
-
-// the tracers [Q0, Q1) of tile (bx, by, bz): the winds' items, then those fields' items of the plan
-template <int MODE, bool HAS_DL, int Q0, int Q1>
 __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtensorMap& map_seam, const CUtensorMap& map_pt,
                                       const MixedConstF& K, const MixedIO& io, const StageParams& sp,
-                                      const TracerPlan& plan, float* smem, int bx, int by, int bz) {
+                                      const TracerPlan& plan, float* smem, int bx, int by, int bz, int q0, int q1) {
+    static_assert(MODE == MODE_STAGE || (MODE == MODE_FINAL && HAS_DL), "stages of the stream layout");
+    constexpr int NH = HAS_DL ? 2 : 1, AHEAD = groups_ahead(HAS_DL);
     float* hs = smem;
     float* ps = hs + NHS * HSLOT_F;
     float* sgeo = ps + NPS * PSLOT_F;
     float* scoef = sgeo + GEO_F;
     uint64_t* bars = reinterpret_cast<uint64_t*>(scoef + COEF_F);
-    const Ring rh{smem_u32(bars), smem_u32(bars + NHS)};
-    const Ring rp{smem_u32(bars + 2 * NHS), smem_u32(bars + 2 * NHS + NPS)};
+    const Ring rg{smem_u32(bars), smem_u32(bars + AHEAD)};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    const int k0 = bx * TILE_K;
-    const int j0 = 2 + by * TILE_J;
+    const int k0 = bx * TTILE_K;
+    const int j0 = 2 + by * TTILE_J;
     const int i0 = 1 + bz * TI;
     int seam = 0, xs = 0;
-    if (k0 == 0 && K.km - 2 > k0 + TILE_K + 3) { seam = 1; xs = (K.km - 2) & ~3; }
-    else if (k0 > 0 && K.km - 2 >= k0 && K.km - 2 < k0 + TILE_K) { seam = 2; xs = 0; }
+    if (k0 == 0 && K.km - 2 > k0 + TTILE_K + 3) { seam = 1; xs = (K.km - 2) & ~3; }
+    else if (k0 > 0 && K.km - 2 >= k0 && K.km - 2 < k0 + TTILE_K) { seam = 2; xs = 0; }
 
     if (smem_u32(smem) & 127u) {
         if (threadIdx.x == 0) atomicOr(plan.err, ERR_ALIGN);
         return;
     }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NHS; s++) { mbar_init(rh.full(s), 1); mbar_init(rh.empty(s), NCW); }
-        for (int s = 0; s < NPS; s++) { mbar_init(rp.full(s), 1); mbar_init(rp.empty(s), NCW); }
+        for (int s = 0; s < AHEAD; s++) { mbar_init(rg.full(s), 1); mbar_init(rg.empty(s), NCW); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
 
+    const int q_end = K.turb ? q1 : (q1 < ATSAT_F_TKE ? q1 : ATSAT_F_TKE);   // tke and dis come last
+
     if (warp == NCW) {
-        // ---- producer: the plan's items in order, each to its ring ----
+        // ---- producer: the plan's groups in order ----
         if (lane == 0) {
-            int nh = 0, np = 0;
+            const int ng = NWIND + (q_end > q0 ? q_end - q0 : 0);
+            const int last = plan.first[NWIND + (q_end > q0 ? q_end : q0) - ATSAT_F_H2O] - plan.withhold;
+            int n = 0, pslot = 0;
             bool ok = true;
-            constexpr int NST = n_state<HAS_DL>();
-            const int skip = Q0 == ATSAT_F_H2O ? 0 : plan.first[Q0 - ATSAT_F_H2O] - NST;   // other groups' items
-            const int n_issue = plan.first[Q1 - ATSAT_F_H2O] - skip - plan.withhold;
-            for (int m = 0; m < n_issue && ok; m++) {
-                const int n = m < NST ? m : m + skip;
-                if (plan.kind[n] == 0) {
-                    const int s = nh % NHS;
-                    if (nh >= NHS && !mbar_wait(rh.empty(s), (uint32_t)(((nh / NHS) - 1) & 1), plan.wait_limit)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dst = smem_u32(hs + s * HSLOT_F);
-                    mbar_expect_tx(rh.full(s), BOX_BYTES + (seam ? SEAM_BYTES : 0u));
-                    tma_load_4d(dst, &map_main, k0 - 4, j0 - 1, i0 - 1, plan.arr[n], rh.full(s));
-                    if (seam) tma_load_4d(dst + BOX_BYTES, &map_seam, xs, j0, i0, plan.arr[n], rh.full(s));
-                    nh++;
-                } else {
-                    const int s = np % NPS;
-                    if (np >= NPS && !mbar_wait(rp.empty(s), (uint32_t)(((np / NPS) - 1) & 1), plan.wait_limit)) {
-                        ok = false;
-                        break;
-                    }
-                    mbar_expect_tx(rp.full(s), PT_BYTES);
-                    tma_load_4d(smem_u32(ps + s * PSLOT_F), &map_pt, k0, j0, i0, plan.arr[n], rp.full(s));
-                    np++;
+            for (; n < ng; n++) {
+                const int g = n < NWIND ? n : n + (q0 - ATSAT_F_H2O);
+                const int m0 = plan.first[g], m1 = plan.first[g + 1], nh = n < NWIND ? 0 : NH, s = n % AHEAD;
+                if (m1 > last) break;                       // withheld
+                if (n >= AHEAD && !mbar_wait(rg.empty(s), (uint32_t)(((n / AHEAD) - 1) & 1), plan.wait_limit)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t bar = rg.full(s);
+                mbar_expect_tx(bar, nh * (BOX_BYTES + (seam ? SEAM_BYTES : 0u)) + (m1 - m0 - nh) * PT_BYTES);
+                for (int m = m0; m < m0 + nh; m++) {
+                    const uint32_t dst = smem_u32(hs + (s * NH + m - m0) * HSLOT_F);
+                    tma_load_4d(dst, &map_main, k0 - 4, j0 - 1, i0 - 1, plan.arr[m], bar);
+                    if (seam) tma_load_4d(dst + BOX_BYTES, &map_seam, xs, j0, i0, plan.arr[m], bar);
+                }
+                for (int m = m0 + nh; m < m1; m++) {
+                    tma_load_4d(smem_u32(ps + pslot * PSLOT_F), &map_pt, k0, j0, i0, plan.arr[m], bar);
+                    pslot = pslot + 1 == NPS ? 0 : pslot + 1;
                 }
             }
             if (!ok) atomicOr(plan.err, ERR_PRODUCER);
-            for (int m = (nh > NHS ? nh - NHS : 0); m < nh; m++)
-                if (!mbar_wait(rh.full(m % NHS), (uint32_t)((m / NHS) & 1))) break;
-            for (int m = (np > NPS ? np - NPS : 0); m < np; m++)
-                if (!mbar_wait(rp.full(m % NPS), (uint32_t)((m / NPS) & 1))) break;
+            // a copy in flight lands by itself: none may land after the block is gone
+            for (int m = (n > AHEAD ? n - AHEAD : 0); m < n; m++)
+                if (!mbar_wait(rg.full(m % AHEAD), (uint32_t)((m / AHEAD) & 1))) break;
         }
         return;
     }
 
     // ---- consumers ----
-    const int j = j0 + warp, k = k0 + lane;
+    const int row_j = warp / WPR, kl = warp % WPR * 32 + lane;   // the lane's place in the tile
+    const int j = j0 + row_j, k = k0 + kl;
     {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -179,12 +214,12 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
             const int i = i0 + ii;
             float v = 0.0f;
             if (i < K.im && j < K.jm) v = __ldg(reinterpret_cast<const float*>(io.geof + ((int64_t)i * K.jm + j)) + f);
-            sgeo[(ii * TILE_J + warp) * 16 + f] = v;
+            sgeo[(ii * NCW + warp) * 16 + f] = v;
         }
         __syncwarp();
         if (lane < TI) {
-            const ColGeoF& g = *reinterpret_cast<const ColGeoF*>(sgeo + (lane * TILE_J + warp) * 16);
-            float* cf = scoef + (lane * TILE_J + warp) * 4;
+            const ColGeoF& g = *reinterpret_cast<const ColGeoF*>(sgeo + (lane * NCW + warp) * 16);
+            float* cf = scoef + (lane * NCW + warp) * 4;
             cf[0] = K.inv_2dr * g.two_inv_rm;
             cf[1] = K.inv_dthe2 * g.inv_rm2;
             cf[2] = K.inv_2dthe * g.costhe_inv_rm2sinthe;
@@ -192,179 +227,165 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
         }
         __syncwarp();
     }
-    bool valid[TI];
-    int c[TI], o[TI], ow[TI], oe[TI], pidx[TI];
-#pragma unroll
-    for (int ii = 0; ii < TI; ii++) {
-        const int i = i0 + ii;
-        valid[ii] = (k <= K.km - 2) && (j <= K.jm - 3) && (i <= K.im - 2);
-        c[ii] = (i * K.jm + j) * K.kp + k;
-        const int row = (1 + ii) * PL + (warp + 1) * TILE_BX;
-        o[ii] = row + lane + 4;
-        ow[ii] = o[ii] - 1;
-        oe[ii] = o[ii] + 1;
-        if (k == 0)
-            ow[ii] = (seam == 1) ? BOX_F + (ii * TILE_J + warp) * TILE_SEAM_X + ((K.km - 2) - xs)
-                                 : row + (K.km - 2) - (k0 - 4);
-        if (k == K.km - 2)
-            oe[ii] = (seam == 2) ? BOX_F + (ii * TILE_J + warp) * TILE_SEAM_X + (0 - xs) : row + 0 - (k0 - 4);
-        pidx[ii] = (ii * TILE_J + warp) * TILE_K + lane;
+    // the lane's cells: c0 + ii plane for ii < nv; their places in a halo box: o + ii PL, the neighbours in k at
+    // ow + ii ows and oe + ii oes (in the seam box for the periodic partner)
+    const int nv = (k <= K.km - 2 && j <= K.jm - 3) ? K.im - 1 - i0 : 0;
+    const int c0 = (i0 * K.jm + j) * K.kp + k, plane = (int)K.plane;
+    const int row = PL + (row_j + 1) * TTILE_BX;
+    const int o = row + kl + 4;
+    int ow = o - 1, oe = o + 1, ows = PL, oes = PL;
+    if (k == 0) {
+        if (seam == 1) { ow = BOX_F + row_j * TILE_SEAM_X + ((K.km - 2) - xs); ows = TTILE_J * TILE_SEAM_X; }
+        else ow = row + (K.km - 2) - (k0 - 4);
     }
-    auto fail = [&]() { if (lane == 0) atomicOr(plan.err, ERR_CONSUMER); };
+    if (k == K.km - 2) {
+        if (seam == 2) { oe = BOX_F + row_j * TILE_SEAM_X + (0 - xs); oes = TTILE_J * TILE_SEAM_X; }
+        else oe = row + 0 - (k0 - 4);
+    }
+    const int px = row_j * TTILE_K + kl;                      // the lane's place in a point box's plane
+    constexpr int PP = TTILE_J * TTILE_K;                     // floats per plane of a point box
+    auto wait = [&](int n) -> bool {
+        const bool ok = mbar_wait(rg.full(n % AHEAD), (uint32_t)((n / AHEAD) & 1), plan.wait_limit);
+        if (!__any_sync(0xffffffffu, !ok)) return true;
+        if (lane == 0) atomicOr(plan.err, ERR_CONSUMER);
+        return false;
+    };
+    auto release = [&](int n) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rg.empty(n % AHEAD));
+    };
 
-    // ---- the winds and the eddy viscosity: point items u, [du] | v, [dv] | w, wlo, [dw] | nue ----
+    // ---- the winds and the eddy viscosity: point boxes u, [du] | v, [dv], nue | w, wlo, [dw] ----
     float tu[TI], tv[TI], tw[TI], nts[TI], nuec[TI];
     {
-        constexpr int DL = HAS_DL ? 1 : 0;
-        constexpr int nU = 0, nV = 1 + DL, nW = 2 + 2 * DL, nN = 4 + 3 * DL;
-        // u
-        if (!wait_items<NPS>(rp, nU, nV, plan.wait_limit)) { fail(); return; }
+        constexpr int sV = n_wind(HAS_DL, 0), sW = sV + n_wind(HAS_DL, 1);
+        const float* p = ps + px;
+        auto P = [&](int slot, int ii) { return p[(slot % NPS) * PSLOT_F + ii * PP]; };
+        if (!wait(0)) return;
 #pragma unroll
         for (int ii = 0; ii < TI; ii++) {
-            const int x = pidx[ii];
-            const float u = HAS_DL ? ps[(nU % NPS) * PSLOT_F + x] + ps[((nU + 1) % NPS) * PSLOT_F + x]
-                                   : ps[(nU % NPS) * PSLOT_F + x];
+            const float u = HAS_DL ? P(0, ii) + P(1, ii) : P(0, ii);
             tu[ii] = u * K.inv_2dr;
         }
         slot_reads_done();
-        release<NPS>(rp, nU, nV);
-        // v
-        if (!wait_items<NPS>(rp, nV, nW, plan.wait_limit)) { fail(); return; }
+        release(0);
+        if (!wait(1)) return;
 #pragma unroll
         for (int ii = 0; ii < TI; ii++) {
-            const int x = pidx[ii];
-            const float v = HAS_DL ? ps[(nV % NPS) * PSLOT_F + x] + ps[((nV + 1) % NPS) * PSLOT_F + x]
-                                   : ps[(nV % NPS) * PSLOT_F + x];
-            const ColGeoF& g = *reinterpret_cast<const ColGeoF*>(sgeo + (ii * TILE_J + warp) * 16);
+            const float v = HAS_DL ? P(sV, ii) + P(sV + 1, ii) : P(sV, ii);
+            const ColGeoF& g = *reinterpret_cast<const ColGeoF*>(sgeo + (ii * NCW + warp) * 16);
             tv[ii] = v * (K.inv_2dthe * g.inv_rm);
-        }
-        slot_reads_done();
-        release<NPS>(rp, nV, nW);
-        // w = (y_n + low word) + increment
-        if (!wait_items<NPS>(rp, nW, nN, plan.wait_limit)) { fail(); return; }
-#pragma unroll
-        for (int ii = 0; ii < TI; ii++) {
-            const int x = pidx[ii];
-            float w = ps[(nW % NPS) * PSLOT_F + x] + ps[((nW + 1) % NPS) * PSLOT_F + x];
-            if (HAS_DL) w = w + ps[((nW + 2) % NPS) * PSLOT_F + x];
-            const ColGeoF& g = *reinterpret_cast<const ColGeoF*>(sgeo + (ii * TILE_J + warp) * 16);
-            tw[ii] = w * (K.inv_2dphi * g.inv_rmsinthe);
-        }
-        slot_reads_done();
-        release<NPS>(rp, nW, nN);
-        // nue
-        if (!wait_items<NPS>(rp, nN, nN + 1, plan.wait_limit)) { fail(); return; }
-#pragma unroll
-        for (int ii = 0; ii < TI; ii++) {
-            const float nue_c = ps[(nN % NPS) * PSLOT_F + pidx[ii]];
+            const float nue_c = P(sW - 1, ii);
             const float nue_t = (K.turb_coupling != 0.0f && isfinite(nue_c)) ? K.turb_coupling * smaxf(0.0f, nue_c) : 0.0f;
             nts[ii] = nue_t * K.inv_pr_t;
             nuec[ii] = nue_c;
         }
         slot_reads_done();
-        release<NPS>(rp, nN, nN + 1);
-        static_assert(nN + 1 == n_state<HAS_DL>(), "state items");
-    }
-
-    const int q_last = K.turb ? ATSAT_F_DIS : ATSAT_F_NH4SH;
-    const float pc = K.precip_coupling, chem = K.chem;
-#pragma unroll
-    for (int q = Q0; q < Q1; q++) {
-        if (q > q_last) break;
-        const int hb = h0<HAS_DL>(q) - h0<HAS_DL>(Q0), npq = n_pt<MODE>(q);
-        const int pb = pt0<MODE, HAS_DL>(q) - pt0<MODE, HAS_DL>(Q0) + n_state<HAS_DL>();
-        if (!wait_items<NHS>(rh, hb, hb + (HAS_DL ? 2 : 1), plan.wait_limit) ||
-            !wait_items<NPS>(rp, pb, pb + npq, plan.wait_limit)) {
-            fail();
-            return;
-        }
-        const float* Y = hs + (hb % NHS) * HSLOT_F;
-        const float* D = hs + ((hb + 1) % NHS) * HSLOT_F;
-        const float* P0 = ps + (pb % NPS) * PSLOT_F;
-        const float* P1 = ps + ((pb + 1) % NPS) * PSLOT_F;
-        const float* P2 = ps + ((pb + 2) % NPS) * PSLOT_F;
-        const float* P3 = ps + ((pb + 3) % NPS) * PSLOT_F;
-        // the field's diffusivity and source weights (RHS_Sat_Turb.cpp:580-1000 via mixed_physics.cuh)
-        float kap0, w0 = 0.0f, w1 = 0.0f;
-        switch (q) {
-            case ATSAT_F_H2O: case ATSAT_F_H2O_CLOUD: case ATSAT_F_H2O_ICE: kap0 = K.inv_sc_re_h2o; w0 = pc; break;
-            case ATSAT_F_H2S: kap0 = K.inv_sc_re_h2s; w0 = chem; break;
-            case ATSAT_F_NH3: kap0 = K.inv_sc_re_nh3; w0 = chem; w1 = pc; break;
-            case ATSAT_F_NH3_CLOUD: case ATSAT_F_NH3_ICE: kap0 = K.inv_sc_re_nh3; w0 = pc; break;
-            case ATSAT_F_CH4: case ATSAT_F_CH4_CLOUD: case ATSAT_F_CH4_ICE: kap0 = K.inv_sc_re_ch4; w0 = pc; break;
-            case ATSAT_F_NH4SH: kap0 = K.inv_sc_re_nh4sh; w0 = 1.0f; w1 = chem; break;
-            default: kap0 = K.inv_re; w0 = 1.0f; break;   // tke, dis: source weight 1
-        }
-        const float inv_sig = (q == ATSAT_F_TKE) ? K.inv_sig_k : K.inv_sig_w;
+        release(1);
+        // w = (y_n + low word) + increment
+        if (!wait(2)) return;
 #pragma unroll
         for (int ii = 0; ii < TI; ii++) {
-            if (!valid[ii]) continue;
+            float w = P(sW, ii) + P(sW + 1, ii);
+            if (HAS_DL) w = w + P(sW + 2, ii);
+            const ColGeoF& g = *reinterpret_cast<const ColGeoF*>(sgeo + (ii * NCW + warp) * 16);
+            tw[ii] = w * (K.inv_2dphi * g.inv_rmsinthe);
+        }
+        slot_reads_done();
+        release(2);
+    }
+
+    int pslot = n_state(HAS_DL) % NPS;                        // the next point slot
+    // field q, group n of the stream
+    auto field = [&](auto nsrc, auto is_turb_field, int q, int n) -> bool {
+        constexpr int NSRC = decltype(nsrc)::value;
+        constexpr bool TURB = decltype(is_turb_field)::value;
+        constexpr int NPT = NSRC + (TURB ? 1 : 0) + ((MODE == MODE_FINAL && !TURB) ? 2 : 0);
+        double yn64[TI];                                      // the final stage's y_n: in flight during the wait
+        if (MODE == MODE_FINAL) {
+            const double* y = io.yn64[q] + c0;
+#pragma unroll
+            for (int ii = 0; ii < TI; ii++) yn64[ii] = ii < nv ? ldd(y + (int64_t)ii * plane) : 0.0;
+        }
+        const TracerField F = plan.fld[q - ATSAT_F_H2O];
+        if (!wait(n)) return false;
+        const float* Y = hs + (n % AHEAD) * NH * HSLOT_F;
+        const float* D = Y + HSLOT_F;
+        const float* P[NPT];
+#pragma unroll
+        for (int m = 0; m < NPT; m++) {
+            P[m] = ps + pslot * PSLOT_F + px;
+            pslot = pslot + 1 == NPS ? 0 : pslot + 1;
+        }
+        Column cy, cd;
+        cy.start(Y, o);
+        if (HAS_DL) cd.start(D, o);
+#pragma unroll
+        for (int ii = 0; ii < TI; ii++) {
+            // cells outside the interior compute on the box's zeros and store nothing
             float a[6];
-            d7(Y, o[ii], ow[ii], oe[ii], a);
+            const float yn_c = cy.d7(Y, o + ii * PL, ow + ii * ows, oe + ii * oes, a);
+            float dl_c = 0.0f;
             if (HAS_DL) {
                 float b[6];
-                d7(D, o[ii], ow[ii], oe[ii], b);
+                dl_c = cd.d7(D, o + ii * PL, ow + ii * ows, oe + ii * oes, b);
 #pragma unroll
                 for (int r = 0; r < 6; r++) a[r] += b[r];
             }
-            const float yn_c = Y[o[ii]], dl_c = HAS_DL ? D[o[ii]] : 0.0f;
-            const float* cf = scoef + (ii * TILE_J + warp) * 4;
+            const float* cf = scoef + (ii * NCW + warp) * 4;
             const float df = K.inv_dr2 * a[1] + cf[0] * a[0] + cf[1] * a[3] + cf[2] * a[2] + cf[3] * a[5];
             const float tr = tu[ii] * a[0] + tv[ii] * a[2] + tw[ii] * a[4];
-            const int x = pidx[ii];
-            float S = w0 * P0[x];
-            if (n_src(q) == 2) S += w1 * P1[x];
-            const float kap = turb_field(q) ? kap0 + nuec[ii] * inv_sig : kap0 + nts[ii];
+            float S = F.w0 * P[0][ii * PP];
+            if (NSRC == 2) S = fmaf(F.w0, P[0][ii * PP], F.w1 * P[1][ii * PP]);
+            const float kap = TURB ? F.kap0 + nuec[ii] * F.inv_sig : F.kap0 + nts[ii];
             const float r = kap * df - tr + S;
-            const int cc = c[ii];
+            const int cc = c0 + ii * plane;
             if (MODE == MODE_STAGE) {
                 const float cr = sp.c_in_f * r;
                 float d = cr;
-                if (turb_field(q)) {
-                    const float accv = (n_src(q) == 2 ? P2 : P1)[x];
-                    io.acc_turb[q - ATSAT_F_TKE][cc] = (sp.stage == 0) ? sp.wgt_f * r : accv + sp.wgt_f * r;
+                if (TURB) {
+                    const float accv = P[NSRC][ii * PP];
+                    const float acc = (sp.stage == 0) ? sp.wgt_f * r : accv + sp.wgt_f * r;
+                    if (ii < nv) store(io.acc_turb[q - ATSAT_F_TKE] + cc, acc);
                     const float y = yn_c + cr;
                     const float yc = (q == ATSAT_F_TKE) ? sminf(smaxf(y, 0.0f), K.tke_max) : smaxf(y, K.dis_min);
                     d = yc - yn_c;
                 }
-                io.dl_out[q][cc] = d;
+                if (ii < nv) store(io.dl_out[q] + cc, d);
             } else {
+                // y_{n+1} = y_n + increment: the increment in FP32, the sum in FP64
                 float inc;
-                if (turb_field(q)) {
-                    inc = sp.sixth_dt_f * (P1[x] + r);
-                } else {
-                    const float dl1 = (n_src(q) == 2 ? P2 : P1)[x], dl2 = (n_src(q) == 2 ? P3 : P2)[x];
-                    inc = THIRD * (dl1 + 2.0f * dl2 + dl_c) + sp.sixth_dt_f * r;
+                if (TURB) inc = sp.sixth_dt_f * (P[1][ii * PP] + r);
+                else inc = THIRD * (P[NSRC][ii * PP] + 2.0f * P[NSRC + 1][ii * PP] + dl_c) + sp.sixth_dt_f * r;
+                double y = yn64[ii] + f2d(inc);
+                if (TURB) y = (q == ATSAT_F_TKE) ? smin(smax(y, 0.0), K.tke_max_d) : smax(y, K.dis_min_d);
+                if (ii < nv) {
+                    store(io.out64[q] + cc, y);
+                    if (io.out32[q]) store(io.out32[q] + cc, d2f(y));
+                    if (sp.write_all_rhs) store(io.rhs[q] + cc, f2d(r));
                 }
-                // the increment of y_{n+1}, in place of dl_1 (read above from this cell's point box);
-                // launch_final_combine adds it to y_n in FP64
-                io.dl1[q][cc] = inc;
-                if (sp.write_all_rhs) io.rhs[q][cc] = f2d(r);
             }
         }
-        release<NHS>(rh, hb, hb + (HAS_DL ? 2 : 1));
-        release<NPS>(rp, pb, pb + npq);
+        release(n);
+        return true;
+    };
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+#pragma unroll 1
+    for (int q = q0, n = NWIND; q < q_end; q++, n++) {
+        const bool ok = turb_field(q) ? field(One{}, std::true_type{}, q, n)
+                      : n_src(q) == 2 ? field(Two{}, std::false_type{}, q, n)
+                                      : field(One{}, std::false_type{}, q, n);
+        if (!ok) return;
     }
-    if (Q1 == NPROG && !K.turb && MODE == MODE_FINAL && sp.write_all_rhs) {
+    if (MODE == MODE_FINAL && q1 == NPROG && !K.turb && sp.write_all_rhs) {
 #pragma unroll
         for (int ii = 0; ii < TI; ii++)
-            if (valid[ii]) {
-                io.rhs[ATSAT_F_TKE][c[ii]] = 0.0;
-                io.rhs[ATSAT_F_DIS][c[ii]] = 0.0;
+            if (ii < nv) {
+                io.rhs[ATSAT_F_TKE][c0 + ii * plane] = 0.0;
+                io.rhs[ATSAT_F_DIS][c0 + ii * plane] = 0.0;
             }
     }
-}
-
-// field group g of NG of tile (bx, by, bz)
-template <int MODE, bool HAS_DL, int NG, int G = 0>
-__device__ __forceinline__ void group_block(const CUtensorMap& map_main, const CUtensorMap& map_seam,
-                                            const CUtensorMap& map_pt, const MixedConstF& K, const MixedIO& io,
-                                            const StageParams& sp, const TracerPlan& plan, float* smem, int bx, int by,
-                                            int bz, int g) {
-    if (NG == 1 || g == G)
-        block<MODE, HAS_DL, group_q0<NG>(G), group_q0<NG>(G + 1)>(map_main, map_seam, map_pt, K, io, sp, plan, smem, bx, by, bz);
-    else if constexpr (G + 1 < NG)
-        group_block<MODE, HAS_DL, NG, G + 1>(map_main, map_seam, map_pt, K, io, sp, plan, smem, bx, by, bz, g);
 }
 
 }  // namespace tracer
