@@ -81,11 +81,16 @@ FusedGrid fused_grid(int im, int jm, int km, int levels) {
 // 21x91x181 575 -> 549, 31x121x241 1063 -> 1018. Beyond, a lone run still gains (41x181x361 replayed 2408 -> 2351 us,
 // 61x271x541 7457 -> 7238), but handles that run concurrently fill those waves with each other's blocks already and
 // lose (three replaying in turn at 41x181x361 2193 -> 2203 us): the launches stay apart.
+// The final stage's momentum blocks need 109 KB (two blocks per SM), so there the line is two waves of those: two
+// iterations at 10x20x36 206 -> 188 us, 9x31x61 204 -> 188, 14x40x97 243 -> 238; at four waves 21x91x181 goes 548 -> 581.
 // Interleaving the momentum blocks with the tracer blocks, so that both kinds share an SM, is slower the finer it is
 // (with the unrolled tracer code, 2489 us apart: every 3rd block 2755, every 4th 2820).
 bool stage_fusable(const MixedConstF& kf, const MarchPlan& mp, int mode) {
-    if (mode != MODE_STAGE || !mp.compact || mp.n_pt > march::Shape<MODE_STAGE, true>::NPT || mp.levels < 1) return false;
+    if (mode == MODE_RHS || mp.levels < 1) return false;
     const FusedGrid G = fused_grid(kf.im, kf.jm, kf.km, mp.levels);
+    if (mode == MODE_FINAL)
+        return mp.p_dl >= 0 && mp.n_pt <= march::Shape<MODE_FINAL, false>::NPT && G.nm + G.nt * G.ng <= 2 * 2 * sm_count();
+    if (!mp.compact || mp.n_pt > march::Shape<MODE_STAGE, true>::NPT) return false;
     return G.nm + G.nt <= 4 * 3 * sm_count();
 }
 
@@ -97,6 +102,8 @@ cudaError_t launch_rk_stage_fused(const TileMaps& maps, const MixedConstF& kf, c
         return cudaErrorInvalidValue;
     const FusedGrid G = fused_grid(kf.im, kf.jm, kf.km, mp.levels);
     if (G.nm + G.nt == 0) return cudaSuccess;
+    if (mode == MODE_FINAL)
+        return has_dl ? launch_one<MODE_FINAL, true>(maps, kf, io, sp, mp, tp, G, s) : cudaErrorInvalidValue;
     return has_dl ? launch_one<MODE_STAGE, true>(maps, kf, io, sp, mp, tp, G, s)
                   : launch_one<MODE_STAGE, false>(maps, kf, io, sp, mp, tp, G, s);
 }
