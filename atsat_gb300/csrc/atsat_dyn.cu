@@ -64,6 +64,7 @@ struct atsat_dyn {
     BaroTables baro{};
     double* p_baro = nullptr;            // null unless set
     double* partial = nullptr;
+    unsigned int* lm_done = nullptr;     // the level mean's finished blocks per level
     double* buoy = nullptr;
     double* sin_j = nullptr;
     double* rm_tab = nullptr;            // 1 / rm(i)
@@ -88,9 +89,6 @@ struct atsat_dyn {
     // stream, and per buffer an event for "copy landed / re-pitched out" and one for "free again"
     double* dstage[2] = {};
     cudaStream_t cstream = nullptr;
-    // the second stream of the step's start (the metric scan beside the level mean) and its fork / join
-    cudaStream_t astream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_ajoin = nullptr;
     cudaEvent_t ev_ready[2] = {}, ev_free[2] = {}, ev_join = nullptr;
     int stage_next = 0;
     // bindings the SMs move in place (host_xfer.cu): host_ok when the device addresses host memory
@@ -861,41 +859,39 @@ StageIO<double> make_io(atsat_dyn* h, double* const* in, double* const* out) {
     return io;
 }
 
+LevelMean level_mean_args(const atsat_dyn* h) {
+    return {h->f[ATSAT_F_T], h->f[ATSAT_F_P_STAT], h->sin_j, h->partial, h->lm_done, h->buoy};
+}
+
+MetricScan metric_scan_args(const atsat_dyn* h) {
+    return {h->f[ATSAT_F_V], h->f[ATSAT_F_W], h->rm_tab, h->cor_j, h->has_pbaro ? h->p_baro : nullptr,
+            h->f[ATSAT_F_P_METRIC]};
+}
+
 int do_level_mean(atsat_dyn* h) {
     Timed t(h, ATSAT_K_LEVEL_MEAN);
-    CK(h, launch_level_mean(h->kc, h->f[ATSAT_F_T], h->f[ATSAT_F_P_STAT], h->sin_j, h->partial, h->buoy, h->stream));
-    h->launches += 2;
+    const LevelMean m = level_mean_args(h);
+    CK(h, launch_level_metric(h->kc, &m, nullptr, h->stream));
+    h->launches += 1;
     return ATSAT_DYN_OK;
 }
 
 int do_metric(atsat_dyn* h) {
     Timed t(h, ATSAT_K_METRIC_SCAN);
-    CK(h, launch_metric_scan(h->kc, h->f[ATSAT_F_V], h->f[ATSAT_F_W], h->rm_tab, h->cor_j,
-                             h->has_pbaro ? h->p_baro : nullptr, h->f[ATSAT_F_P_METRIC], h->stream));
+    const MetricScan c = metric_scan_args(h);
+    CK(h, launch_level_metric(h->kc, nullptr, &c, h->stream));
     h->launches += 1;
     return ATSAT_DYN_OK;
 }
 
-// the start of a step: the buoyancy level mean and, where metric_split is on, the metric pressure. Both
-// read y_n only and are latency-bound scans (GB300's FP64 pipe sets their pace, not HBM), so the metric scan
-// runs on a second stream beside the level mean, forked from and joined back into the handle's stream by
-// events (CUDA-graph capture records the fork and the join).
+// the start of a step: the buoyancy level mean and, where metric_split is on, the metric pressure
 int do_level_metric(atsat_dyn* h) {
     if (!h->p.metric_split) return do_level_mean(h);
-    if (!h->astream) {
-        CK(h, cudaStreamCreateWithFlags(&h->astream, cudaStreamNonBlocking));
-        CK(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-        CK(h, cudaEventCreateWithFlags(&h->ev_ajoin, cudaEventDisableTiming));
-    }
     Timed t(h, ATSAT_K_LEVEL_MEAN);
-    CK(h, cudaEventRecord(h->ev_fork, h->stream));
-    CK(h, cudaStreamWaitEvent(h->astream, h->ev_fork, 0));
-    CK(h, launch_metric_scan(h->kc, h->f[ATSAT_F_V], h->f[ATSAT_F_W], h->rm_tab, h->cor_j,
-                             h->has_pbaro ? h->p_baro : nullptr, h->f[ATSAT_F_P_METRIC], h->astream));
-    CK(h, launch_level_mean(h->kc, h->f[ATSAT_F_T], h->f[ATSAT_F_P_STAT], h->sin_j, h->partial, h->buoy, h->stream));
-    CK(h, cudaEventRecord(h->ev_ajoin, h->astream));
-    CK(h, cudaStreamWaitEvent(h->stream, h->ev_ajoin, 0));
-    h->launches += 3;
+    const LevelMean m = level_mean_args(h);
+    const MetricScan c = metric_scan_args(h);
+    CK(h, launch_level_metric(h->kc, &m, &c, h->stream));
+    h->launches += 1;
     return ATSAT_DYN_OK;
 }
 
@@ -1948,7 +1944,7 @@ int atsat_dyn_create(const atsat_dyn_grid* g, const atsat_dyn_params* p, atsat_d
     // fields, FP64 stage buffers and accumulators (FP64 path only), source; then the small tables
     const bool fp64_stage = p->precision != ATSAT_DYN_MIXED;
     const int64_t nbig = ATSAT_NFIELDS + (fp64_stage ? 2 * NPROG : 0) + 2;
-    const int64_t nsmall = 2LL * K.im * 16 + K.im + K.jm + K.im + K.jm + 64;
+    const int64_t nsmall = 2LL * K.im * LEVEL_MEAN_CHUNKS + K.im + K.im + K.jm + K.im + K.jm + 64;
     const size_t bytes = (size_t)(nbig * K.fsz + nsmall) * 8 + (sizeof(ColGeo) + (fp64_stage ? sizeof(StageGeo) : 0)) * (size_t)K.im * K.jm + 4096;
     if ((e = cudaMalloc(&h->slab, bytes)) != cudaSuccess) return cuda_fail(e, "cudaMalloc");
     if ((e = cudaMemsetAsync(h->slab, 0, bytes, h->stream)) != cudaSuccess) return cuda_fail(e, "cudaMemset");
@@ -1960,7 +1956,8 @@ int atsat_dyn_create(const atsat_dyn_grid* g, const atsat_dyn_params* p, atsat_d
     }
     h->src = q; q += K.fsz;
     h->p_baro = q; q += K.fsz;
-    h->partial = q; q += 2LL * K.im * 16;
+    h->partial = q; q += 2LL * K.im * LEVEL_MEAN_CHUNKS;
+    h->lm_done = reinterpret_cast<unsigned int*>(q); q += K.im;
     h->buoy = q; q += K.im;
     h->sin_j = q; q += K.jm;
     h->rm_tab = q; q += K.im;
@@ -2068,12 +2065,6 @@ void atsat_dyn_destroy(atsat_dyn_t h) {
     stage_pipe_free(h);
     for (int f = 0; f < ATSAT_NFIELDS; f++)
         if (h->dev_rows[f]) cudaFree(h->dev_rows[f]);
-    if (h->astream) {
-        cudaStreamSynchronize(h->astream);
-        cudaStreamDestroy(h->astream);
-    }
-    if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-    if (h->ev_ajoin) cudaEventDestroy(h->ev_ajoin);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }

@@ -416,10 +416,19 @@ const std::vector<double>& poisson_null_vector(PoissonSolver* P);   // [(j-1) * 
 void poisson_sweep_stats(PoissonSolver* P, int* sweeps_per_pass, double* sweep_ms);
 cudaError_t poisson_run(PoissonSolver* P, int method, double tol, int max_iter, int inner, double omega,
                         int* iters, int* inner_total, double* rel);
-cudaError_t launch_level_mean(const KConst& kc, const double* t, const double* p_stat,
-                              const double* sin_j, double* partial, double* buoy, cudaStream_t s);
-cudaError_t launch_metric_scan(const KConst& kc, const double* v, const double* w, const double* inv_rm,
-                               const double* cor_j, const double* p_baro, double* p_metric, cudaStream_t s);
+constexpr int LEVEL_MEAN_CHUNKS = 16;
+struct LevelMean {
+    const double *t, *p_stat, *sin_j;
+    double* partial;               // [im][LEVEL_MEAN_CHUNKS][2]
+    unsigned int* done;            // [im], zero between launches
+    double* buoy;
+};
+struct MetricScan {
+    const double *v, *w, *inv_rm, *cor_j, *p_baro;   // p_baro: null where off
+    double* p_metric;
+};
+// the buoyancy level mean and the metric pressure scan, either null
+cudaError_t launch_level_metric(const KConst& kc, const LevelMean* m, const MetricScan* c, cudaStream_t s);
 cudaError_t launch_density(const KConst& kc, const double* t, const double* p_stat, double R_mix,
                            double* rho, cudaStream_t s);
 cudaError_t launch_projection_prep(const KConst& kc, double* const six[6], cudaStream_t s);

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
 // ---- computeBuoyancyRefLevel (RungeKutta_Sat_Turb.cpp:31-50): two-level deterministic reduction ----
 // One block per (level, chunk of rows); a warp takes whole rows, its lanes the meridians, four at a time
 // so that eight loads are in flight per lane.
-constexpr int LM_CHUNKS = 16;
+constexpr int LM_CHUNKS = LEVEL_MEAN_CHUNKS;
 constexpr int LM_THREADS = 128;
 
 // the buoyancy g p / (r_mix R_mix T t_ref) = bc p / t of one cell (bc formed on the host); false where
@@ -326,11 +326,12 @@ __device__ __forceinline__ bool below_pow2(double x, uint32_t e) {
 // |bc| < 2^256 every fast-path term and sum is finite, as the reference's isfinite test needs.
 // Measured at 41x181x361: 33.8 -> 28 us with the rare path called (5.1 -> 3.9 FP64 slots a cell); two or three warps
 // of a block sharing a running sum's rows changed nothing (28, 27 us), four filled two waves (42 us).
-__global__ void __launch_bounds__(LM_THREADS) level_mean_partial_kernel(const KConst K, const double* __restrict__ t,
-                                                                         const double* __restrict__ ps,
-                                                                         const double* __restrict__ sin_j,
-                                                                         double* __restrict__ partial) {
-    const int i = blockIdx.x, chunk = blockIdx.y;
+//
+// The last of a level's blocks to finish adds the chunks' sums in order (`done` counts the level's finished blocks
+// and is zero again afterwards).
+__device__ __forceinline__ void level_mean_block(const KConst& K, const double* __restrict__ t,
+                                                 const double* __restrict__ ps, const double* __restrict__ sin_j,
+                                                 double* partial, unsigned int* done, double* buoy, int i, int chunk) {
     const int j0 = (int)((int64_t)K.jm * chunk / LM_CHUNKS), j1 = (int)((int64_t)K.jm * (chunk + 1) / LM_CHUNKS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool bc_ok = below_pow2(K.buoy_c, 256);
@@ -374,41 +375,38 @@ __global__ void __launch_bounds__(LM_THREADS) level_mean_partial_kernel(const KC
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
         for (int q = 0; q < LM_THREADS / 32; q++) { a += s_sum[q]; b += s_w[q]; }
-        partial[((int64_t)i * LM_CHUNKS + chunk) * 2 + 0] = a;
-        partial[((int64_t)i * LM_CHUNKS + chunk) * 2 + 1] = b;
+        double* part = partial + (int64_t)i * LM_CHUNKS * 2;
+        __stcg(part + chunk * 2 + 0, a);
+        __stcg(part + chunk * 2 + 1, b);
+        __threadfence();
+        if (atomicAdd(done + i, 1u) == LM_CHUNKS - 1) {
+            __threadfence();
+            double s = 0.0, w = 0.0;
+            for (int q = 0; q < LM_CHUNKS; q++) {
+                s += __ldcg(part + q * 2 + 0);
+                w += __ldcg(part + q * 2 + 1);
+            }
+            buoy[i] = (w > 0.0) ? s / w : 0.0;
+            done[i] = 0u;
+        }
     }
-}
-
-__global__ void level_mean_final_kernel(const KConst K, const double* __restrict__ partial, double* __restrict__ buoy) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K.im) return;
-    double s = 0.0, w = 0.0;
-    for (int q = 0; q < LM_CHUNKS; q++) {
-        s += partial[((int64_t)i * LM_CHUNKS + q) * 2 + 0];
-        w += partial[((int64_t)i * LM_CHUNKS + q) * 2 + 1];
-    }
-    buoy[i] = (w > 0.0) ? s / w : 0.0;
 }
 
 // ---- computeMetricPressure (RungeKutta_Sat_Turb.cpp:60-108): one radial trapezoid scan per column ----
-// The scan is serial in i; the loads of eight levels are issued ahead of the dependent sums. inv_rm holds
+// The scan is serial in i. inv_rm holds
 // 1 / rm(i) (a product instead of the reference's quotient: at most one rounding apart). Six FP64 operations
 // per cell (seven with p_baro): f = (v^2 + w^2) / rm + cor w as two products and two fmas, and the
 // trapezoid acc += dr/2 (f_{i-1} + f_i) as one add and one fma.
-// The next eight levels' loads are in flight while these are summed, and p_baro is a switch of the code: 45.5 -> 39.7 us
-// at 41x181x361 (26 us of FP64 issue).
-constexpr int MS_BATCH = 8;
+// The next four levels' loads are in flight while these are summed (two, four or eight alike), and p_baro is a switch
+// of the code: 45.5 -> 39.7 us by itself at 41x181x361 (26 us of FP64 issue).
+constexpr int MS_BATCH = 4;
 
 template <bool BARO>
-__global__ void __launch_bounds__(128) metric_scan_kernel(const KConst K, const double* __restrict__ v,
-                                                          const double* __restrict__ w,
-                                                          const double* __restrict__ inv_rm,
-                                                          const double* __restrict__ cor_j,
-                                                          const double* __restrict__ p_baro,
-                                                          double* __restrict__ pm, double half_dr) {
-    const int k = blockIdx.x * 32 + threadIdx.x;
-    const int j = blockIdx.y * 4 + threadIdx.y;
-    if (k >= K.km || j >= K.jm) return;
+__device__ __forceinline__ void metric_scan_column(const KConst& K, const double* __restrict__ v,
+                                                   const double* __restrict__ w, const double* __restrict__ inv_rm,
+                                                   const double* __restrict__ cor_j,
+                                                   const double* __restrict__ p_baro, double* __restrict__ pm,
+                                                   double half_dr, int j, int k) {
     const double cor = __ldg(cor_j + j);
     const int64_t c0 = (int64_t)j * K.kp + k;
     double vv[MS_BATCH], ww[MS_BATCH], pb[MS_BATCH];
@@ -445,6 +443,32 @@ __global__ void __launch_bounds__(128) metric_scan_kernel(const KConst K, const 
             pm[c0 + (int64_t)i * K.plane] = BARO ? acc + cb[q] : acc;
         }
     }
+}
+
+// The step's two FP64-bound scans in one launch: the level mean's blocks (one per level and chunk), then the metric
+// scan's (32 x 4 columns; the other order is 0.6 % of a step slower). They read different fields of y_n and fill each other's thin waves: 66 us at 41x181x361
+// (44 us of FP64 issue). Apart, on two streams forked and joined by events, with the level mean's last sum a launch of
+// its own, they took three launches: two iterations at 10x20x36 214 -> 206 us, 41x181x361 replayed 2408 -> 2385.
+struct LevelMetricArgs {
+    const double *t, *ps, *sin_j;                  // level mean
+    double *partial, *buoy;
+    unsigned int* done;
+    const double *v, *w, *inv_rm, *cor_j, *p_baro; // metric scan
+    double* pm;
+    double half_dr;
+    int mean_blocks, bk;                           // level mean blocks; metric scan blocks along k
+};
+
+template <bool BARO>
+__global__ void __launch_bounds__(LM_THREADS) level_metric_kernel(const KConst K, const LevelMetricArgs A) {
+    if ((int)blockIdx.x < A.mean_blocks) {
+        level_mean_block(K, A.t, A.ps, A.sin_j, A.partial, A.done, A.buoy, blockIdx.x / LM_CHUNKS, blockIdx.x % LM_CHUNKS);
+        return;
+    }
+    const int b = blockIdx.x - A.mean_blocks;
+    const int k = b % A.bk * 32 + (threadIdx.x & 31), j = b / A.bk * 4 + (threadIdx.x >> 5);
+    if (k < K.km && j < K.jm)
+        metric_scan_column<BARO>(K, A.v, A.w, A.inv_rm, A.cor_j, A.p_baro, A.pm, A.half_dr, j, k);
 }
 
 // ---- computeMixtureDensity (Pressure_Sat.cpp:49-62) ----
@@ -493,18 +517,21 @@ cudaError_t launch_rk_stage_fp64(const KConst& kc, const StageIO<double>& io, co
     return cudaGetLastError();
 }
 
-cudaError_t launch_level_mean(const KConst& kc, const double* t, const double* p_stat, const double* sin_j,
-                              double* partial, double* buoy, cudaStream_t s) {
-    level_mean_partial_kernel<<<dim3(kc.im, LM_CHUNKS), LM_THREADS, 0, s>>>(kc, t, p_stat, sin_j, partial);
-    level_mean_final_kernel<<<(kc.im + 63) / 64, 64, 0, s>>>(kc, partial, buoy);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_metric_scan(const KConst& kc, const double* v, const double* w, const double* inv_rm,
-                               const double* cor_j, const double* p_baro, double* p_metric, cudaStream_t s) {
-    dim3 block(32, 4), grid((kc.km + 31) / 32, (kc.jm + 3) / 4);
-    auto kernel = p_baro ? metric_scan_kernel<true> : metric_scan_kernel<false>;
-    kernel<<<grid, block, 0, s>>>(kc, v, w, inv_rm, cor_j, p_baro, p_metric, 0.5 * kc.dr);
+cudaError_t launch_level_metric(const KConst& kc, const LevelMean* m, const MetricScan* c, cudaStream_t s) {
+    LevelMetricArgs A{};
+    if (m) {
+        A.t = m->t; A.ps = m->p_stat; A.sin_j = m->sin_j;
+        A.partial = m->partial; A.done = m->done; A.buoy = m->buoy;
+    }
+    if (c) {
+        A.v = c->v; A.w = c->w; A.inv_rm = c->inv_rm; A.cor_j = c->cor_j; A.p_baro = c->p_baro; A.pm = c->p_metric;
+        A.half_dr = 0.5 * kc.dr;
+        A.bk = (kc.km + 31) / 32;
+    }
+    A.mean_blocks = m ? kc.im * LM_CHUNKS : 0;
+    const int blocks = A.mean_blocks + A.bk * ((kc.jm + 3) / 4);
+    auto kernel = A.p_baro ? level_metric_kernel<true> : level_metric_kernel<false>;
+    kernel<<<blocks, LM_THREADS, 0, s>>>(kc, A);
     return cudaGetLastError();
 }
 
