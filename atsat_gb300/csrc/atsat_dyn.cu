@@ -537,18 +537,18 @@ bool make_tile_maps(atsat_dyn* h) {
     const CUresult r2 = enc(reinterpret_cast<CUtensorMap*>(h->maps.seam), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
                             dims, strides, box_seam, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const cuuint32_t box_main4[4] = {TTILE_BX, TTILE_BY, TTILE_BZ, 1};
-    const cuuint32_t box_seam4[4] = {TILE_SEAM_X, TTILE_J, TTILE_I, 1};
-    const CUresult r3 = enc(reinterpret_cast<CUtensorMap*>(h->maps.main4), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
-                            dims, strides, box_main4, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const CUresult r4 = enc(reinterpret_cast<CUtensorMap*>(h->maps.seam4), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
-                            dims, strides, box_seam4, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    const cuuint32_t box_pt4[4] = {TTILE_K, TTILE_J, TTILE_I, 1};
-    const CUresult r5 = enc(reinterpret_cast<CUtensorMap*>(h->maps.pt4), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
-                            dims, strides, box_pt4, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    // the tracer kernel's tiles, 64 and 32 cells wide
+    bool tracer_ok = true;
+    for (int m = 0; m < 2; m++) {
+        const cuuint32_t tk = m == 0 ? 64 : 32, tj = 256 / tk;
+        const cuuint32_t box[3][4] = {{tk + 8, tj + 2, TTILE_BZ, 1}, {TILE_SEAM_X, tj, TTILE_I, 1}, {tk, tj, TTILE_I, 1}};
+        unsigned char* const out[3] = {h->maps.main4[m], h->maps.seam4[m], h->maps.pt4[m]};
+        for (int b = 0; b < 3; b++)
+            tracer_ok = tracer_ok &&
+                        enc(reinterpret_cast<CUtensorMap*>(out[b]), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32, dims,
+                            strides, box[b], estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
     const cuuint32_t box_pt2[4] = {TILE_K, TILE_J, TILE_I, 1};
     const CUresult r6 = enc(reinterpret_cast<CUtensorMap*>(h->maps.pt2), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->slab32,
                             dims, strides, box_pt2, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -566,7 +566,7 @@ bool make_tile_maps(atsat_dyn* h) {
     const CUresult r9 = enc(reinterpret_cast<CUtensorMap*>(h->maps.pt1), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                             h->slab32, dims, strides, box_pt1, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r1 == CUDA_SUCCESS && r2 == CUDA_SUCCESS && r3 == CUDA_SUCCESS && r4 == CUDA_SUCCESS && r5 == CUDA_SUCCESS &&
+    return r1 == CUDA_SUCCESS && r2 == CUDA_SUCCESS && tracer_ok &&
            r6 == CUDA_SUCCESS && r7 == CUDA_SUCCESS && r8 == CUDA_SUCCESS && r9 == CUDA_SUCCESS;
 }
 

@@ -296,9 +296,8 @@ constexpr long long TILE_WAIT_LIMIT = 1LL << 31;   // SM clocks (about a second)
 constexpr int TILE_BX = TILE_K + 8, TILE_BY = TILE_J + 2, TILE_BZ = TILE_I + 2;
 constexpr int TILE_SEAM_X = 4;
 constexpr int TILE_MAX_ITEMS = 2 * NPROG + 1;
-// the tracer kernel's tile: 256 columns, four radial levels per thread
-constexpr int TTILE_K = 64, TTILE_J = 4, TTILE_I = 4;
-constexpr int TTILE_BX = TTILE_K + 8, TTILE_BY = TTILE_J + 2, TTILE_BZ = TTILE_I + 2;
+// the tracer kernel's tile: 64 x 4 or 32 x 8 columns, four radial levels per thread
+constexpr int TTILE_I = 4, TTILE_BZ = TTILE_I + 2;
 struct TilePlan {
     int n_items;
     int item[TILE_MAX_ITEMS];
@@ -335,9 +334,10 @@ cudaError_t launch_rk_split(const MixedConstF& kf, const MixedIO& io, const Stag
 struct TileMaps {
     alignas(64) unsigned char main[128];    // box TILE_BX x TILE_BY x TILE_BZ
     alignas(64) unsigned char seam[128];    // box TILE_SEAM_X x TILE_J x TILE_I
-    alignas(64) unsigned char main4[128];   // box TTILE_BX x TTILE_BY x TTILE_BZ
-    alignas(64) unsigned char seam4[128];   // box TILE_SEAM_X x TTILE_J x TTILE_I
-    alignas(64) unsigned char pt4[128];     // box TTILE_K x TTILE_J x TTILE_I (point values, no halo)
+    // the tracer kernel's boxes: tiles 64 cells wide [0] and 32 [1]
+    alignas(64) unsigned char main4[2][128];   // halo box, TTILE_BZ planes
+    alignas(64) unsigned char seam4[2][128];   // TILE_SEAM_X columns
+    alignas(64) unsigned char pt4[2][128];     // point values, no halo
     alignas(64) unsigned char pt2[128];     // box TILE_K x TILE_J x TILE_I (point values, no halo)
     alignas(64) unsigned char plane1[128];  // box TILE_BX x TILE_BY x 1: one radial plane with its halo
     alignas(64) unsigned char seam1[128];   // box TILE_SEAM_X x TILE_J x 1
@@ -370,6 +370,7 @@ cudaError_t launch_rk_tracer_tile(const TileMaps& maps, const MixedConstF& kf, c
                                   const StageParams& sp, const TracerPlan& plan, int mode, cudaStream_t s);
 cudaError_t launch_rk_mom(const MixedConstF& kf, const MixedIO& io, const StageParams& sp, int mode, cudaStream_t s);
 int tracer_plan_items(int mode, bool has_dl, bool turb);
+int tracer_tile_k(int jm, int km);  // the tracer kernel's tile width for this grid
 int tracer_groups(int64_t tiles);   // field groups (blocks per tile) of the tracer kernel for this many tiles
 int sm_count();                     // SMs of the current device
 // the momentum / temperature equations alone, TMA-tiled (species_divu off)

@@ -16,15 +16,15 @@ struct FusedGrid {
     int ng;                        // field groups per tracer tile
 };
 
-template <int MODE>
+template <int MODE, int TK>
 struct Fused {
     static constexpr bool CMP = MODE == MODE_STAGE;
-    static constexpr size_t SMEM = march::Shape<MODE, CMP>::SMEM > tracer::SMEM_BYTES ? march::Shape<MODE, CMP>::SMEM
-                                                                                      : tracer::SMEM_BYTES;
+    static constexpr size_t SMEM = march::Shape<MODE, CMP>::SMEM > tracer::Tile<TK>::SMEM ? march::Shape<MODE, CMP>::SMEM
+                                                                                          : tracer::Tile<TK>::SMEM;
 };
 
-template <int MODE, bool HAS_DL>
-__global__ void __launch_bounds__(march::THREADS, Fused<MODE>::CMP ? 3 : 2)
+template <int MODE, bool HAS_DL, int TK>
+__global__ void __launch_bounds__(march::THREADS, Fused<MODE, TK>::CMP ? 3 : 2)
 rk_stage_fused_kernel(const __grid_constant__ CUtensorMap plane, const __grid_constant__ CUtensorMap plane_seam,
                       const __grid_constant__ CUtensorMap plane_pt, const __grid_constant__ CUtensorMap box,
                       const __grid_constant__ CUtensorMap box_seam, const __grid_constant__ CUtensorMap box_pt,
@@ -37,27 +37,35 @@ rk_stage_fused_kernel(const __grid_constant__ CUtensorMap plane, const __grid_co
     const int nk = mom ? G.nk : G.tk, nj = mom ? G.nj : G.tj;
     const int bx = n % nk, r = n / nk, by = r % nj, bz = r / nj;
     if (mom)
-        march::block<MODE, HAS_DL, Fused<MODE>::CMP>(plane, plane_seam, plane_pt, K, io, sp, mp, smem, bx, by, bz);
+        march::block<MODE, HAS_DL, Fused<MODE, TK>::CMP>(plane, plane_seam, plane_pt, K, io, sp, mp, smem, bx, by, bz);
     else
-        tracer::block<MODE, HAS_DL>(box, box_seam, box_pt, K, io, sp, tp, smem, bx, by, bz, tracer::group_q0(G.ng, g),
+        tracer::block<MODE, HAS_DL, TK>(box, box_seam, box_pt, K, io, sp, tp, smem, bx, by, bz, tracer::group_q0(G.ng, g),
                                     tracer::group_q0(G.ng, g + 1));
+}
+
+template <int MODE, bool HAS_DL, int TK>
+cudaError_t launch_tile(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
+                       const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
+    static bool attr = false;
+    constexpr size_t smem = Fused<MODE, TK>::SMEM;
+    if (!attr) {
+        const cudaError_t e = cudaFuncSetAttribute(rk_stage_fused_kernel<MODE, HAS_DL, TK>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
+    constexpr int t = TK == 64 ? 0 : 1;
+    auto map = [](const unsigned char* p) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(p); };
+    rk_stage_fused_kernel<MODE, HAS_DL, TK><<<G.nm + G.nt * G.ng, march::THREADS, smem, s>>>(
+        map(m.plane1), map(m.seam1), map(m.pt1), map(m.main4[t]), map(m.seam4[t]), map(m.pt4[t]), kf, io, sp, mp, tp, G);
+    return cudaGetLastError();
 }
 
 template <int MODE, bool HAS_DL>
 cudaError_t launch_one(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
-    static bool attr = false;
-    constexpr size_t smem = Fused<MODE>::SMEM;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_stage_fused_kernel<MODE, HAS_DL>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
-    auto map = [](const unsigned char* p) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(p); };
-    rk_stage_fused_kernel<MODE, HAS_DL><<<G.nm + G.nt * G.ng, march::THREADS, smem, s>>>(
-        map(m.plane1), map(m.seam1), map(m.pt1), map(m.main4), map(m.seam4), map(m.pt4), kf, io, sp, mp, tp, G);
-    return cudaGetLastError();
+    return tracer_tile_k(kf.jm, kf.km) == 64 ? launch_tile<MODE, HAS_DL, 64>(m, kf, io, sp, mp, tp, G, s)
+                                             : launch_tile<MODE, HAS_DL, 32>(m, kf, io, sp, mp, tp, G, s);
 }
 
 // blocks of the momentum kernel and tiles of the tracer kernel
@@ -66,8 +74,9 @@ FusedGrid fused_grid(int im, int jm, int km, int levels) {
     G.nk = (km - 1 + TILE_K - 1) / TILE_K;
     G.nj = (jm - 4 + TILE_J - 1) / TILE_J;
     if (G.nk <= 0 || G.nj <= 0 || im < 3) return G;
-    G.tk = (km - 1 + TTILE_K - 1) / TTILE_K;
-    G.tj = (jm - 4 + TTILE_J - 1) / TTILE_J;
+    const int tk = tracer_tile_k(jm, km), tj = 256 / tk;
+    G.tk = (km - 1 + tk - 1) / tk;
+    G.tj = (jm - 4 + tj - 1) / tj;
     G.nm = G.nk * G.nj * ((im - 2 + levels - 1) / levels);
     G.nt = G.tk * G.tj * ((im - 2 + TTILE_I - 1) / TTILE_I);
     G.ng = tracer_groups(G.nt);

@@ -2,18 +2,18 @@
 // stage handling of RungeKutta_Sat_Turb.cpp:250-375), run after the momentum / temperature kernel of the
 // split variant (rk_mixed.cu) when species_divu is off.
 //
-// A block owns 64 x 4 x 4 cells (k, j, i). A producer warp streams every array the tracers read with tensor
-// copies, in groups: the advecting winds and the eddy viscosity (three groups of point boxes, 64 x 4 x 4 floats,
-// no halo), then one group per field: the halo boxes (72 x 6 x 6 floats) of its y_n copy and stage increment and
+// A block owns TK x 256 / TK x 4 cells (k, j, i), TK 64 or 32 (tracer_tile_k). A producer warp streams every array the tracers read with tensor
+// copies, in groups: the advecting winds and the eddy viscosity (three groups of point boxes, without a
+// halo), then one group per field: the halo boxes (72 x 6 x 6 or 40 x 10 x 6 floats) of its y_n copy and stage increment and
 // the point boxes of its sources, the tke/dis running sum and, at the final stage, dl_1 and dl_2. A group has one
 // "full" barrier for all of its copies and one "empty" barrier; with increments two groups are in flight, without
-// four. Eight consumer warps (half a row j, lane k, four radial levels per lane) read the boxes from shared memory;
+// four. Eight consumer warps (32 columns of a row j, lane k, four radial levels per lane) read the boxes from shared memory;
 // at the final stage each lane loads its y_n (FP64) before it waits for the field's boxes and forms y_{n+1} there.
 // A block needs 73 KB of shared memory and 72 registers a thread: three blocks fit on an SM.
 //
 // What bounds it: memory (HBM at 88-93 % of a plain copy's rate at 41x181x361) and, close behind, issue (60 %).
 // Launches at 41x181x361, before -> now: intermediate with increments 144 -> 134 us, final stage with its FP64 half
-// 184 + 118 -> 258 us. 32 x 8 cells per tile read a halo a fifth larger per cell (2221 us a step pair against 2193).
+// 184 + 118 -> 258 us.
 // Prefetching the next groups into L2 did not help (2209-2240).
 //
 // The fields run through three copies of the code (one source, two sources, tke / dis) in a loop that is not
@@ -45,22 +45,27 @@ using namespace mixed;
 using namespace tma;
 
 constexpr int TI = TTILE_I;                               // 4 radial levels per thread
-constexpr int PL = TTILE_BX * TTILE_BY;                   // floats per plane of a halo box
-constexpr int BOX_F = PL * TTILE_BZ;
-constexpr int SEAM_F = TILE_SEAM_X * TTILE_J * TI;
-constexpr int HSLOT_F = (BOX_F + SEAM_F + 31) / 32 * 32;
-constexpr int PSLOT_F = TTILE_K * TTILE_J * TI;           // 1024 floats = 4096 bytes
-constexpr uint32_t BOX_BYTES = BOX_F * 4, SEAM_BYTES = SEAM_F * 4, PT_BYTES = PSLOT_F * 4;
 constexpr int NHS = 4, NPS = 7;                           // halo and point slots
-constexpr int WPR = TTILE_K / 32;                         // warps per row
-constexpr int NCW = WPR * TTILE_J;
+constexpr int NCW = 8;                                    // consumer warps
 constexpr int THREADS = (NCW + 1) * 32;
 constexpr int GEO_F = TI * NCW * 16;                      // ColGeoF of each warp's four columns
 constexpr int COEF_F = TI * NCW * 4;                      // their four diffusion factors
-constexpr size_t SMEM_BYTES = (size_t)NHS * HSLOT_F * 4 + (size_t)NPS * PSLOT_F * 4 + (size_t)(GEO_F + COEF_F) * 4
-                            + 2 * NHS * 8;
 
-static_assert((HSLOT_F * 4) % 128 == 0 && (PSLOT_F * 4) % 128 == 0 && (BOX_F * 4) % 128 == 0, "slot alignment");
+// a tile TK cells wide (k), 256 / TK rows, TI levels
+template <int TK>
+struct Tile {
+    static constexpr int TJ = 256 / TK, BX = TK + 8, BY = TJ + 2;
+    static constexpr int PL = BX * BY;                    // floats per plane of a halo box
+    static constexpr int BOX_F = PL * TTILE_BZ, SEAM_F = TILE_SEAM_X * TJ * TI;
+    static constexpr int HSLOT_F = (BOX_F + SEAM_F + 31) / 32 * 32;
+    static constexpr int PP = TK * TJ, PSLOT_F = PP * TI; // floats per plane of a point box, per box
+    static constexpr uint32_t BOX_BYTES = BOX_F * 4, SEAM_BYTES = SEAM_F * 4, PT_BYTES = PSLOT_F * 4;
+    static constexpr int WPR = TK / 32;                   // warps per row
+    static constexpr size_t SMEM = (size_t)NHS * HSLOT_F * 4 + (size_t)NPS * PSLOT_F * 4 + (size_t)(GEO_F + COEF_F) * 4
+                                 + 2 * NHS * 8;
+    static_assert((HSLOT_F * 4) % 128 == 0 && (PSLOT_F * 4) % 128 == 0 && (BOX_F * 4) % 128 == 0, "slot alignment");
+    static_assert(WPR * TJ == NCW && 3 * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
+};
 
 // ---- the stream layout (the host builds the same, make_plan_tracer) ----
 constexpr int NTRACER = NPROG - ATSAT_F_H2O;
@@ -99,7 +104,9 @@ static_assert(slots_fit(MODE_STAGE, false, 1) && slots_fit(MODE_STAGE, false, 4)
 
 // One array's stencil of a lane's column of TI cells: the centre values at i-1 and i stay in registers from cell to
 // cell, so a cell costs five shared loads instead of seven.
+template <int TK>
 struct Column {
+    static constexpr int PL = Tile<TK>::PL, BX = Tile<TK>::BX;
     float rn, x;                   // the values at i-1 and i
 
     __device__ __forceinline__ void start(const float* s, int o) {
@@ -109,7 +116,7 @@ struct Column {
     // the raw differences of cell i; returns its centre value and moves on to i+1
     __device__ __forceinline__ float d7(const float* s, int o, int ow, int oe, float* e) {
         const float rp = s[o + PL];
-        const float tp = s[o + TTILE_BX], tn = s[o - TTILE_BX];
+        const float tp = s[o + BX], tn = s[o - BX];
         const float pe = s[oe], pw = s[ow];
         const float c = x;
         e[0] = rp - rn;
@@ -135,12 +142,14 @@ __device__ __forceinline__ void store(double* p, double x) {
 }
 
 // the tracers [q0, q1) of tile (bx, by, bz): the winds' groups, then those fields' groups of the plan
-template <int MODE, bool HAS_DL>
+template <int MODE, bool HAS_DL, int TK>
 __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtensorMap& map_seam, const CUtensorMap& map_pt,
                                       const MixedConstF& K, const MixedIO& io, const StageParams& sp,
                                       const TracerPlan& plan, float* smem, int bx, int by, int bz, int q0, int q1) {
     static_assert(MODE == MODE_STAGE || (MODE == MODE_FINAL && HAS_DL), "stages of the stream layout");
     constexpr int NH = HAS_DL ? 2 : 1, AHEAD = groups_ahead(HAS_DL);
+    using T = Tile<TK>;
+    constexpr int TJ = T::TJ, PL = T::PL, BOX_F = T::BOX_F, HSLOT_F = T::HSLOT_F, PSLOT_F = T::PSLOT_F, PP = T::PP;
     float* hs = smem;
     float* ps = hs + NHS * HSLOT_F;
     float* sgeo = ps + NPS * PSLOT_F;
@@ -149,12 +158,12 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
     const Ring rg{smem_u32(bars), smem_u32(bars + AHEAD)};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    const int k0 = bx * TTILE_K;
-    const int j0 = 2 + by * TTILE_J;
+    const int k0 = bx * TK;
+    const int j0 = 2 + by * TJ;
     const int i0 = 1 + bz * TI;
     int seam = 0, xs = 0;
-    if (k0 == 0 && K.km - 2 > k0 + TTILE_K + 3) { seam = 1; xs = (K.km - 2) & ~3; }
-    else if (k0 > 0 && K.km - 2 >= k0 && K.km - 2 < k0 + TTILE_K) { seam = 2; xs = 0; }
+    if (k0 == 0 && K.km - 2 > k0 + TK + 3) { seam = 1; xs = (K.km - 2) & ~3; }
+    else if (k0 > 0 && K.km - 2 >= k0 && K.km - 2 < k0 + TK) { seam = 2; xs = 0; }
 
     if (smem_u32(smem) & 127u) {
         if (threadIdx.x == 0) atomicOr(plan.err, ERR_ALIGN);
@@ -184,11 +193,11 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
                     break;
                 }
                 const uint32_t bar = rg.full(s);
-                mbar_expect_tx(bar, nh * (BOX_BYTES + (seam ? SEAM_BYTES : 0u)) + (m1 - m0 - nh) * PT_BYTES);
+                mbar_expect_tx(bar, nh * (T::BOX_BYTES + (seam ? T::SEAM_BYTES : 0u)) + (m1 - m0 - nh) * T::PT_BYTES);
                 for (int m = m0; m < m0 + nh; m++) {
                     const uint32_t dst = smem_u32(hs + (s * NH + m - m0) * HSLOT_F);
                     tma_load_4d(dst, &map_main, k0 - 4, j0 - 1, i0 - 1, plan.arr[m], bar);
-                    if (seam) tma_load_4d(dst + BOX_BYTES, &map_seam, xs, j0, i0, plan.arr[m], bar);
+                    if (seam) tma_load_4d(dst + T::BOX_BYTES, &map_seam, xs, j0, i0, plan.arr[m], bar);
                 }
                 for (int m = m0 + nh; m < m1; m++) {
                     tma_load_4d(smem_u32(ps + pslot * PSLOT_F), &map_pt, k0, j0, i0, plan.arr[m], bar);
@@ -204,7 +213,7 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
     }
 
     // ---- consumers ----
-    const int row_j = warp / WPR, kl = warp % WPR * 32 + lane;   // the lane's place in the tile
+    const int row_j = warp / T::WPR, kl = warp % T::WPR * 32 + lane;   // the lane's place in the tile
     const int j = j0 + row_j, k = k0 + kl;
     {
 #pragma unroll
@@ -231,19 +240,18 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
     // ow + ii ows and oe + ii oes (in the seam box for the periodic partner)
     const int nv = (k <= K.km - 2 && j <= K.jm - 3) ? K.im - 1 - i0 : 0;
     const int c0 = (i0 * K.jm + j) * K.kp + k, plane = (int)K.plane;
-    const int row = PL + (row_j + 1) * TTILE_BX;
+    const int row = PL + (row_j + 1) * T::BX;
     const int o = row + kl + 4;
     int ow = o - 1, oe = o + 1, ows = PL, oes = PL;
     if (k == 0) {
-        if (seam == 1) { ow = BOX_F + row_j * TILE_SEAM_X + ((K.km - 2) - xs); ows = TTILE_J * TILE_SEAM_X; }
+        if (seam == 1) { ow = BOX_F + row_j * TILE_SEAM_X + ((K.km - 2) - xs); ows = TJ * TILE_SEAM_X; }
         else ow = row + (K.km - 2) - (k0 - 4);
     }
     if (k == K.km - 2) {
-        if (seam == 2) { oe = BOX_F + row_j * TILE_SEAM_X + (0 - xs); oes = TTILE_J * TILE_SEAM_X; }
+        if (seam == 2) { oe = BOX_F + row_j * TILE_SEAM_X + (0 - xs); oes = TJ * TILE_SEAM_X; }
         else oe = row + 0 - (k0 - 4);
     }
-    const int px = row_j * TTILE_K + kl;                      // the lane's place in a point box's plane
-    constexpr int PP = TTILE_J * TTILE_K;                     // floats per plane of a point box
+    const int px = row_j * TK + kl;                      // the lane's place in a point box's plane
     auto wait = [&](int n) -> bool {
         const bool ok = mbar_wait(rg.full(n % AHEAD), (uint32_t)((n / AHEAD) & 1), plan.wait_limit);
         if (!__any_sync(0xffffffffu, !ok)) return true;
@@ -317,7 +325,7 @@ __device__ __forceinline__ void block(const CUtensorMap& map_main, const CUtenso
             P[m] = ps + pslot * PSLOT_F + px;
             pslot = pslot + 1 == NPS ? 0 : pslot + 1;
         }
-        Column cy, cd;
+        Column<TK> cy, cd;
         cy.start(Y, o);
         if (HAS_DL) cd.start(D, o);
 #pragma unroll

@@ -8,33 +8,41 @@ namespace {
 
 using namespace tracer;
 
-template <int MODE, bool HAS_DL>
+template <int MODE, bool HAS_DL, int TK>
 __global__ void __launch_bounds__(tracer::THREADS, 3)
 rk_tracer_tile_kernel(const __grid_constant__ CUtensorMap map_main, const __grid_constant__ CUtensorMap map_seam,
                       const __grid_constant__ CUtensorMap map_pt, const MixedConstF K, const MixedIO io,
                       const StageParams sp, const TracerPlan plan, const int ng) {
     extern __shared__ __align__(128) float smem[];
     const int bz = blockIdx.z / ng, g = blockIdx.z - bz * ng;
-    tracer::block<MODE, HAS_DL>(map_main, map_seam, map_pt, K, io, sp, plan, smem, blockIdx.x, blockIdx.y, bz,
+    tracer::block<MODE, HAS_DL, TK>(map_main, map_seam, map_pt, K, io, sp, plan, smem, blockIdx.x, blockIdx.y, bz,
                                 group_q0(ng, g), group_q0(ng, g + 1));
 }
 
-template <int MODE, bool HAS_DL>
+template <int MODE, bool HAS_DL, int TK>
 cudaError_t launch_one(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
-                       const TracerPlan& plan, dim3 grid, cudaStream_t s) {
+                       const TracerPlan& plan, cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_tracer_tile_kernel<MODE, HAS_DL>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+        const cudaError_t e = cudaFuncSetAttribute(rk_tracer_tile_kernel<MODE, HAS_DL, TK>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<TK>::SMEM);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    const int ng = tracer_groups((int64_t)grid.x * grid.y * grid.z);
+    dim3 grid((kf.km - 1 + TK - 1) / TK, (kf.jm - 4 + Tile<TK>::TJ - 1) / Tile<TK>::TJ, (kf.im - 2 + TI - 1) / TI);
+    const int ng = tracer_groups((int64_t)grid.x * grid.y * grid.z), m = TK == 64 ? 0 : 1;
     grid.z *= ng;
-    rk_tracer_tile_kernel<MODE, HAS_DL><<<grid, THREADS, SMEM_BYTES, s>>>(
-        *reinterpret_cast<const CUtensorMap*>(maps.main4), *reinterpret_cast<const CUtensorMap*>(maps.seam4),
-        *reinterpret_cast<const CUtensorMap*>(maps.pt4), kf, io, sp, plan, ng);
+    rk_tracer_tile_kernel<MODE, HAS_DL, TK><<<grid, THREADS, Tile<TK>::SMEM, s>>>(
+        *reinterpret_cast<const CUtensorMap*>(maps.main4[m]), *reinterpret_cast<const CUtensorMap*>(maps.seam4[m]),
+        *reinterpret_cast<const CUtensorMap*>(maps.pt4[m]), kf, io, sp, plan, ng);
     return cudaGetLastError();
+}
+
+template <int MODE, bool HAS_DL>
+cudaError_t launch_tiles(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
+                         const TracerPlan& plan, cudaStream_t s) {
+    return tracer_tile_k(kf.jm, kf.km) == 64 ? launch_one<MODE, HAS_DL, 64>(maps, kf, io, sp, plan, s)
+                                             : launch_one<MODE, HAS_DL, 32>(maps, kf, io, sp, plan, s);
 }
 
 }  // namespace
@@ -49,19 +57,24 @@ int tracer_groups(int64_t tiles) {
     return tiles * 13 <= slots ? 13 : (tiles * 4 <= 2 * slots ? 4 : 1);
 }
 
+// 64 x 4 tiles read a halo a tenth smaller per cell and in longer rows than 32 x 8, so they are taken unless they pad
+// the grid by more (a ring of 66 meridians fills 128 columns of 64-wide tiles, 96 of 32-wide ones): two iterations (us)
+// at 41x181x361 (the same padding) 2194 with 64 against 2221 with 32, at 81x361x721 (276480 columns against 264960)
+// 16640 against 16500.
+int tracer_tile_k(int jm, int km) {
+    auto cells = [&](int tk, int tj) { return (int64_t)((km - 1 + tk - 1) / tk * tk) * ((jm - 4 + tj - 1) / tj * tj); };
+    return cells(64, 4) <= cells(32, 8) ? 64 : 32;
+}
+
 cudaError_t launch_rk_tracer_tile(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io,
                                   const StageParams& sp, const TracerPlan& plan, int mode, cudaStream_t s) {
-    const int nk = (kf.km - 1 + TTILE_K - 1) / TTILE_K;
-    const int nj = (kf.jm - 4 + TTILE_J - 1) / TTILE_J;
-    const int ni = (kf.im - 2 + TI - 1) / TI;
-    if (nk <= 0 || nj <= 0 || ni <= 0) return cudaSuccess;
+    if (kf.km < 2 || kf.jm < 5 || kf.im < 3) return cudaSuccess;
     if (mode == MODE_RHS || kf.divu_on || kf.fsz_over_int || plan.n_items > TRACER_MAX_ITEMS) return cudaErrorInvalidValue;
-    const dim3 grid(nk, nj, ni);
     const bool has_dl = io.dl_in[0] != nullptr;
     if (mode == MODE_STAGE)
-        return has_dl ? launch_one<MODE_STAGE, true>(maps, kf, io, sp, plan, grid, s)
-                      : launch_one<MODE_STAGE, false>(maps, kf, io, sp, plan, grid, s);
-    return has_dl ? launch_one<MODE_FINAL, true>(maps, kf, io, sp, plan, grid, s) : cudaErrorInvalidValue;
+        return has_dl ? launch_tiles<MODE_STAGE, true>(maps, kf, io, sp, plan, s)
+                      : launch_tiles<MODE_STAGE, false>(maps, kf, io, sp, plan, s);
+    return has_dl ? launch_tiles<MODE_FINAL, true>(maps, kf, io, sp, plan, s) : cudaErrorInvalidValue;
 }
 
 // the number of items the kernel consumes (the host's plan must match)

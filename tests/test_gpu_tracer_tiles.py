@@ -1,4 +1,4 @@
-"""The tracer kernel's tiles (64 x 4 x 4 cells) and stream at the sizes where they can go wrong: rings around one and two
+"""The tracer kernel's tiles (64 x 4 x 4 or 32 x 8 x 4 cells, whichever pads less) and stream at the sizes where they can go wrong: rings around one and two
 tiles' width (the periodic partner inside the box, in the seam box, alone in a tile), rows and levels that leave a
 remainder, the fields with two sources at couplings other than 1, without turbulence, in the march and tiled2 variants.
 One step, its tracers against the direct kernel (1e-7: the same FP32 arithmetic, differently contracted) and all
@@ -25,7 +25,8 @@ def step(g, P, st, variant):
 @pytest.mark.parametrize("over", [{}, {"turb_active": 0}, {"precip_coupling": 0.7, "chemical_reaction": 1.3}],
                          ids=["default", "no_turb", "couplings"])
 @pytest.mark.parametrize("shape", [(5, 9, 17), (6, 8, 64), (7, 10, 65), (8, 11, 66), (9, 12, 68), (10, 13, 69),
-                                   (11, 14, 70), (6, 9, 129), (7, 11, 134)], ids=str)
+                                   (11, 14, 70), (6, 9, 129), (7, 11, 134),
+                                   (5, 8, 33), (6, 11, 36), (7, 12, 128), (8, 10, 126), (5, 11, 193)], ids=str)
 def test_tiles_match_direct_and_oracle(shape, over):
     g, P, st = case(shape, seed=8, precision=1, **over)
     ref = st.copy()
