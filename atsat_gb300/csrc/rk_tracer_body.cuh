@@ -2,19 +2,18 @@
 // stage handling of RungeKutta_Sat_Turb.cpp:250-375), run after the momentum / temperature kernel of the
 // split variant (rk_mixed.cu) when species_divu is off.
 //
-// A block owns TK x 256 / TK x 4 cells (k, j, i), TK 64 or 32 (tracer_tile_k). A producer warp streams every array the tracers read with tensor
-// copies, in groups: the advecting winds and the eddy viscosity (three groups of point boxes, without a
-// halo), then one group per field: the halo boxes (72 x 6 x 6 or 40 x 10 x 6 floats) of its y_n copy and stage increment and
-// the point boxes of its sources, the tke/dis running sum and, at the final stage, dl_1 and dl_2. A group has one
-// "full" barrier for all of its copies and one "empty" barrier; with increments two groups are in flight, without
-// four. Eight consumer warps (32 columns of a row j, lane k, four radial levels per lane) read the boxes from shared memory;
-// at the final stage each lane loads its y_n (FP64) before it waits for the field's boxes and forms y_{n+1} there.
-// A block needs 73 KB of shared memory and 72 registers a thread: three blocks fit on an SM.
+// A block owns TK x 256 / TK x 4 cells (k, j, i), TK 64 or 32 (tracer_tile_k). A producer warp streams every array
+// the tracers read with tensor copies, in groups: the advecting winds and the eddy viscosity (three groups of point
+// boxes, without a halo), then one group per field: the halo boxes (72 x 6 x 6 or 40 x 10 x 6 floats) of its y_n copy
+// and stage increment and the point boxes of its sources, the tke/dis running sum and, at the final stage, dl_1 and
+// dl_2. A group has one "full" barrier for all of its copies and one "empty" barrier; with increments two groups are
+// in flight, without four. Eight consumer warps (32 columns of a row j, four radial levels per lane) read the boxes
+// from shared memory; at the final stage each lane loads its y_n (FP64) before it waits for the field's boxes and forms
+// y_{n+1} there. A block needs 73 KB of shared memory and 72 registers a thread: three blocks fit on an SM.
 //
-// What bounds it: memory (HBM at 88-93 % of a plain copy's rate at 41x181x361) and, close behind, issue (60 %).
-// Launches at 41x181x361, before -> now: intermediate with increments 144 -> 134 us, final stage with its FP64 half
-// 184 + 118 -> 258 us.
-// Prefetching the next groups into L2 did not help (2209-2240).
+// What bounds it: memory (84-88 % of a plain copy's rate at 41x181x361) and, close behind, issue (60 %). Launches at
+// 41x181x361, before -> now: intermediate with increments 144 -> 134 us, final stage with its FP64 half 184 + 118 ->
+// 255 us. Prefetching the next groups into L2 did not help (2209-2240 us a step pair against 2193).
 //
 // The fields run through three copies of the code (one source, two sources, tke / dis) in a loop that is not
 // unrolled. With one copy per field the program was 90 KB: at the final stage a warp in eight waited for instructions,

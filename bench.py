@@ -230,13 +230,11 @@ KERNEL_NAME = {"fp64": "rk_stage_fp64_kernel (fused RHSSat + RK4 stage, FP64)",
                "mixed_split": "rk_mom_kernel + rk_tracer_kernel<1> (split RHSSat + RK4 stage, FP32 stencils / FP64 state)",
                "mixed_split3": "rk_mom_kernel + rk_tracer_kernel<3> (split RHSSat + RK4 stage, FP32 stencils / FP64 state)",
                "mixed_split13": "rk_mom_kernel + rk_tracer_kernel<13> (split RHSSat + RK4 stage, FP32 stencils / FP64 state)",
-               "mixed_split_tiled": "rk_mom_kernel + rk_tracer_tile_kernel (split RHSSat + RK4 stage, TMA-tiled tracers; "
-                                    "final stage + final_combine_kernel)",
+               "mixed_split_tiled": "rk_mom_kernel + rk_tracer_tile_kernel (split RHSSat + RK4 stage, TMA-tiled tracers)",
                "mixed_tiled2": "rk_mom_tile_kernel + rk_tracer_tile_kernel (split RHSSat + RK4 stage, all inputs "
-                               "TMA-streamed; final stage + final_combine_kernel)",
+                               "TMA-streamed)",
                "mixed_march": "rk_mom_march_kernel + rk_tracer_tile_kernel (split RHSSat + RK4 stage: the momentum "
-                              "part as a radial march, one TMA plane per stencil array and level; final stage + "
-                              "final_combine_kernel)"}
+                              "part as a radial march, one TMA plane per stencil array and level)"}
 
 
 def cpu_baseline(g, P, seed, target_s=3.0):
@@ -480,7 +478,7 @@ def measure(a, rank, world, g, P, st, pinned, precision):
         # the FP64 roofline that binds: FP64 instructions per interior cell and stage counted by ncu
         # (profiles/rk_stage_fp64_21x91x181.md) over the same CUDA-event stage time, against 2 per SM per cycle
         sm_hz = (clk.get("sm_mhz") or 2070.0) * 1e6
-        per_cell = 590.0
+        per_cell = 303.0
         ach = per_cell * interior_rk(g) / (avg_ms / 1e3)
         peak64 = 2.0 * 152 * sm_hz
         roof["fp64_pipe"] = {"instructions_per_cell": per_cell, "achieved_per_s": ach, "peak_per_s": peak64,
