@@ -1293,7 +1293,7 @@ MarchPlan make_plan_march(atsat_dyn* h, const MixedIO& io, int mode) {
     return pl;
 }
 
-// kernels of one stage without the final combine
+// kernels of one stage
 int launches_per_stage(atsat_dyn* h, const MixedIO& io, int mode) {
     if (h->variant < ATSAT_DYN_STAGE_SPLIT) return 1;
     return h->variant == ATSAT_DYN_STAGE_MARCH && stage_fusable(h->kf, make_plan_march(h, io, mode), mode) ? 1 : 2;

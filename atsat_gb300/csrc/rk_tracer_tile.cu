@@ -1,5 +1,5 @@
-// Launches of the TMA-tiled tracer kernel on its own (rk_tracer_body.cuh): the split_tiled and tiled2 variants and the
-// march variant's final stage. The march variant's intermediate stages run it fused (rk_stage_fused.cu).
+// Launches of the TMA-tiled tracer kernel on its own (rk_tracer_body.cuh): the split_tiled and tiled2 variants, and the
+// march variant where its two kernels do not share a launch (stage_fusable in rk_stage_fused.cu).
 #include "rk_tracer_body.cuh"
 
 namespace atsat {
