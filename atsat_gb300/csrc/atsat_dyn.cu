@@ -457,9 +457,11 @@ cudaError_t upload_stage_geo(atsat_dyn* h) {
         s.c_the = K.Coriolis * c.cor_the;
         s.c_v = K.Coriolis * c.cor_phi * c.costhe;
         s.c_u = K.Coriolis * c.cor_phi * c.sinthe_true;
-        s.c_0 = s.c_v * c.vbar0 + s.c_u * c.ubar0;
+        s.vbar0 = c.vbar0;
+        s.ubar0 = c.ubar0;
         s.cent_rad = K.centrifugal * c.cent_rad;
         s.cent_the = K.centrifugal * c.cent_the;
+        s.pad = 0.0;
     }
     const cudaError_t e = cudaMemcpyAsync(h->sgeo, sg.data(), sizeof(StageGeo) * sg.size(), cudaMemcpyHostToDevice,
                                           h->stream);

@@ -104,16 +104,18 @@ static_assert(sizeof(ColGeo) == 36 * 8, "ColGeo layout");
 // host. Diffusion as one weight per stencil value (l_rp for f(i+1), l_rm for f(i-1), l_tp / l_tm along theta,
 // l_p for both phi neighbours, l_0 for the centre; lu_rp / lu_rm for u, whose radial term is 4/rm du/dr), the
 // gradients' scales (s_the = 1 / (2 dtheta rm), s_phi = 1 / (2 dphi rm sin)), the cross terms of the u, v, w
-// diffusion (x_*) and the body forces (c_v v + c_u u - c_0 is the phi Coriolis term with the held means).
+// diffusion (x_*) and the body forces (c_v (v - vbar0) + c_u (u - ubar0) is the phi Coriolis term; vbar0, ubar0 the held
+// means, subtracted first: near them the term is a small difference that products formed before it would round away).
 struct alignas(16) StageGeo {
     double s_the, s_phi, l_rp, l_rm;
     double lu_rp, lu_rm, l_tp, l_tm;
     double l_p, l_0, inv_rm, cot;
     double v_metric, u_metric, x_v1, x_v2;
     double x_w1, c_rad, c_the, c_v;
-    double c_u, c_0, cent_rad, cent_the;
+    double c_u, vbar0, ubar0, cent_rad;
+    double cent_the, pad;
 };
-static_assert(sizeof(StageGeo) == 24 * 8, "StageGeo layout");
+static_assert(sizeof(StageGeo) == 26 * 8, "StageGeo layout");
 
 // Grid-wide constants, every one formed on the host in the reference's own expression order.
 struct KConst {

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
         const double xw = fma(g.x_w1, u_p, fma(g.x_v2, v_p, -(g.v_metric * w)));
         const double rhs_v = apply_centred(wt, dv, fma(visc, xv, fma(-mv, g.inv_rm, fma(-g.c_the, w, g.cent_the) - pth)));
         const double rhs_w = apply_centred(wt, dw, fma(visc, xw, fma(-mw, g.inv_rm,
-                                           fma(-g.c_v, v, fma(-g.c_u, u, g.c_0)) - pph)));
+                                           fma(-g.c_v, v - g.vbar0, fma(-g.c_u, u - g.ubar0, -pph)))));
         emit<MODE>(io, sp, K, ATSAT_F_U, c, rhs_u);
         emit<MODE>(io, sp, K, ATSAT_F_V, c, rhs_v);
         emit<MODE>(io, sp, K, ATSAT_F_W, c, rhs_w);
