@@ -44,22 +44,24 @@ __device__ __forceinline__ double clip_half(double x) {
     return (hi_word(x) >> 31) ? -0.5 : 0.5;
 }
 
+// The tendency r of field q into the state; `out` the tendency as it is written where it is asked for. What is written
+// must not change the state, so the sums are pinned: every instance rounds them alike.
 template <int MODE>
 __device__ __forceinline__ void emit(const StageIO<double>& io, const StageParams& sp, const KConst& K, int q,
-                                     int64_t c, double r) {
+                                     int64_t c, double r, double out) {
     if (MODE == MODE_RHS) {
-        io.rhs[q][c] = r;
+        io.rhs[q][c] = out;
         return;
     }
     double y;
     if (MODE == MODE_STAGE) {
         const double a = fma(sp.wgt, r, (sp.stage == 0) ? 0.0 : io.acc[q][c]);
         io.acc[q][c] = a;
-        y = ldg(io.yn[q] + c) + sp.c_in * r;
+        y = fma(sp.c_in, r, ldg(io.yn[q] + c));
     } else {
-        const double a = io.acc[q][c] + sp.wgt * r;
-        y = ldg(io.yn[q] + c) + sp.sixth_dt * a;
-        if (sp.write_all_rhs || q < 3) io.rhs[q][c] = r;
+        const double a = fma(sp.wgt, r, io.acc[q][c]);
+        y = fma(sp.sixth_dt, a, ldg(io.yn[q] + c));
+        if (sp.write_all_rhs || q < 3) io.rhs[q][c] = out;
     }
     if (q == ATSAT_F_TKE) {
         if (hi_word(y) >= hi_word(K.tke_max)) y = smin(smax(y, 0.0), K.tke_max);
@@ -122,9 +124,9 @@ constexpr int RKS_ROWS = 4, RKS_BLOCKS = 4;
 //   u, v, w always combine differences to the centre (five operations more per field): their tendencies are
 //   results (the projection's source), w's zonal differences are small against w, and differences of near-equal
 //   values are exact. So do k* and omega*: the closure floors k* to a uniform value and divides by gradients that
-//   a uniform field must leave at zero. t and the species do the same where their tendencies are asked for
-//   (CENTRED); else the tendency only enters y + dt r, and the rounding of weight times value, eps sum |weight| |f|,
-//   is there below eps |f| times dt sum |weight| -- the Courant number that a stable step keeps under 3.
+//   a uniform field must leave at zero. t and the species enter y + dt r by weights on the values: the rounding,
+//   eps sum |weight| |f|, is there below eps |f| times dt sum |weight| -- the Courant number that a stable step keeps
+//   under 3. Where their tendencies are results too (CENTRED), those are formed from the differences beside.
 // PLAIN: the default switches (`plain_knobs`), whose branches are then left out at compile time: an instruction
 // the compiler predicates off still takes its slot of the FP64 pipe.
 template <int MODE, bool CENTRED, bool PLAIN>
@@ -203,9 +205,9 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
         const double rhs_v = apply_centred(wt, dv, fma(visc, xv, fma(-mv, g.inv_rm, fma(-g.c_the, w, g.cent_the) - pth)));
         const double rhs_w = apply_centred(wt, dw, fma(visc, xw, fma(-mw, g.inv_rm,
                                            fma(-g.c_v, v - g.vbar0, fma(-g.c_u, u - g.ubar0, -pph)))));
-        emit<MODE>(io, sp, K, ATSAT_F_U, c, rhs_u);
-        emit<MODE>(io, sp, K, ATSAT_F_V, c, rhs_v);
-        emit<MODE>(io, sp, K, ATSAT_F_W, c, rhs_w);
+        emit<MODE>(io, sp, K, ATSAT_F_U, c, rhs_u, rhs_u);
+        emit<MODE>(io, sp, K, ATSAT_F_V, c, rhs_v, rhs_v);
+        emit<MODE>(io, sp, K, ATSAT_F_W, c, rhs_w, rhs_w);
         if (MODE != MODE_STAGE) {
             io.aux[0][c] = rhs_u + dpr;
             io.aux[1][c] = rhs_v + dpth;
@@ -217,10 +219,12 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
     }
 
     // kappa diffusion - transport + extra of field q
-    auto tendency = [&](int q, const Wt& wt, double extra) -> double {
+    auto tendency = [&](int q, const Wt& wt, double extra) {
         const S7 f = load(q);
-        const bool turb = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
-        return (CENTRED || turb) ? apply_centred(wt, centred(f), extra) : apply_values(wt, f, extra);
+        const bool centre = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
+        const double out = CENTRED || centre ? apply_centred(wt, centred(f), extra) : 0.0;
+        const double r = MODE == MODE_RHS || centre ? out : apply_values(wt, f, extra);
+        emit<MODE>(io, sp, K, q, c, r, out);
     };
 
     // ---- temperature (RHS_Sat_Turb.cpp:368-386, 409, 435-437, 611-665, 752-759) ----
@@ -242,14 +246,14 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
         }
         if (K.precip_on) r += clip_half(K.precip_factor * ldg(io.q_precip + c));
         if (!PLAIN && K.tmf_on) r -= K.tmf_chem * ldg(io.thermalmassflux + c);
-        emit<MODE>(io, sp, K, ATSAT_F_T, c, tendency(ATSAT_F_T, weights(K.inv_re_pr + nue_t_s, U, V, W, g), r));
+        tendency(ATSAT_F_T, weights(K.inv_re_pr + nue_t_s, U, V, W, g), r);
     }
 
     // ---- species (RHS_Sat_Turb.cpp:409-431, 457-491, 839-937) ----
     auto species = [&](int q, const Wt& wt, double extra) {
         double r = extra;
         if (!PLAIN && K.divu_on) r -= sd * ldg(io.in[q] + c);
-        emit<MODE>(io, sp, K, q, c, tendency(q, wt, r));
+        tendency(q, wt, r);
     };
     const double pc = PLAIN ? 1.0 : K.precip_coupling, chem = PLAIN ? 1.0 : K.chem;
     // fma(1, a, b) is a + b bit for bit
@@ -274,9 +278,9 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
     // ---- k-omega transport (RHS_Sat_Turb.cpp:511-538) ----
     if (K.turb) {
         wt = weights(fma(nue_c, K.inv_sig_k, K.inv_re), U, V, W, g);
-        emit<MODE>(io, sp, K, ATSAT_F_TKE, c, tendency(ATSAT_F_TKE, wt, ldg(io.tke_source + c)));
+        tendency(ATSAT_F_TKE, wt, ldg(io.tke_source + c));
         wt = weights(fma(nue_c, K.inv_sig_w, K.inv_re), U, V, W, g);
-        emit<MODE>(io, sp, K, ATSAT_F_DIS, c, tendency(ATSAT_F_DIS, wt, ldg(io.dis_source + c)));
+        tendency(ATSAT_F_DIS, wt, ldg(io.dis_source + c));
     } else if (MODE == MODE_RHS || (MODE == MODE_FINAL && sp.write_all_rhs)) {
         io.rhs[ATSAT_F_TKE][c] = 0.0;
         io.rhs[ATSAT_F_DIS][c] = 0.0;
