@@ -92,7 +92,11 @@ __device__ __forceinline__ Wt weights(double kappa, double U, double V, double W
               fma(kappa, g.l_p, -W), fma(kappa, g.l_p, W), kappa * g.l_0};
 }
 
-// extra + sum over the neighbours of weight times difference to the centre
+// sum over the neighbours of weight times difference to the centre
+__device__ __forceinline__ double apply_centred(const Wt& w, const S7& d) {
+    return fma(w.rp, d.rp, fma(w.rm, d.rm, fma(w.tp, d.tp, fma(w.tm, d.tm, fma(w.pe, d.pe, w.pw * d.pw)))));
+}
+// the same and `extra`, first in the chain: no operation of its own, but six roundings at its size
 __device__ __forceinline__ double apply_centred(const Wt& w, const S7& d, double extra) {
     return fma(w.rp, d.rp, fma(w.rm, d.rm, fma(w.tp, d.tp, fma(w.tm, d.tm, fma(w.pe, d.pe, fma(w.pw, d.pw, extra))))));
 }
@@ -116,8 +120,8 @@ constexpr int RKS_ROWS = 4, RKS_BLOCKS = 4;
 
 // What bounds it: the FP64 pipe (two operations per SM per cycle). With the differences of each field scaled and
 // combined one by one it was 590 FP64 instructions per interior cell and 2.38 ms per launch at 41x181x361, while
-// the launch's 1.97 GB take 0.29 ms. So the kernel is written for the fewest FP64 operations: 302 per cell, 1.46 ms
-// (the two-iteration step 20.03 -> 12.68 ms; at 27x118x222 the launch 0.595 -> 0.362 ms). Transport and diffusion of
+// the launch's 1.97 GB take 0.29 ms. So the kernel is written for the fewest FP64 operations: 307 per cell, 1.47 ms
+// (the two-iteration step 20.03 -> 12.84 ms). Transport and diffusion of
 // RHS_Sat_Turb.cpp:300-1000 together are one weight per stencil value: seven fused multiply-adds per field with
 // weights that cost seven more per diffusivity -- shared by the three phases of a species, by u, v and w, and by the
 // water and ammonia groups where their Schmidt numbers are equal. Comparisons run on the integer pipe.
@@ -189,29 +193,33 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
                 else buoyancy_u = K.kbuoy * (K.g * ps / (K.rR * t_c * K.t_ref) - ldg(io.buoy + i));
             }
         }
-        double fu = fma(visc, g.u_metric * u, fma(-g.c_rad, w, g.cent_rad + buoyancy_u) - dpr);
+        double fu = fma(visc, g.u_metric * u, fma(-g.c_rad, w, g.cent_rad + buoyancy_u));
         if (!PLAIN && !K.metric_split) fu = fma(K.metric_on * g.inv_rm, fma(v, v, w * w), fu);
-        const double rhs_u = apply_centred(wu, du, fu);
 
-        double pth = dpth, pph = dpph;
-        if (PLAIN || K.metric_split) {
-            pth = fma(ldg(io.p_metric + c + kp) - ldg(io.p_metric + c - kp), g.s_the, pth);
-            pph = fma(ldg(io.p_metric + c + dke) - ldg(io.p_metric + c + dkw), g.s_phi, pph);
-        }
+        // p_metric's gradient with the metric terms (theta) and with the Coriolis force (phi)
         const double wcot = w * g.cot;
-        const double mv = fma(u, v, -(w * wcot)), mw = fma(w, u, v * wcot);
+        double mv = fma(u, v, -(w * wcot));
+        const double mw = fma(w, u, v * wcot);
+        double fw = fma(-g.c_v, v - g.vbar0, -(g.c_u * (u - g.ubar0)));
+        if (PLAIN || K.metric_split) {
+            mv = fma(ldg(io.p_metric + c + kp) - ldg(io.p_metric + c - kp), K.inv_2dthe, mv);
+            fw = fma(-(ldg(io.p_metric + c + dke) - ldg(io.p_metric + c + dkw)), g.s_phi, fw);
+        }
         const double xv = fma(g.x_v1, u_t, -fma(g.x_v2, w_p, g.v_metric * v));
         const double xw = fma(g.x_w1, u_p, fma(g.x_v2, v_p, -(g.v_metric * w)));
-        const double rhs_v = apply_centred(wt, dv, fma(visc, xv, fma(-mv, g.inv_rm, fma(-g.c_the, w, g.cent_the) - pth)));
-        const double rhs_w = apply_centred(wt, dw, fma(visc, xw, fma(-mw, g.inv_rm,
-                                           fma(-g.c_v, v - g.vbar0, fma(-g.c_u, u - g.ubar0, -pph)))));
+        // The tendencies without p_dyn's gradient (aux), which would round away part of them: it comes last. The large
+        // forces of v and w come after their stencil sums too, whose steps would each round at the forces' size.
+        const double aux_u = apply_centred(wu, du, fu);
+        const double aux_v = fma(-mv, g.inv_rm, fma(visc, xv, apply_centred(wt, dv))) + fma(-g.c_the, w, g.cent_the);
+        const double aux_w = fma(-mw, g.inv_rm, fma(visc, xw, apply_centred(wt, dw))) + fw;
+        const double rhs_u = aux_u - dpr, rhs_v = aux_v - dpth, rhs_w = aux_w - dpph;
         emit<MODE>(io, sp, K, ATSAT_F_U, c, rhs_u, rhs_u);
         emit<MODE>(io, sp, K, ATSAT_F_V, c, rhs_v, rhs_v);
         emit<MODE>(io, sp, K, ATSAT_F_W, c, rhs_w, rhs_w);
         if (MODE != MODE_STAGE) {
-            io.aux[0][c] = rhs_u + dpr;
-            io.aux[1][c] = rhs_v + dpth;
-            io.aux[2][c] = rhs_w + dpph;
+            io.aux[0][c] = aux_u;
+            io.aux[1][c] = aux_v;
+            io.aux[2][c] = aux_w;
         }
         if (!PLAIN && K.divu_on)
             sd = K.species_divu * ((du.rp - du.rm) * K.inv_2dr + 2.0 * u * g.inv_rm + (dv.tp - dv.tm) * g.s_the
@@ -222,7 +230,8 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
     auto tendency = [&](int q, const Wt& wt, double extra) {
         const S7 f = load(q);
         const bool centre = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
-        const double out = CENTRED || centre ? apply_centred(wt, centred(f), extra) : 0.0;
+        const double out = centre ? apply_centred(wt, centred(f)) + extra
+                                  : CENTRED ? apply_centred(wt, centred(f), extra) : 0.0;
         const double r = MODE == MODE_RHS || centre ? out : apply_values(wt, f, extra);
         emit<MODE>(io, sp, K, q, c, r, out);
     };

@@ -33,3 +33,18 @@ def test_no_zonal_coriolis_force_on_the_held_means(shape):
     a = rhs_pass(g, P, st)
     assert np.all(a[F.RHS_W][1:-1, 2:-2, :-1] == 0.0)
     assert np.any(a[F.RHS_V][1:-1, 2:-2, :-1] != 0.0)
+
+
+@pytest.mark.parametrize("over", [{}, {"metric_split": 0, "coriolis_split": 0}, {"species_divu": 1.0}],
+                         ids=lambda o: ",".join(o) or "default")
+def test_aux_does_not_see_the_pressure_gradient(over):
+    """aux_u, aux_v, aux_w are the tendencies without the gradient of p_dyn. Formed as the tendency plus that gradient,
+    they carry its rounding, which is large against them where the gradient is; so they are the same bits at any p_dyn."""
+    g, P, st = case((7, 12, 34), seed=4, **over)
+    a = rhs_pass(g, P, st)
+    strong = st.copy()
+    strong.arrays[F.P_DYN] *= 1.0e3
+    b = rhs_pass(g, P, strong)
+    for aux, rhs in ((F.AUX_U, F.RHS_U), (F.AUX_V, F.RHS_V), (F.AUX_W, F.RHS_W)):
+        assert np.array_equal(a[aux], b[aux]), F.NAMES[aux]
+        assert not np.array_equal(a[rhs], b[rhs])
