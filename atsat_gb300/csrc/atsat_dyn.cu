@@ -427,6 +427,14 @@ void build_mixed_constants(atsat_dyn* h) {
     F.tke_max_d = K.tke_max; F.dis_min_d = K.dis_min;
 }
 
+// Host data into device memory on the handle's stream, there when it returns. That stream does not wait for the default
+// stream, on which a copy from pageable memory may return before the data is on the device: a kernel launched next could
+// read the memory before the copy.
+cudaError_t upload_now(atsat_dyn* h, void* dst, const void* src, size_t bytes) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(h->stream);
+}
+
 // the FP64 stage kernel's column table, from the geometry
 cudaError_t upload_stage_geo(atsat_dyn* h) {
     const KConst& K = h->kc;
@@ -463,9 +471,7 @@ cudaError_t upload_stage_geo(atsat_dyn* h) {
         s.cent_the = K.centrifugal * c.cent_the;
         s.pad = 0.0;
     }
-    const cudaError_t e = cudaMemcpyAsync(h->sgeo, sg.data(), sizeof(StageGeo) * sg.size(), cudaMemcpyHostToDevice,
-                                          h->stream);
-    return e != cudaSuccess ? e : cudaStreamSynchronize(h->stream);
+    return upload_now(h, h->sgeo, sg.data(), sizeof(StageGeo) * sg.size());
 }
 
 cudaError_t upload_geof(atsat_dyn* h) {
@@ -776,7 +782,7 @@ int route_binding(atsat_dyn* h, int fid) {
         }
         // a transfer queued earlier (asynchronous mode) may still read the old table
         CK(h, cudaStreamSynchronize(h->stream));
-        CK(h, cudaMemcpy(h->dev_rows[fid], h->bind_rows[fid].data(), n * sizeof(double*), cudaMemcpyHostToDevice));
+        CK(h, upload_now(h, h->dev_rows[fid], h->bind_rows[fid].data(), n * sizeof(double*)));
     }
     h->direct[fid] = true;
     return ATSAT_DYN_OK;
@@ -820,7 +826,7 @@ int finish(atsat_dyn* h, bool host_result = false) {
         unsigned int v = 0;
         CK(h, cudaMemcpy(&v, h->dev_err, sizeof(v), cudaMemcpyDeviceToHost));
         if (v) {
-            CK(h, cudaMemset(h->dev_err, 0, sizeof(v)));
+            CK(h, cudaMemsetAsync(h->dev_err, 0, sizeof(v), h->stream));
             h->timeouts++;
             return fail(h, ATSAT_DYN_E_TIMEOUT, "tiled stage kernel: device status 0x%x (1 producer wait, 2 consumer "
                         "wait, 4 plan mismatch, 8 shared-memory alignment)", v);
@@ -1780,7 +1786,7 @@ int setup_press_variants(atsat_dyn* h) {
             A2 += 1.0 / (rm * rm);
         }
         double* dtab = q; q += n_tab;
-        e = cudaMemcpy(dtab, tab.data(), (size_t)n_tab * 8, cudaMemcpyHostToDevice);
+        e = upload_now(h, dtab, tab.data(), (size_t)n_tab * 8);
         if (e != cudaSuccess) return fail(h, ATSAT_DYN_E_CUDA, "pressure variant tables: %s", cudaGetErrorString(e));
         BaroTables& T = h->baro;
         T.N = N; T.NM = NM; T.J = J; T.NU = (int)NU;
@@ -1809,7 +1815,7 @@ int setup_turbulence(atsat_dyn* h) {
     const int64_t total = K.fsz + (int64_t)jm * K.kp + n_tab + 16;
     cudaError_t e = cudaMalloc(&h->turb_buf, (size_t)total * 8);
     if (e != cudaSuccess) { h->turb_buf = nullptr; return fail(h, ATSAT_DYN_E_NOMEM, "turbulence: %s", cudaGetErrorString(e)); }
-    e = cudaMemset(h->turb_buf, 0, (size_t)total * 8);
+    e = cudaMemsetAsync(h->turb_buf, 0, (size_t)total * 8, h->stream);
     if (e != cudaSuccess) return fail(h, ATSAT_DYN_E_CUDA, "turbulence: %s", cudaGetErrorString(e));
     double* q = h->turb_buf;
     h->turb_prod = q; q += K.fsz;
@@ -1850,7 +1856,7 @@ int setup_turbulence(atsat_dyn* h) {
         for (int j = 0; j < jm; j++) s_p2[(size_t)i * jm + j] = irs[(size_t)i * jm + j] * irs[(size_t)i * jm + j];
     }
     double* d = q;
-    e = cudaMemcpy(d, t.data(), (size_t)n_tab * 8, cudaMemcpyHostToDevice);
+    e = upload_now(h, d, t.data(), (size_t)n_tab * 8);
     if (e != cudaSuccess) return fail(h, ATSAT_DYN_E_CUDA, "turbulence tables: %s", cudaGetErrorString(e));
     TurbTables& T = h->ttab;
     T.rm = d; T.inv_rm = d + im; T.inv_rm2dthe = d + 2 * im; T.height_m = d + 3 * im; T.thick_m = d + 4 * im;
@@ -2042,7 +2048,7 @@ int atsat_dyn_create(const atsat_dyn_grid* g, const atsat_dyn_params* p, atsat_d
         return cuda_fail(e, "cudaMalloc (budget)");
     h->clamp_cells = reinterpret_cast<unsigned long long*>(h->clamp_added + 22);
     h->clamp_partial = h->clamp_added + 44;
-    if ((e = cudaMemset(h->clamp_added, 0, 44 * 8)) != cudaSuccess) return cuda_fail(e, "cudaMemset (budget)");
+    if ((e = cudaMemsetAsync(h->clamp_added, 0, 44 * 8, h->stream)) != cudaSuccess) return cuda_fail(e, "cudaMemset (budget)");
     *out = h;
     return setup_press_variants(h);
 }
