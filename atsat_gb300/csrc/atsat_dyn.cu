@@ -1618,19 +1618,6 @@ int enqueue_clamp(atsat_dyn* h, bool resident = false) {
 
 }  // namespace
 
-int atsat::sm_count() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
-            cudaGetLastError();
-            v = 152;
-        }
-        return v;
-    }();
-    return n;
-}
-
 extern "C" {
 
 int atsat_dyn_abi_version(void) { return ATSAT_DYN_ABI_VERSION; }

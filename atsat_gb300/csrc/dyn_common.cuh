@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/atsat_dyn.h"
+#include "per_device.h"
 
 namespace atsat {
 
@@ -374,7 +375,6 @@ cudaError_t launch_rk_mom(const MixedConstF& kf, const MixedIO& io, const StageP
 int tracer_plan_items(int mode, bool has_dl, bool turb);
 int tracer_tile_k(int jm, int km);  // the tracer kernel's tile width for this grid
 int tracer_groups(int64_t tiles);   // field groups (blocks per tile) of the tracer kernel for this many tiles
-int sm_count();                     // SMs of the current device
 // the momentum / temperature equations alone, TMA-tiled (species_divu off)
 cudaError_t launch_rk_mom_tile(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                                const TracerPlan& plan, int mode, cudaStream_t s);

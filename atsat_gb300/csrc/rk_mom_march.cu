@@ -21,14 +21,10 @@ rk_mom_march_kernel(const __grid_constant__ CUtensorMap map_plane, const __grid_
 template <int MODE, bool HAS_DL, bool CMP>
 cudaError_t launch_one(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const MarchPlan& plan, dim3 grid, cudaStream_t s) {
-    static bool attr = false;
     constexpr size_t smem = Shape<MODE, CMP>::SMEM;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_mom_march_kernel<MODE, HAS_DL, CMP>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SharedMemory shared;
+    const cudaError_t e = shared.allow((const void*)rk_mom_march_kernel<MODE, HAS_DL, CMP>, smem);
+    if (e != cudaSuccess) return e;
     rk_mom_march_kernel<MODE, HAS_DL, CMP><<<grid, THREADS, smem, s>>>(
         *reinterpret_cast<const CUtensorMap*>(maps.plane1), *reinterpret_cast<const CUtensorMap*>(maps.seam1),
         *reinterpret_cast<const CUtensorMap*>(maps.pt1), kf, io, sp, plan);

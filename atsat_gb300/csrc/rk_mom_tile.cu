@@ -383,13 +383,9 @@ rk_mom_tile_kernel(const __grid_constant__ CUtensorMap map_main, const __grid_co
 template <int MODE, bool HAS_DL>
 cudaError_t launch_one(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const TracerPlan& plan, dim3 grid, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_mom_tile_kernel<MODE, HAS_DL>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SharedMemory shared;
+    const cudaError_t e = shared.allow((const void*)rk_mom_tile_kernel<MODE, HAS_DL>, SMEM_BYTES);
+    if (e != cudaSuccess) return e;
     rk_mom_tile_kernel<MODE, HAS_DL><<<grid, THREADS, SMEM_BYTES, s>>>(
         *reinterpret_cast<const CUtensorMap*>(maps.main), *reinterpret_cast<const CUtensorMap*>(maps.seam),
         *reinterpret_cast<const CUtensorMap*>(maps.pt2), kf, io, sp, plan);

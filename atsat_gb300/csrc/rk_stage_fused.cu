@@ -46,14 +46,10 @@ rk_stage_fused_kernel(const __grid_constant__ CUtensorMap plane, const __grid_co
 template <int MODE, bool HAS_DL, int TK>
 cudaError_t launch_tile(const TileMaps& m, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const MarchPlan& mp, const TracerPlan& tp, const FusedGrid& G, cudaStream_t s) {
-    static bool attr = false;
     constexpr size_t smem = Fused<MODE, TK>::SMEM;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_stage_fused_kernel<MODE, HAS_DL, TK>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SharedMemory shared;
+    const cudaError_t e = shared.allow((const void*)rk_stage_fused_kernel<MODE, HAS_DL, TK>, smem);
+    if (e != cudaSuccess) return e;
     constexpr int t = TK == 64 ? 0 : 1;
     auto map = [](const unsigned char* p) -> const CUtensorMap& { return *reinterpret_cast<const CUtensorMap*>(p); };
     rk_stage_fused_kernel<MODE, HAS_DL, TK><<<G.nm + G.nt * G.ng, march::THREADS, smem, s>>>(

@@ -214,13 +214,9 @@ rk_tile_kernel(const __grid_constant__ CUtensorMap map_main, const __grid_consta
 template <int MODE, bool HAS_DL>
 cudaError_t launch_one(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const TilePlan& plan, dim3 grid, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_tile_kernel<MODE, HAS_DL>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SharedMemory shared;
+    const cudaError_t e = shared.allow((const void*)rk_tile_kernel<MODE, HAS_DL>, SMEM_BYTES);
+    if (e != cudaSuccess) return e;
     rk_tile_kernel<MODE, HAS_DL><<<grid, THREADS, SMEM_BYTES, s>>>(
         *reinterpret_cast<const CUtensorMap*>(maps.main), *reinterpret_cast<const CUtensorMap*>(maps.seam), kf, io,
         sp, plan);

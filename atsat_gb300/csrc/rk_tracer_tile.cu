@@ -22,13 +22,9 @@ rk_tracer_tile_kernel(const __grid_constant__ CUtensorMap map_main, const __grid
 template <int MODE, bool HAS_DL, int TK>
 cudaError_t launch_one(const TileMaps& maps, const MixedConstF& kf, const MixedIO& io, const StageParams& sp,
                        const TracerPlan& plan, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(rk_tracer_tile_kernel<MODE, HAS_DL, TK>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<TK>::SMEM);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SharedMemory shared;
+    const cudaError_t e = shared.allow((const void*)rk_tracer_tile_kernel<MODE, HAS_DL, TK>, Tile<TK>::SMEM);
+    if (e != cudaSuccess) return e;
     dim3 grid((kf.km - 1 + TK - 1) / TK, (kf.jm - 4 + Tile<TK>::TJ - 1) / Tile<TK>::TJ, (kf.im - 2 + TI - 1) / TI);
     const int ng = tracer_groups((int64_t)grid.x * grid.y * grid.z), m = TK == 64 ? 0 : 1;
     grid.z *= ng;
