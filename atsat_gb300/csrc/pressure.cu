@@ -11,6 +11,8 @@
 
 #include "dyn_common.cuh"
 
+#include <cmath>
+
 namespace atsat {
 
 namespace {
@@ -72,8 +74,8 @@ __global__ void prep_seam_kernel(const KConst K, double* const* __restrict__ six
 // the integer pipe (positive doubles order as integers, finiteness is an exponent test), lc_old's three second
 // differences accumulate into div by fma. LEGACY: the source div(aux - rhs); INCR: lc_old is added. They are compiled in
 // because an instruction predicated off still takes its slot of that pipe: 98 -> 88 us at 41x181x361
-// (the operations alone are 64).
-template <bool LEGACY, bool INCR>
+// (the operations alone are 64). CAP: the cap may be negative or NaN, whose bits do not order so: the comparison itself.
+template <bool LEGACY, bool INCR, bool CAP>
 __global__ void __launch_bounds__(256) press_source_kernel(
         const KConst K, const ColGeo* __restrict__ geo, const double* __restrict__ su,
         const double* __restrict__ sv, const double* __restrict__ sw, const double* __restrict__ rhs_u,
@@ -107,7 +109,9 @@ __global__ void __launch_bounds__(256) press_source_kernel(
         const double src_max = ldg(&g->p_den) * K.pdyn_cap;
         const long long bits = __double_as_longlong(div), mag = bits & 0x7FFFFFFFFFFFFFFFll;
         if (mag >= 0x7FF0000000000000ll) { div = 0.0; clamped = true; }
-        else if (mag > __double_as_longlong(src_max)) {      // src_max > 0
+        else if (CAP) {
+            if (fabs(div) > src_max) { div = (div > src_max) ? src_max : -src_max; clamped = true; }
+        } else if (mag > __double_as_longlong(src_max)) {
             div = __longlong_as_double(__double_as_longlong(src_max) | (bits & (long long)0x8000000000000000ull));
             clamped = true;
         }
@@ -231,12 +235,20 @@ cudaError_t launch_press_source(const KConst& kc, const ColGeo* geo, const doubl
                                 const double* rhs_u, const double* rhs_v, const double* rhs_w, const double* p,
                                 double* src, unsigned long long* nclamp, cudaStream_t s) {
     dim3 block(32, 8), grid((kc.km - 1 + 31) / 32, (kc.jm + 7) / 8, kc.im);
-    if (kc.press_src == 0)          // press_incr is off then
-        press_source_kernel<true, false><<<grid, block, 0, s>>>(kc, geo, aux_u, aux_v, aux_w, rhs_u, rhs_v, rhs_w, p, src, nclamp);
-    else if (kc.press_incr)
-        press_source_kernel<false, true><<<grid, block, 0, s>>>(kc, geo, su, sv, sw, rhs_u, rhs_v, rhs_w, p, src, nclamp);
-    else
-        press_source_kernel<false, false><<<grid, block, 0, s>>>(kc, geo, su, sv, sw, rhs_u, rhs_v, rhs_w, p, src, nclamp);
+    auto go = [&](auto kernel, const double* x, const double* y, const double* z) {
+        kernel<<<grid, block, 0, s>>>(kc, geo, x, y, z, rhs_u, rhs_v, rhs_w, p, src, nclamp);
+    };
+    const bool cap = !(kc.pdyn_cap >= 0.0) || std::signbit(kc.pdyn_cap);
+    if (kc.press_src == 0) {        // press_incr is off then
+        if (cap) go(press_source_kernel<true, false, true>, aux_u, aux_v, aux_w);
+        else go(press_source_kernel<true, false, false>, aux_u, aux_v, aux_w);
+    } else if (kc.press_incr) {
+        if (cap) go(press_source_kernel<false, true, true>, su, sv, sw);
+        else go(press_source_kernel<false, true, false>, su, sv, sw);
+    } else {
+        if (cap) go(press_source_kernel<false, false, true>, su, sv, sw);
+        else go(press_source_kernel<false, false, false>, su, sv, sw);
+    }
     return cudaGetLastError();
 }
 
