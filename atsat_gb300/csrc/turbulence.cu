@@ -12,6 +12,8 @@
 // closure (SST) has a source kernel of its own that applies the floors and caps where it reads and writes (sst_kernel).
 #include "dyn_common.cuh"
 
+#include <cmath>
+
 namespace atsat {
 namespace {
 
@@ -225,20 +227,22 @@ __device__ __forceinline__ double floor_at(double x, double lo) {
     const unsigned long long b = bits_of(x);
     return b > bits_of(lo) && b <= INF_BITS ? x : lo;
 }
-// (hi < x) ? hi : x for x, hi >= 0 or NaN
+// (hi < x) ? hi : x for x >= +0 or NaN, hi any but -0 and a NaN with its sign bit set (as signed integers a negative hi
+// is below every x)
 __device__ __forceinline__ double cap_at(double x, double hi) {
     const unsigned long long b = bits_of(x);
-    return b > bits_of(hi) && b <= INF_BITS ? hi : x;
+    return (long long)b > __double_as_longlong(hi) && b <= INF_BITS ? hi : x;
 }
 // clamp3(x, -s, s), s >= 0
 __device__ __forceinline__ double clip_to(double x, double s) {
     const unsigned long long b = bits_of(x), m = b & ~SIGN_BIT;
     return m > bits_of(s) && m <= INF_BITS ? __longlong_as_double((long long)(bits_of(s) | (b & SIGN_BIT))) : x;
 }
-// clamp3(x, 0, hi)
+// clamp3(x, 0, hi), hi as in cap_at
 __device__ __forceinline__ double clip_positive(double x, double hi) {
     const unsigned long long b = bits_of(x);
-    if (b & SIGN_BIT) return b > SIGN_BIT && b <= (SIGN_BIT | INF_BITS) ? 0.0 : x;
+    if (b > SIGN_BIT) return b <= (SIGN_BIT | INF_BITS) ? 0.0 : x;
+    if (b == SIGN_BIT) return __double_as_longlong(hi) < 0 ? hi : x;
     return cap_at(x, hi);
 }
 __device__ __forceinline__ bool finite_double(double x) { return (bits_of(x) & INF_BITS) != INF_BITS; }
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(256) turb_floor_kernel(const TurbArgs A) {
     A.dis[c] = floor_at(A.dis[c], DIS_MIN);
 }
 
-// The wall copy at i = 0 and the cap of nue on the cells the source kernel leaves alone (no taper: the cap is then
+// The wall copy at i = 0 and the cap of nue on the cells the source kernel leaves alone (no taper, a cap >= 0: it is then
 // idempotent there). blockIdx.z: the planes i = 0 and im-1; the rows j = 0 and jm-1; the meridian km-1, and k = 0 where
 // the seam is not periodic.
 __global__ void __launch_bounds__(128) turb_edges_kernel(const TurbArgs A) {
@@ -547,7 +551,8 @@ cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const 
     A.L_m = p.L_atm * 1.0e3;
     A.nue_air = tp.nue_gas;
     A.re_turb = tp.vel_star_ref * tp.z_0 / tp.nue_gas;
-    A.nue_max = tp.nue_max_phys / (p.u_0 * A.L_m);
+    A.nue_max = tp.nue_max_phys / (p.u_0 * A.L_m) + 0.0;     // -0 becomes +0, which compares the same
+    if (std::isnan(A.nue_max)) A.nue_max = std::fabs(A.nue_max);
     A.k_bg_nd = tp.k_bg / (p.u_0 * p.u_0);
     A.vel_star_max = tp.vel_star_max;
     A.dr = tab.dr; A.dthe = tab.dthe; A.dphi = tab.dphi;
@@ -592,7 +597,7 @@ cudaError_t launch_turbulence(const KConst& K, const atsat_dyn_params& p, const 
         sst_kernel<<<g4, b4, 0, s>>>(A);
         turb_floor_kernel<<<g8, b8, 0, s>>>(A);
         *launches += 3;
-        if (tp.abl_taper) {
+        if (tp.abl_taper || !(A.nue_max >= 0.0)) {           // capping twice is not capping once
             turb_wall_kernel<<<gw, 128, 0, s>>>(A);
             turb_nue_cap_kernel<<<g8, b8, 0, s>>>(A);
             *launches += 2;
