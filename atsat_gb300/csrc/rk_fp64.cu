@@ -121,7 +121,7 @@ constexpr int RKS_ROWS = 4, RKS_BLOCKS = 4;
 // What bounds it: the FP64 pipe (two operations per SM per cycle). With the differences of each field scaled and
 // combined one by one it was 590 FP64 instructions per interior cell and 2.38 ms per launch at 41x181x361, while
 // the launch's 1.97 GB take 0.29 ms. So the kernel is written for the fewest FP64 operations: 307 per cell, 1.47 ms
-// (the two-iteration step 20.03 -> 12.84 ms). Transport and diffusion of
+// (the two-iteration step 20.03 -> 12.72 ms). Transport and diffusion of
 // RHS_Sat_Turb.cpp:300-1000 together are one weight per stencil value: seven fused multiply-adds per field with
 // weights that cost seven more per diffusivity -- shared by the three phases of a species, by u, v and w, and by the
 // water and ammonia groups where their Schmidt numbers are equal. Comparisons run on the integer pipe.
@@ -226,13 +226,11 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
                                    + v * g.cot * g.inv_rm + w_p * g.s_phi);
     }
 
-    // kappa diffusion - transport + extra of field q
+    // kappa diffusion - transport + extra of t or a species
     auto tendency = [&](int q, const Wt& wt, double extra) {
         const S7 f = load(q);
-        const bool centre = q == ATSAT_F_TKE || q == ATSAT_F_DIS;
-        const double out = centre ? apply_centred(wt, centred(f)) + extra
-                                  : CENTRED ? apply_centred(wt, centred(f), extra) : 0.0;
-        const double r = MODE == MODE_RHS || centre ? out : apply_values(wt, f, extra);
+        const double out = CENTRED ? apply_centred(wt, centred(f), extra) : 0.0;
+        const double r = MODE == MODE_RHS ? out : apply_values(wt, f, extra);
         emit<MODE>(io, sp, K, q, c, r, out);
     };
 
@@ -285,11 +283,19 @@ __global__ void __launch_bounds__(32 * RKS_ROWS, RKS_BLOCKS) rk_stage_fp64_kerne
     species(ATSAT_F_NH4SH, wt, fma(chem, ldg(io.massflux_nh4sh + c), ldg(io.fluxlim_nh4sh + c)));
 
     // ---- k-omega transport (RHS_Sat_Turb.cpp:511-538) ----
+    // The eddy viscosity enters as it is: an infinite one makes the diffusion infinite, which the limits of k* and
+    // omega* in emit take; as weights on differences of either sign it would make it NaN.
+    auto closure = [&](int q, double inv_sig, double source) {
+        const double kappa = fma(nue_c, inv_sig, K.inv_re);
+        const S7 d = centred(load(q));
+        double r;
+        if (finite(nue_c)) r = apply_centred(weights(kappa, U, V, W, g), d) + source;
+        else r = fma(kappa, apply_centred(weights(1.0, 0.0, 0.0, 0.0, g), d), apply_centred(weights(0.0, U, V, W, g), d) + source);
+        emit<MODE>(io, sp, K, q, c, r, r);
+    };
     if (K.turb) {
-        wt = weights(fma(nue_c, K.inv_sig_k, K.inv_re), U, V, W, g);
-        tendency(ATSAT_F_TKE, wt, ldg(io.tke_source + c));
-        wt = weights(fma(nue_c, K.inv_sig_w, K.inv_re), U, V, W, g);
-        tendency(ATSAT_F_DIS, wt, ldg(io.dis_source + c));
+        closure(ATSAT_F_TKE, K.inv_sig_k, ldg(io.tke_source + c));
+        closure(ATSAT_F_DIS, K.inv_sig_w, ldg(io.dis_source + c));
     } else if (MODE == MODE_RHS || (MODE == MODE_FINAL && sp.write_all_rhs)) {
         io.rhs[ATSAT_F_TKE][c] = 0.0;
         io.rhs[ATSAT_F_DIS][c] = 0.0;
