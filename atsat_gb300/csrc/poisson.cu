@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <omp.h>
@@ -689,20 +690,35 @@ struct PoissonSolver {
 
 namespace {
 
-// The transform's blocks: a few row pairs (warps) each, so that they even out over the SMs and the stores of a mode still
-// fill a sector or more (four FP32 pairs are 64 bytes, two FP64 pairs too): FP64 at 21x91x181, 855 pairs, 53 us with
-// eight pairs per block, 25 with two; FP32 at 41x181x361 17.0 with eight, 15.6 with four. False: the ring length is
-// beyond one row pair in shared memory.
+// The transform's blocks: a few row pairs each, a warp per pair, so that they even out over the SMs and the stores of a
+// mode still fill a sector or more (four FP32 pairs are 64 bytes, two FP64 pairs too): FP64 at 21x91x181, 855 pairs, 53 us
+// with eight pairs per block, 25 with two; FP32 at 41x181x361 17.0 with eight, 15.6 with four. A ring with a prime
+// factor above 64 has more outputs per stage than a warp has lanes for, and long ones: a block of BLOCK_LANES per pair.
+// Direct solves (FP64, FP32; us) with a warp and with a block: 9x21x360 (ring of 359) 451, 159 against 210, 109;
+// 11x41x548 920, 264 against 499, 160; 41x181x360 2867, 533 against 2842, 544. Below, the warp is the faster by up to
+// 5 % (refined solve at 41x181x134, a ring of 7 x 19, 1464 against 1528 us; at 41x181x97 1376 against 1441).
+// False: the ring length is beyond one row pair in shared memory.
+constexpr int BLOCK_LANES = 128;
+
 template <typename T>
 bool plan_spectral(const Spec& S, FftPlan& F) {
     fft_plan(S.n, F);
-    for (F.warps = sizeof(T) == 4 ? 4 : 2; F.warps > 1 && fft_smem<T>(F, S.n) > 100 * 1024; F.warps--) {}
+    F.lanes = 32;
+    for (int q = 0; q < F.stages; q++)
+        if (F.radix[q] > 64) F.lanes = BLOCK_LANES;
+    for (F.pairs = F.lanes > 32 ? 1 : sizeof(T) == 4 ? 4 : 2; F.pairs > 1 && fft_smem<T>(F, S.n) > 100 * 1024; F.pairs--) {}
     if (fft_smem<T>(F, S.n) > 220 * 1024) return false;
-    auto allow = [](const void* fn) {      // the limit is the kernel's, shared by every handle
-        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) == cudaSuccess;
+    auto allow = [](auto lanes) {          // the limit is the kernel's, shared by every handle
+        constexpr int N = decltype(lanes)::value;
+        auto one = [](const void* fn) {
+            return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) == cudaSuccess;
+        };
+        bool ok = one((const void*)fft_fwd_kernel<T, N>) && one((const void*)fft_inv_kernel<T, N, T, false>);
+        if constexpr (sizeof(T) == 4) ok = ok && one((const void*)fft_inv_kernel<T, N, double, true>);
+        return ok;
     };
-    bool ok = allow((const void*)fft_fwd_kernel<T>) && allow((const void*)fft_inv_kernel<T, T, false>);
-    if constexpr (sizeof(T) == 4) ok = ok && allow((const void*)fft_inv_kernel<T, double, true>);
+    const bool ok = F.lanes == 32 ? allow(std::integral_constant<int, 32>{})
+                                  : allow(std::integral_constant<int, BLOCK_LANES>{});
     if (!ok) cudaGetLastError();
     return ok;
 }
@@ -1149,11 +1165,17 @@ cudaError_t direct(PoissonSolver* P, const T* rhs, To* x, T* spec, const T* W, c
     const Spec& S = P->S;
     const FftPlan& F = fft_of<T>(P);
     if (!(sizeof(T) == 8 ? P->spectral64 : P->spectral32)) return cudaErrorInvalidValue;
-    const dim3 rows(((S.NI + 1) / 2 + F.warps - 1) / F.warps, S.NJ);
-    fft_fwd_kernel<T><<<rows, 32 * F.warps, fft_smem<T>(F, S.n), P->stream>>>(K, S, F, rhs, tw, spec);
-    const cudaError_t e = launch_bt<T>(S, sizeof(T) == 8 ? P->bt64 : P->bt32, W, P->bvec_d, P->cvec_d, spec, P->stream);
+    const dim3 rows(((S.NI + 1) / 2 + F.pairs - 1) / F.pairs, S.NJ);
+    const size_t smem = fft_smem<T>(F, S.n);
+    auto both = [&](auto fwd, auto inv) -> cudaError_t {
+        fwd<<<rows, F.lanes * F.pairs, smem, P->stream>>>(K, S, F, rhs, tw, spec);
+        const cudaError_t e = launch_bt<T>(S, sizeof(T) == 8 ? P->bt64 : P->bt32, W, P->bvec_d, P->cvec_d, spec, P->stream);
+        if (e == cudaSuccess) inv<<<rows, F.lanes * F.pairs, smem, P->stream>>>(K, S, F, spec, tw, x);
+        return e;
+    };
+    const cudaError_t e = F.lanes == 32 ? both(fft_fwd_kernel<T, 32>, fft_inv_kernel<T, 32, To, ADD>)
+                                        : both(fft_fwd_kernel<T, BLOCK_LANES>, fft_inv_kernel<T, BLOCK_LANES, To, ADD>);
     if (e != cudaSuccess) return e;
-    fft_inv_kernel<T, To, ADD><<<rows, 32 * F.warps, fft_smem<T>(F, S.n), P->stream>>>(K, S, F, spec, tw, x);
     return cudaGetLastError();
 }
 

@@ -26,7 +26,7 @@ template <typename T> struct alignas(4 * sizeof(T)) Quad { T x, y, z, w; };
 // product of the radices before the stage and mag = ceil(2^32 / s) for the division by it.
 constexpr int FFT_MAX_STAGES = 16;
 struct FftPlan {
-    int stages, warps, stride;           // row pairs (warps) per block; complex values per pair and buffer
+    int stages, pairs, lanes, stride;    // row pairs per block; threads per pair; complex values per pair and buffer
     int radix[FFT_MAX_STAGES], s[FFT_MAX_STAGES];
     uint32_t mag[FFT_MAX_STAGES];
 };
@@ -95,25 +95,48 @@ __device__ __forceinline__ void stage(const Cx<T>* x, Cx<T>* y, const Cx<T>* tw,
     }
 }
 
-// any other radix: a lane per output value
-template <typename T>
-__device__ __forceinline__ void stage_any(const Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, int R, int s, uint32_t mag,
-                                          int lane, int step) {
-    const int items = n / R;
-    int u = lane / items, e = lane - u * items;
+// Any other radix, an odd one: the inputs t and R - t become their sum and difference in place, and a lane forms the
+// outputs u and R - u together from the sums' cosine part and the differences' sine part, 2 R operations a pair of
+// outputs where R complex products each took 8 R. A ring of one prime R takes R^2 / 2 operations per real row; the direct
+// real sums took R^2.
+template <typename T, class Sync>
+__device__ __forceinline__ void stage_any(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, int R, int s, uint32_t mag,
+                                          int lane, int step, Sync sync) {
+    const int items = n / R, h = R / 2;
     const int du = step / items, de = step - du * items;
-    for (int w = lane; w < n; w += step) {
+    int u = lane / items, e = lane - u * items;
+    for (int w = lane; w < h * items; w += step) {
+        Cx<T>*p = x + e + (u + 1) * items, *q = x + e + (R - 1 - u) * items;
+        const Cx<T> a = *p, b = *q;
+        *p = a + b;
+        *q = a - b;
+        u += du;
+        if ((e += de) >= items) { e -= items; u++; }
+    }
+    sync();
+    u = lane / items;
+    e = lane - u * items;
+    for (int w = lane; w < (h + 1) * items; w += step) {
         const int p = s == 1 ? e : (int)__umulhi((uint32_t)e, mag), q = e - p * s, turn_by = u * items;
-        Cx<T> b = x[e];
+        Cx<T> c = x[e], d = {(T)0, (T)0};
         int idx = 0;
-        for (int t = 1; t < R; t++) {
+#pragma unroll 4
+        for (int t = 1; t <= h; t++) {
             idx += turn_by;                                          // t u (n / R) mod n
             if (idx >= n) idx -= n;
-            const Cx<T> c = tw[idx];
-            b = b + turn(x[e + t * items], c.re, c.im);
+            const Cx<T> f = tw[idx], a = x[e + t * items], b = x[e + (R - t) * items];
+            c.re = fma(f.re, a.re, c.re);
+            c.im = fma(f.re, a.im, c.im);
+            d.re = fma(f.im, b.re, d.re);
+            d.im = fma(f.im, b.im, d.im);
         }
-        const Cx<T> c = tw[p * s * u];
-        y[q + s * (R * p + u)] = turn(b, c.re, c.im);
+        const Cx<T> f = tw[p * s * u];
+        Cx<T>* o = y + q + s * R * p;
+        o[s * u] = turn(Cx<T>{c.re + d.im, c.im - d.re}, f.re, f.im);
+        if (u) {
+            const Cx<T> g = tw[p * s * (R - u)];
+            o[s * (R - u)] = turn(Cx<T>{c.re - d.im, c.im + d.re}, g.re, g.im);
+        }
         u += du;
         if ((e += de) >= items) { e -= items; u++; }
     }
@@ -132,49 +155,53 @@ __device__ __forceinline__ Cx<T>* fft(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n
             case 3: stage<T, 3>(x, y, tw, n, s, mag, lane, step); break;
             case 4: stage<T, 4>(x, y, tw, n, s, mag, lane, step); break;
             case 5: stage<T, 5>(x, y, tw, n, s, mag, lane, step); break;
-            default: stage_any<T>(x, y, tw, n, R, s, mag, lane, step); break;
+            default: stage_any<T>(x, y, tw, n, R, s, mag, lane, step, sync); break;
         }
         sync();
         Cx<T>* z = x; x = y; y = z;
     }
     return x;
 }
-template <typename T>
-__device__ __forceinline__ Cx<T>* fft_warp(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, const FftPlan& F, int lane) {
-    return fft(x, y, tw, n, F, lane, 32, [] { __syncwarp(); });
+// by a warp, or by a block of LANES threads
+template <typename T, int LANES>
+__device__ __forceinline__ Cx<T>* fft_lanes(Cx<T>* x, Cx<T>* y, const Cx<T>* tw, int n, const FftPlan& F, int lane) {
+    if constexpr (LANES == 32) return fft(x, y, tw, n, F, lane, 32, [] { __syncwarp(); });
+    else return fft(x, y, tw, n, F, lane, LANES, [] { __syncthreads(); });
 }
 
 template <typename T>
-size_t fft_smem(const FftPlan& F, int n) { return ((size_t)F.warps * 2 * F.stride + n) * sizeof(Cx<T>); }
+size_t fft_smem(const FftPlan& F, int n) { return ((size_t)F.pairs * 2 * F.stride + n) * sizeof(Cx<T>); }
 
-// Two real rows per complex transform (radial rows 2q and 2q + 1 as real and imaginary part), one warp per pair, the
-// stages in shared memory without block barriers. The direct sums this replaces took n (n + 2) multiply-adds per row:
-// 343 us forward and 387 us inverse (FP32) for the 39 x 179 rows of 360 at 41x181x361, 104 and 178 us (FP64) at
-// 21x91x181; now 15.8 and 29.2 us (with the FP64 p += e), 24.8 and 25.5 us. Bound by its traffic in FP32 (20 MB in and
-// out) and by the FP64 pipe in FP64.
-template <typename T>
+// Two real rows per complex transform (radial rows 2q and 2q + 1 as real and imaginary part), LANES threads per pair: a
+// warp, whose stages in shared memory need no block barrier, or a block (plan_spectral). The direct sums this replaces
+// took n (n + 2) multiply-adds per row: 343 us forward and 387 us inverse (FP32) for the 39 x 179 rows of 360 at
+// 41x181x361, 104 and 178 us (FP64) at 21x91x181; now 15.8 and 29.2 us (with the FP64 p += e), 24.8 and 25.5 us. The
+// FP32 passes' 20 MB take 3 us at the copy rate: the rest is the stages' steps through shared memory; FP64 is bound by
+// its pipe. The rounding error is relative to the larger row of a pair. The equation couples the two more strongly than
+// any other neighbours, so a row's own rounding reaches the other through the solve at the same size.
+template <typename T, int LANES>
 __global__ void fft_fwd_kernel(const KConst K, const Spec S, const FftPlan F, const T* __restrict__ x,
                                const T* __restrict__ twt, T* __restrict__ spec) {
     extern __shared__ __align__(16) unsigned char dsm[];
     Cx<T>* tw = reinterpret_cast<Cx<T>*>(dsm);
     Cx<T>* buf = tw + S.n;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int jj = blockIdx.y, pair0 = blockIdx.x * F.warps, ii = 2 * (pair0 + warp);
+    const int lane = threadIdx.x % LANES, pair = threadIdx.x / LANES;
+    const int jj = blockIdx.y, pair0 = blockIdx.x * F.pairs, ii = 2 * (pair0 + pair);
     for (int k = threadIdx.x; k < S.n; k += blockDim.x) tw[k] = {twt[k], twt[S.n + k]};
-    Cx<T>* a = buf + (size_t)warp * 2 * F.stride;
+    Cx<T>* a = buf + (size_t)pair * 2 * F.stride;
     const int64_t row = ((int64_t)(ii + 1) * K.jm + jj + 1) * K.kp;
     const bool two = ii + 1 < S.NI;
     if (ii < S.NI)
-        for (int k = lane; k < S.n; k += 32) a[k] = {x[row + k], two ? x[row + K.plane + k] : (T)0};
+        for (int k = lane; k < S.n; k += LANES) a[k] = {x[row + k], two ? x[row + K.plane + k] : (T)0};
     __syncthreads();
     if (ii < S.NI) {
-        Cx<T>* r = fft_warp(a, a + F.stride, tw, S.n, F, lane);
+        Cx<T>* r = fft_lanes<T, LANES>(a, a + F.stride, tw, S.n, F, lane);
         if (r != a)
-            for (int k = lane; k < S.n; k += 32) a[k] = r[k];
+            for (int k = lane; k < S.n; k += LANES) a[k] = r[k];
     }
     __syncthreads();
     // split Z into the rows' cosine and sine sums; the pairs of a mode side by side
-    const int np = min(F.warps, (S.NI + 1) / 2 - pair0);
+    const int np = min(F.pairs, (S.NI + 1) / 2 - pair0);
     for (int e = threadIdx.x; e < np * S.M; e += blockDim.x) {
         const int m = e / np, q = e - m * np;
         const Cx<T>* z = buf + (size_t)q * 2 * F.stride;
@@ -186,16 +213,16 @@ __global__ void fft_fwd_kernel(const KConst K, const Spec S, const FftPlan F, co
 }
 
 // The inverse; ADD: add the result to `x` in FP64 (the defect correction's p += e) instead of storing it.
-template <typename T, typename To, bool ADD>
+template <typename T, int LANES, typename To, bool ADD>
 __global__ void fft_inv_kernel(const KConst K, const Spec S, const FftPlan F, const T* __restrict__ spec,
                                const T* __restrict__ twt, To* __restrict__ x) {
     extern __shared__ __align__(16) unsigned char dsm[];
     Cx<T>* tw = reinterpret_cast<Cx<T>*>(dsm);
     Cx<T>* buf = tw + S.n;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int jj = blockIdx.y, pair0 = blockIdx.x * F.warps, ii = 2 * (pair0 + warp);
+    const int lane = threadIdx.x % LANES, pair = threadIdx.x / LANES;
+    const int jj = blockIdx.y, pair0 = blockIdx.x * F.pairs, ii = 2 * (pair0 + pair);
     for (int k = threadIdx.x; k < S.n; k += blockDim.x) tw[k] = {twt[k], twt[S.n + k]};
-    const int np = min(F.warps, (S.NI + 1) / 2 - pair0);
+    const int np = min(F.pairs, (S.NI + 1) / 2 - pair0);
     for (int e = threadIdx.x; e < np * S.M; e += blockDim.x) {
         const int m = e / np, q = e - m * np;
         const Quad<T> v = *reinterpret_cast<const Quad<T>*>(spec + ((int64_t)m * S.NJ + jj) * S.RS + 4 * (pair0 + q));
@@ -210,12 +237,12 @@ __global__ void fft_inv_kernel(const KConst K, const Spec S, const FftPlan F, co
     }
     __syncthreads();
     if (ii >= S.NI) return;
-    Cx<T>* a = buf + (size_t)warp * 2 * F.stride;
-    const Cx<T>* r = fft_warp(a, a + F.stride, tw, S.n, F, lane);
+    Cx<T>* a = buf + (size_t)pair * 2 * F.stride;
+    const Cx<T>* r = fft_lanes<T, LANES>(a, a + F.stride, tw, S.n, F, lane);
     const T inv_n = (T)1 / (T)S.n;
     const int64_t row = ((int64_t)(ii + 1) * K.jm + jj + 1) * K.kp;
     const bool two = ii + 1 < S.NI;
-    for (int k = lane; k < S.n; k += 32) {
+    for (int k = lane; k < S.n; k += LANES) {
         const T u = r[k].re * inv_n, v = -r[k].im * inv_n;
         if constexpr (ADD) {
             x[row + k] += f2d(u);

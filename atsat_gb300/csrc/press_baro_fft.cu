@@ -156,7 +156,8 @@ __global__ void baro_inverse_sums_kernel(const BaroTables B) {
 // the stages for N and the shared memory, 0 where a pair does not fit
 size_t plan(int N, FftPlan& F) {
     fft_plan(N, F);
-    F.warps = 1;                       // one pair per block
+    F.pairs = 1;
+    F.lanes = BT;
     const size_t b = fft_smem<double>(F, N);
     return b > 220 * 1024 ? 0 : b;
 }
