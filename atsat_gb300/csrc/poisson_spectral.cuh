@@ -444,41 +444,66 @@ __global__ void bt_solve_kernel(const Spec S, const BtLayout L, const T* __restr
         for (int jj = 0; jj < NJ; jj++) f[(int64_t)jj * rs + o] -= avg;
 }
 
-// The same solve for radial systems whose rows do not fit the registers: one block per mode and part, W from global
-// memory (column-major) inside the chain, the FP64 kernel's sums.
-template <typename T>
-__global__ void bt_solve_wide_kernel(const Spec S, const T* __restrict__ W, const double* __restrict__ bvec,
-                                     const double* __restrict__ cvec, T* __restrict__ spec) {
+// The same solve for radial systems whose rows do not fit the registers: one block per mode and part, the FP64 kernel's
+// sums, W from global memory (column-major) in batches of AHEAD columns. A batch is loaded while the one before is summed,
+// and a product's first batch and its row of f before the barrier that releases the vector: with single loads the
+// chain waited for a load every four columns (the FP64 direct solve at
+// 61x61x121, 59 rows: 1266 -> 555 us; FP32 at 90x61x121: 1729 -> 547).
+template <typename T, int AHEAD, int THREADS>
+__global__ void __launch_bounds__(THREADS) bt_solve_wide_kernel(const Spec S, const T* __restrict__ W,
+                                                                const double* __restrict__ bvec,
+                                                                const double* __restrict__ cvec, T* __restrict__ spec) {
     const int m = blockIdx.x >> 1, part = blockIdx.x & 1;
     const int NI = S.NI, NJ = S.NJ, r = threadIdx.x;
     extern __shared__ __align__(16) unsigned char dsm[];
     T* g = reinterpret_cast<T*>(dsm);
     T* f = spec + (int64_t)m * NJ * S.RS + part;
     const int64_t ws = (int64_t)NI * NI;
-    const T* Wm = W + (int64_t)m * NJ * ws;
-    const bool pin = m == 0 && r == 0;
+    const bool own = r < NI, pin = m == 0 && r == 0;
+    const T* Wr = W + (int64_t)m * NJ * ws + (own ? r : 0);
+    T w[AHEAD];                                             // the next product's first batch
+    auto load = [&](T* b, const T* wp, int c0) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; u++) b[u] = c0 + u < NI ? wp[(int64_t)(c0 + u) * NI] : (T)0;
+    };
     auto product = [&](int jj) {
+        const T* wp = Wr + jj * ws;
         T acc = 0;
-        if (r < NI)
-            for (int c = 0; c < NI; c++) acc += Wm[jj * ws + (int64_t)c * NI + r] * g[c];
-        __syncthreads();
+        for (int c0 = 0; c0 < NI; c0 += AHEAD) {
+            T next[AHEAD];
+            if (c0 + AHEAD < NI) load(next, wp, c0 + AHEAD);
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++)
+                if (c0 + u < NI) acc += w[u] * g[c0 + u];
+#pragma unroll
+            for (int u = 0; u < AHEAD; u++) w[u] = next[u];
+        }
         return acc;
     };
-    if (r < NI) f[2 * r] = g[r] = pin ? (T)0 : f[2 * r];
+    load(w, Wr, 0);
+    if (own) f[2 * r] = g[r] = pin ? (T)0 : f[2 * r];
     __syncthreads();
     for (int jj = 1; jj < NJ; jj++) {
+        T* row = f + (int64_t)jj * S.RS + 2 * r;
+        const T fj = own ? *row : (T)0, b = own ? (T)bvec[jj * NI + r] : (T)0;
         const T acc = product(jj - 1);
-        if (r < NI) f[(int64_t)jj * S.RS + 2 * r] = g[r] = f[(int64_t)jj * S.RS + 2 * r] - (T)bvec[jj * NI + r] * acc;
+        load(w, Wr + jj * ws, 0);
+        __syncthreads();
+        if (own) *row = g[r] = fj - b * acc;
         __syncthreads();
     }
     double sum = 0.0;
     for (int jj = NJ - 1; jj >= 0; jj--) {
+        T* row = f + (int64_t)jj * S.RS + 2 * r;
+        const T fj = own && jj > 0 ? row[-S.RS] : (T)0;
+        const T cj = own && jj > 0 && !(pin && jj == 1) ? (T)cvec[(jj - 1) * NI + r] : (T)0;
         const T x = product(jj);
-        if (r < NI) {
-            f[(int64_t)jj * S.RS + 2 * r] = x;
+        if (jj > 0) load(w, Wr + (jj - 1) * ws, 0);
+        __syncthreads();
+        if (own) {
+            *row = x;
             sum += (double)x;
-            if (jj > 0)
-                g[r] = f[(int64_t)(jj - 1) * S.RS + 2 * r] - (pin && jj == 1 ? (T)0 : (T)cvec[(jj - 1) * NI + r]) * x;
+            if (jj > 0) g[r] = fj - cj * x;
         }
         __syncthreads();
     }
@@ -488,9 +513,9 @@ __global__ void bt_solve_wide_kernel(const Spec S, const T* __restrict__ W, cons
         if ((r & 31) == 0) red[r >> 5] = sum;
         __syncthreads();
         double s = 0.0;
-        for (unsigned w = 0; w < blockDim.x / 32; w++) s += red[w];
+        for (unsigned w_ = 0; w_ < blockDim.x / 32; w_++) s += red[w_];
         const T avg = (T)(s / ((double)NI * NJ));
-        if (r < NI)
+        if (own)
             for (int jj = 0; jj < NJ; jj++) f[(int64_t)jj * S.RS + 2 * r] -= avg;
     }
 }
@@ -509,8 +534,13 @@ cudaError_t launch_bt(const Spec& S, const BtLayout& L, const T* W, const double
         else if (L.nc == 20) go(bt_solve_kernel<T, 20, 1>);
         else if (L.nc == 40) go(bt_solve_kernel<T, 40, 1>);
     }
-    if (!L.nc)
-        bt_solve_wide_kernel<T><<<2 * S.M, (S.NI + 31) / 32 * 32, (size_t)S.NI * sizeof(T), s>>>(S, W, bvec, cvec, spec);
+    if (!L.nc) {                       // the wider batch where the registers of a larger block allow it
+        auto wide = [&](auto kernel) {
+            kernel<<<2 * S.M, (S.NI + 31) / 32 * 32, (size_t)S.NI * sizeof(T), s>>>(S, W, bvec, cvec, spec);
+        };
+        if (S.NI <= 256) wide(bt_solve_wide_kernel<T, 16, 256>);
+        else wide(bt_solve_wide_kernel<T, 4, 1024>);
+    }
     return cudaGetLastError();
 }
 
