@@ -263,8 +263,11 @@ __global__ void fft_inv_kernel(const KConst K, const Spec S, const FftPlan F, co
 // matrix-vector products, so what counts is the latency of one step, and with a few warps per SM that is its number of
 // instructions. W, f and g are in registers before the vector is ready, loaded DEPTH steps ahead; W is laid out so that
 // a thread's share of a product is NC / 2 vector loads without bounds (BtLayout); the vector is read from shared memory
-// in 16-byte words; one barrier a step. LANES lanes share a dot product where the sum's order is free (FP32); in FP64 a
-// lane keeps the sequential sum: on this ill-conditioned operator another order moves the result by as much as its error.
+// in 16-byte words; one barrier a step. In FP32 LANES lanes share a dot product, each a contiguous range of columns: the
+// defect that a correction leaves oscillates from row to row, so sums over neighbours stay small where sums over every
+// LANES-th row grow and cancel only at the end. (With strided lanes the corrections contracted by 0.8 instead of 0.63 at
+// 42x9x9, and a solve at 61x61x121 took 16 of them instead of 12.) In FP64 a lane keeps the sequential sum: on this
+// ill-conditioned operator another order moves the result by as much as its error.
 // At 41x181x361 (181 modes, 357 steps), FP32: 2487 us with W and f read from global memory inside the chain, a mode part
 // per block; 248 us with W streamed through a shared-memory ring by bulk copies (waiting for a phase, reading the ring
 // and releasing the slot took 550 of a step's 1140 cycles); 235 us with plain column-major W in registers (260 cycles of
@@ -273,7 +276,7 @@ __global__ void fft_inv_kernel(const KConst K, const Spec S, const FftPlan F, co
 template <typename T> struct BtShape { static constexpr int LANES = sizeof(T) == 4 ? 4 : 1; };
 
 // W of a (mode, polar row): value u of thread t at (u / 2 * width + t) * 2 + u % 2, zero beyond the matrix.
-//   FP32: t = 4 r + q (width: the block's threads), u -> column q + 4 u;  FP64: t = r (width: NI), u -> column u
+//   FP32: t = 4 r + q (width: the block's threads), u -> column q nc + u;  FP64: t = r (width: NI), u -> column u
 // nc = 0: plain column-major, element (r, c) at c NI + r (the wide kernel).
 struct BtLayout {
     int nc, width, threads;
@@ -297,7 +300,7 @@ template <typename T>
 inline int64_t bt_place(const BtLayout& L, int NI, int r, int c) {
     constexpr int LANES = BtShape<T>::LANES;
     if (!L.nc) return (int64_t)c * NI + r;
-    const int t = LANES == 4 ? 4 * r + c % 4 : r, u = c / LANES;
+    const int t = LANES == 4 ? 4 * r + c / L.nc : r, u = LANES == 4 ? c % L.nc : c;
     return ((int64_t)(u / 2) * L.width + t) * 2 + (u & 1);
 }
 
@@ -306,8 +309,8 @@ __global__ void bt_solve_kernel(const Spec S, const BtLayout L, const T* __restr
                                 const double* __restrict__ cvec, T* __restrict__ spec) {
     using V2 = typename Vec2<T>::V;
     constexpr int LANES = BtShape<T>::LANES;
-    // the vector, double buffered: FP32 the pairs (a, b) of column c at lane c % 4, place c / 4; FP64 a part after the
-    // other. Zero beyond NI.
+    // the vector, double buffered: FP32 the pairs (a, b) of the columns in order; FP64 a part after the other. Zero
+    // beyond NI.
     constexpr int HALF = LANES == 4 ? 2 * NC : NC;          // values of one lane (FP32) or part (FP64)
     constexpr int NV = LANES == 4 ? 4 * HALF : 2 * HALF;
     __shared__ __align__(16) T gb[2][NV];
@@ -329,7 +332,7 @@ __global__ void bt_solve_kernel(const Spec S, const BtLayout L, const T* __restr
     if (r >= NI) r = 0;
     const bool pin = m == 0 && r == 0;
     const int o = 2 * r + part;
-    const int place = LANES == 4 ? (r & 3) * HALF + 2 * (r >> 2) + part : part * HALF + r;
+    const int place = LANES == 4 ? o : part * HALF + r;
     // the couplings do not depend on j but for the folded end rows
     const T b_mid = (T)bvec[NI + r], b_end = (T)bvec[(NJ - 1) * NI + r];
     const T c_mid = (T)cvec[NI + r], c_0 = pin ? (T)0 : (T)cvec[r];
