@@ -3002,8 +3002,13 @@ int atsat_dyn_poisson_solve(atsat_dyn_t h, int32_t method, const double* src, do
     // The source goes up and the result comes down by the SMs in place where they address host memory (host_xfer.cu).
     // A result array fresh from the allocator has no pages yet, and the GPU's faults on them cost more than the
     // transfer (21 MB at 41x181x361: 4.8 ms): the host threads touch its pages, values unchanged, while the source is
-    // on its way up (2.92 -> 2.67 ms for the whole refined solve there, 0.53 -> 0.49 ms direct at 21x91x181).
-    const bool in_place = h->host_direct && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(p)) & 7u) == 0;
+    // on its way up. Copies against in place, whole calls, FP64 direct: 41x181x361 2290 -> 2030 us, 21x91x181 509 -> 452,
+    // 21x60x121 324 -> 309. Below, the threads and the faults cost more than a copy's staging (13x50x101 254 against
+    // 258 us, 9x21x33 143 against 162, 5x7x9 107 against 133): copies up to IN_PLACE_CELLS.
+    constexpr int64_t IN_PLACE_CELLS = 100000;
+    const int64_t cells = (int64_t)K.im * K.jm * K.km;
+    const bool in_place = h->host_direct && cells >= IN_PLACE_CELLS &&
+                          ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(p)) & 7u) == 0;
     auto move = [&](const double* host, double* dev, int to_device) {
         HostBatch b{};
         b.n = 1;
@@ -3013,7 +3018,6 @@ int atsat_dyn_poisson_solve(atsat_dyn_t h, int32_t method, const double* src, do
     };
     if (in_place) {
         CK(h, move(src, f, 1));
-        const int64_t cells = (int64_t)K.im * K.jm * K.km;
 #pragma omp parallel for schedule(static)
         for (int64_t c = 0; c < cells; c += 512) {
             volatile double* page = p + c;
