@@ -11,6 +11,7 @@
 #include "dyn_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace atsat {
 
@@ -124,7 +125,10 @@ __global__ void bc_phi_kernel(const KConst K, const BCArgs A) {
 // use: the extrapolation forms are compiled in (a runtime choice left the others' operations in the pipe as
 // predicated-off slots), a species whose wall or lid is a copy reads only the plane it copies, and a thread
 // takes BC_SPECIES species of its column, so that the copy's density ratio -- a division, a dozen FP64
-// operations -- is formed once for them and not once per field. 41.7 -> 26 us at 41x181x361 (16 us of FP64 issue).
+// operations -- is formed once for them and not once per field. Where the wall or the lid is extrapolated there is
+// less to share and more to load: a thread per species, a path of its own (taking four there put loads between stores:
+// 9x31x61 6.2 us, now 4.2; and with that path apart the copies need fewer registers). The whole boundary call at
+// 41x181x361: 56.9 us with a thread per field, 39.6 with one path for both, 33.5 now; without copies 44.8, 38.5, 36.5.
 constexpr int BC_SPECIES = 4;                                   // species per thread (11: three threads a column)
 constexpr int BC_NSPEC = 11, BC_SPECIES_TASKS = (BC_NSPEC + BC_SPECIES - 1) / BC_SPECIES;
 constexpr int BC_PLAIN = 9;                                     // radius fields that are not species
@@ -160,31 +164,43 @@ __global__ void __launch_bounds__(128) bc_radius_kernel(const KConst K, const BC
     auto at = [&](int i) { return c0 + (int64_t)i * P; };
     const bool inner = j >= 1 && j <= K.jm - 2 && k <= K.km - 2;
     if (task >= BC_PLAIN + 3) {
-        const int s0 = (task - BC_PLAIN - 3) * BC_SPECIES;
         const bool lid = A.lid_copy != 0, wall = A.wall_copy != 0;
+        const int s0 = (task - BC_PLAIN - 3) * (lid && wall ? BC_SPECIES : 1);
         if (!inner && !lid && !wall) return;
-        double x1[BC_SPECIES], y2[BC_SPECIES];
+        const auto species = [&](auto extrapolate, int first, int last) {
+            constexpr bool EX = decltype(extrapolate)::value;
+            constexpr int N = EX ? 1 : BC_SPECIES;
+            const bool inx = EX && !wall && inner, iny = EX && !lid && inner;
+            double x1[N], x2[N], x3[N], y2[N], y3[N], y4[N];
 #pragma unroll
-        for (int q = 0; q < BC_SPECIES; q++) {
-            if (s0 + q >= BC_NSPEC) break;
-            x1[q] = get(A, A.species[s0 + q], at(1));
-            y2[q] = get(A, A.species[s0 + q], at(im - 2));
-        }
-        if (wall && A.wall_copy == 2) {
-            const double fr = wall_ratio(A, c0, P);
+            for (int q = 0; q < N; q++) {
+                if (first + q >= last) break;
+                const int F = A.species[first + q];
+                x1[q] = get(A, F, at(1));
+                y2[q] = get(A, F, at(im - 2));
+                if (EX) {
+                    x2[q] = inx ? get(A, F, at(2)) : 0.0;
+                    x3[q] = inx ? get(A, F, at(3)) : 0.0;
+                    y3[q] = iny ? get(A, F, at(im - 3)) : 0.0;
+                    y4[q] = iny ? get(A, F, at(im - 4)) : 0.0;
+                }
+            }
+            if (wall && A.wall_copy == 2) {
+                const double fr = wall_ratio(A, c0, P);
 #pragma unroll
-            for (int q = 0; q < BC_SPECIES; q++)
-                if (s0 + q < BC_NSPEC) x1[q] *= fr;
-        }
+                for (int q = 0; q < N; q++)
+                    if (first + q < last) x1[q] *= fr;
+            }
 #pragma unroll
-        for (int q = 0; q < BC_SPECIES; q++) {
-            if (s0 + q >= BC_NSPEC) break;
-            const int F = A.species[s0 + q];
-            if (!wall && inner) x1[q] = form_t<WALL>(x1[q], get(A, F, at(2)), get(A, F, at(3)), K.c43, K.c13);
-            if (!lid && inner) y2[q] = form_t<LID>(y2[q], get(A, F, at(im - 3)), get(A, F, at(im - 4)), K.c43, K.c13);
-            if (wall || inner) put(A, F, at(0), x1[q]);
-            if (lid || inner) put(A, F, at(im - 1), y2[q]);
-        }
+            for (int q = 0; q < N; q++) {
+                if (first + q >= last) break;
+                const int F = A.species[first + q];
+                if (wall || inner) put(A, F, at(0), inx ? form_t<WALL>(x1[q], x2[q], x3[q], K.c43, K.c13) : x1[q]);
+                if (lid || inner) put(A, F, at(im - 1), iny ? form_t<LID>(y2[q], y3[q], y4[q], K.c43, K.c13) : y2[q]);
+            }
+        };
+        if (lid && wall) species(std::false_type{}, s0, min(s0 + BC_SPECIES, BC_NSPEC));
+        else species(std::true_type{}, s0, s0 + 1);
         return;
     }
     if (task >= BC_PLAIN) {
@@ -529,7 +545,8 @@ cudaError_t launch_boundary_conditions(const KConst& kc, const atsat_dyn_params&
     static const Kernel kernels[3][3] = {{bc_radius_kernel<1, 1>, bc_radius_kernel<1, 2>, bc_radius_kernel<1, 3>},
                                          {bc_radius_kernel<2, 1>, bc_radius_kernel<2, 2>, bc_radius_kernel<2, 3>},
                                          {bc_radius_kernel<3, 1>, bc_radius_kernel<3, 2>, bc_radius_kernel<3, 3>}};
-    kernels[lid - 1][wall - 1]<<<dim3(gx, kc.jm, BC_PLAIN + 3 + BC_SPECIES_TASKS), 128, 0, s>>>(kc, A);
+    const int species_tasks = A.lid_copy != 0 && A.wall_copy != 0 ? BC_SPECIES_TASKS : BC_NSPEC;
+    kernels[lid - 1][wall - 1]<<<dim3(gx, kc.jm, BC_PLAIN + 3 + species_tasks), 128, 0, s>>>(kc, A);
     return cudaGetLastError();
 }
 
