@@ -3003,9 +3003,10 @@ int atsat_dyn_poisson_solve(atsat_dyn_t h, int32_t method, const double* src, do
     // A result array fresh from the allocator has no pages yet, and the GPU's faults on them cost more than the
     // transfer (21 MB at 41x181x361: 4.8 ms): the host threads touch its pages, values unchanged, while the source is
     // on its way up. Copies against in place, whole calls, FP64 direct: 41x181x361 2290 -> 2030 us, 21x91x181 509 -> 452,
-    // 21x60x121 324 -> 309. Below, the threads and the faults cost more than a copy's staging (13x50x101 254 against
-    // 258 us, 9x21x33 143 against 162, 5x7x9 107 against 133): copies up to IN_PLACE_CELLS.
-    constexpr int64_t IN_PLACE_CELLS = 100000;
+    // 18x60x97 301 -> 286. Below about 65,000 cells the threads and the faults cost what a copy's staging does
+    // (13x50x101 268 against 266 us, 11x41x81 208 against 211), and on the smallest grids more (9x21x33 143 against 162,
+    // 5x7x9 107 against 133): copies there.
+    constexpr int64_t IN_PLACE_CELLS = 65536;
     const int64_t cells = (int64_t)K.im * K.jm * K.km;
     const bool in_place = h->host_direct && cells >= IN_PLACE_CELLS &&
                           ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(p)) & 7u) == 0;

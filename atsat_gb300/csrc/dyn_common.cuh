@@ -451,7 +451,7 @@ size_t clamp_partial_doubles();
 cudaError_t launch_clamp_species(const KConst& kc, double* const f[11], float* const s32[11], double* added,
                                  unsigned long long* cells, double* partial, cudaStream_t s);
 
-// the final stage's FP64 half of fields q0..q1 after a tiled stage kernel (rk_mixed.cu)
+// adds the non-finite cells of n fields to *count (the restart check)
 cudaError_t launch_nonfinite_fields(const KConst& kc, const double* const* f, int n, unsigned long long* count,
                                     cudaStream_t s);
 

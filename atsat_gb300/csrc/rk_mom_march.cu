@@ -1,6 +1,7 @@
-// Launches of the radial-march momentum / temperature kernel on its own (rk_march_body.cuh): the final stage, knob sets
-// with more than 12 point arrays, and the regular rings. The intermediate stages of the default knob set run fused
-// with the tracers (rk_stage_fused.cu).
+// Launches of the radial-march momentum / temperature kernel on its own (rk_march_body.cuh): every stage that does not
+// share a launch with the tracers. That is any stage of a grid beyond the waves of stage_fusable (rk_stage_fused.cu; the
+// 41x181x361 shell among them), and on smaller grids the intermediate stages of knob sets with more than 12 point arrays
+// or with the regular rings.
 #include "rk_march_body.cuh"
 
 namespace atsat {
