@@ -69,12 +69,12 @@ __global__ void prep_seam_kernel(const KConst K, double* const* __restrict__ six
     f[c + K.km - 1] = f[c];
 }
 
-// The projection source with its clamp and lc_old. Bound by the FP64 pipe (two operations per SM per cycle): 16
+// The projection source with its clamp and lc_old. Bound by the FP64 pipe (two operations per SM per cycle): 17
 // operations per cell -- the scales of each difference are one product from the column table, the clamp's compare runs on
 // the integer pipe (positive doubles order as integers, finiteness is an exponent test), lc_old's three second
 // differences accumulate into div by fma. LEGACY: the source div(aux - rhs); INCR: lc_old is added. They are compiled in
 // because an instruction predicated off still takes its slot of that pipe: 98 -> 88 us at 41x181x361
-// (the operations alone are 64). CAP: the cap may be negative or NaN, whose bits do not order so: the comparison itself.
+// (the operations alone are 68). CAP: the cap may be negative or NaN, whose bits do not order so: the comparison itself.
 template <bool LEGACY, bool INCR, bool CAP>
 __global__ void __launch_bounds__(256) press_source_kernel(
         const KConst K, const ColGeo* __restrict__ geo, const double* __restrict__ su,

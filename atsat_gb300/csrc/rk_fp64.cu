@@ -120,7 +120,7 @@ constexpr int RKS_ROWS = 4, RKS_BLOCKS = 4;
 
 // What bounds it: the FP64 pipe (two operations per SM per cycle). With the differences of each field scaled and
 // combined one by one it was 590 FP64 instructions per interior cell and 2.38 ms per launch at 41x181x361, while
-// the launch's 1.97 GB take 0.29 ms. So the kernel is written for the fewest FP64 operations: 307 per cell, 1.47 ms
+// the launch's 1.97 GB take 0.29 ms. So the kernel is written for the fewest FP64 operations: 308 per cell, 1.47 ms
 // (the two-iteration step 20.03 -> 12.72 ms). Transport and diffusion of
 // RHS_Sat_Turb.cpp:300-1000 together are one weight per stencil value: seven fused multiply-adds per field with
 // weights that cost seven more per diffusivity -- shared by the three phases of a species, by u, v and w, and by the

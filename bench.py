@@ -478,7 +478,7 @@ def measure(a, rank, world, g, P, st, pinned, precision):
         # the FP64 roofline that binds: FP64 instructions per interior cell and stage counted by ncu
         # (profiles/rk_stage_fp64_21x91x181.md) over the same CUDA-event stage time, against 2 per SM per cycle
         sm_hz = (clk.get("sm_mhz") or 2070.0) * 1e6
-        per_cell = 303.0
+        per_cell = 308.0
         ach = per_cell * interior_rk(g) / (avg_ms / 1e3)
         peak64 = 2.0 * 152 * sm_hz
         roof["fp64_pipe"] = {"instructions_per_cell": per_cell, "achieved_per_s": ach, "peak_per_s": peak64,
