@@ -3017,30 +3017,37 @@ int atsat_dyn_poisson_solve(atsat_dyn_t h, int32_t method, const double* src, do
         b.f[0].dev = dev;
         return launch_host_transfer(b, to_device, (int64_t)K.im * K.jm, K.km, K.kp, h->stream);
     };
-    if (in_place) {
-        CK(h, move(src, f, 1));
-#pragma omp parallel for schedule(static)
-        for (int64_t c = 0; c < cells; c += 512) {
-            volatile double* page = p + c;
-            *page = *page;
-        }
-    } else {
-        CK(h, cudaMemcpy2DAsync(f, (size_t)K.kp * 8, src, (size_t)K.km * 8, (size_t)K.km * 8, (size_t)K.im * K.jm,
-                                cudaMemcpyHostToDevice, h->stream));
-    }
     cudaEvent_t ev[2];
     CK(h, cudaEventCreate(&ev[0]));
     CK(h, cudaEventCreate(&ev[1]));
-    CK(h, cudaEventRecord(ev[0], h->stream));
     int iters = 0, inner_total = 0;
     double rel = 0.0;
-    CK(h, poisson_run(h->poisson, method, tol, max_iter, inner, omega, &iters, &inner_total, &rel));
-    CK(h, cudaEventRecord(ev[1], h->stream));
-    CK(h, cudaEventSynchronize(ev[1]));
     float ms = 0.0f;
-    CK(h, cudaEventElapsedTime(&ms, ev[0], ev[1]));
+    auto solve = [&]() -> cudaError_t {
+        cudaError_t e;
+        if (in_place) {
+            if ((e = move(src, f, 1)) != cudaSuccess) return e;
+#pragma omp parallel for schedule(static)
+            for (int64_t c = 0; c < cells; c += 512) {
+                volatile double* page = p + c;
+                *page = *page;
+            }
+        } else if ((e = cudaMemcpy2DAsync(f, (size_t)K.kp * 8, src, (size_t)K.km * 8, (size_t)K.km * 8, (size_t)K.im * K.jm,
+                                          cudaMemcpyHostToDevice, h->stream)) != cudaSuccess) {
+            return e;
+        }
+        if ((e = cudaEventRecord(ev[0], h->stream)) != cudaSuccess) return e;
+        if ((e = poisson_run(h->poisson, method, tol, max_iter, inner, omega, &iters, &inner_total, &rel)) != cudaSuccess) return e;
+        if ((e = cudaEventRecord(ev[1], h->stream)) != cudaSuccess) return e;
+        if ((e = cudaEventSynchronize(ev[1])) != cudaSuccess) return e;
+        return cudaEventElapsedTime(&ms, ev[0], ev[1]);
+    };
+    const cudaError_t solved = solve();
+    // a refused solve too leaves nothing behind that still reads the caller's source
+    if (solved != cudaSuccess) cudaStreamSynchronize(h->stream);
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
+    if (solved != cudaSuccess) return fail(h, ATSAT_DYN_E_CUDA, "poisson_solve: %s", cudaGetErrorString(solved));
     if (in_place) CK(h, move(p, poisson_p(h->poisson), 0));
     else CK(h, cudaMemcpy2DAsync(p, (size_t)K.km * 8, poisson_p(h->poisson), (size_t)K.kp * 8, (size_t)K.km * 8,
                                  (size_t)K.im * K.jm, cudaMemcpyDeviceToHost, h->stream));
