@@ -96,10 +96,10 @@ constexpr bool slots_fit(int mode, bool dl, int ng) {
     }
     return true;
 }
-static_assert(slots_fit(MODE_STAGE, false, 1) && slots_fit(MODE_STAGE, false, 4) && slots_fit(MODE_STAGE, false, 13) &&
-              slots_fit(MODE_STAGE, true, 1) && slots_fit(MODE_STAGE, true, 4) && slots_fit(MODE_STAGE, true, 13) &&
-              slots_fit(MODE_FINAL, true, 1) && slots_fit(MODE_FINAL, true, 4) && slots_fit(MODE_FINAL, true, 13),
-              "point slots");
+constexpr bool slots_fit(int ng) {
+    return slots_fit(MODE_STAGE, false, ng) && slots_fit(MODE_STAGE, true, ng) && slots_fit(MODE_FINAL, true, ng);
+}
+static_assert(slots_fit(1) && slots_fit(2) && slots_fit(4) && slots_fit(13), "point slots");
 
 // One array's stencil of a lane's column of TI cells: the centre values at i-1 and i stay in registers from cell to
 // cell, so a cell costs five shared loads instead of seven.

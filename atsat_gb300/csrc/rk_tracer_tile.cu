@@ -45,12 +45,22 @@ cudaError_t launch_tiles(const TileMaps& maps, const MixedConstF& kf, const Mixe
 
 // What bounds a small grid is the serial stream of 13 fields through each of too few blocks (10 tiles at 10x20x36,
 // mostly latency). So where the resident blocks (three per SM) outnumber the tiles, the fields of a tile go to several
-// blocks, each streaming the winds again: 13 blocks per tile while all of them are resident at once, 4 while they make
-// at most two waves. Two iterations of the march variant (us) with 1, 4 and 13 groups: 10x20x36 286, 229, 214; 9x31x61
-// 274, 217, 210; 14x40x97 288, 246, 258; 21x60x121 385, 361, 400; 21x91x181 549, 567, 698.
+// blocks, each streaming the winds again: 13, 4 or 2 blocks per tile while all of them are resident at once. Two
+// iterations of the march variant (us), a lone state's replays and, after the bar, three states' in turn, whose blocks
+// fill idle SMs anyway and pay for the winds:
+//   tiles                    1           2           4          13 groups
+//      8  10x20x36   185 |  70   148 |  58   132 |  54   114 |  50
+//     45  14x40x97   189 | 110   157 | 102   156 | 106   167 | 122
+//    108  26x49x97   293 | 193   257 | 184   237 | 186   287 | 242
+//    135  61x40x60   331 | 232   299 | 230   309 | 247   351 | 312
+//    180  50x21x154  352 | 243   314 | 241   323 | 263   382 | 349
+//    240  31x121x61  378 | 284   366 | 287   375 | 307   457 | 411
+//    330  21x91x181  453 | 366   454 | 390   474 | 396   605 | 541
 int tracer_groups(int64_t tiles) {
     const int64_t slots = 3 * sm_count();
-    return tiles * 13 <= slots ? 13 : (tiles * 4 <= 2 * slots ? 4 : 1);
+    for (int ng : {13, 4, 2})
+        if (tiles * ng <= slots) return ng;
+    return 1;
 }
 
 // 64 x 4 tiles read a halo a tenth smaller per cell and in longer rows than 32 x 8, so they are taken unless they pad
